@@ -235,6 +235,7 @@ struct mf_ctx {
 	DevBuf<unsigned long long> bbox;
 	DevBuf<uint32_t> total_cells, keys, keys_sorted, perm_in, perm, cell_start, rec_body;
 	DevBuf<unsigned char> rec, sort_tmp;
+	DevBuf<float> pos;           // UL, FP64 forms: cell-ordered float-float positions (4 per row)
 	DevBuf<unsigned char> rec2;  // mixed UL: the second record buffer (stages alternate between the two)
 	int sort_bits = 1;
 	uint32_t cell_cap = 0;
@@ -456,6 +457,7 @@ ULArgs ul_args(mf_ctx* c, uint32_t stage) {
 	a.max_nbh = c->cfg.max_nbh;
 	a.strict_grid = c->mixed ? 0u : 1u;
 	a.nbh_eps = c->cfg.nbh_eps;
+	a.nbh_eps_f = (float)a.nbh_eps;
 	a.params = c->params.p;
 	a.geom = c->geom.p;
 	a.bbox = c->bbox.p;
@@ -471,6 +473,7 @@ ULArgs ul_args(mf_ctx* c, uint32_t stage) {
 	a.keys = c->keys.p; a.keys_sorted = c->keys_sorted.p; a.perm_in = c->perm_in.p; a.perm = c->perm.p;
 	a.cell_start = c->cell_start.p;
 	a.rec = c->rec.p;
+	a.pos = c->pos.p;
 	a.rec_body = c->rec_body.p;
 	if (c->mixed && c->rec2.p && !a.strict_grid) {
 		// the cell order holds for the whole step: stage s reads record buffer s % 2, and
@@ -688,6 +691,7 @@ mf_status finalize(mf_ctx* c) {
 		CK(c->rec_body.alloc(n));
 		CK(c->rec.alloc((size_t)n * 128));
 		if (c->mixed) CK(c->rec2.alloc((size_t)n * 128));
+		CK(c->pos.alloc((size_t)n * 4));
 		int bits = 1;
 		while (bits < 32 && (1ull << bits) < (uint64_t)c->cell_cap + 1) bits++;
 		c->sort_bits = bits;
@@ -2305,7 +2309,7 @@ mf_ctx::~mf_ctx() {
 		for (int q = 0; q < 4; q++) sf[k][q].free();
 	}
 	body_of.free(); params.free(); geom.free(); bbox.free(); total_cells.free(); keys.free(); keys_sorted.free();
-	perm_in.free(); perm.free(); cell_start.free(); rec_body.free(); rec.free(); rec2.free(); sort_tmp.free();
+	perm_in.free(); perm.free(); cell_start.free(); rec_body.free(); rec.free(); rec2.free(); pos.free(); sort_tmp.free();
 	{
 		DevBuf<uint32_t>* w32s[] = {&gp_body, &g_sl, &g_snbr, &t_sl, &t_snbr, &p_sl, &p_snbr};
 		for (auto* p : w32s) p->free();
@@ -3314,16 +3318,17 @@ MF_API mf_status mf_autotune(mf_ctx* c, int32_t trial_steps, char* report, uint3
 	for (uint32_t bs : {64u, 128u, 256u}) {
 		Tune t = c->tune;
 		if (c->cfg.method == MF_METHOD_UL) {
+			if (!c->mixed && bs != c->tune.ul_block) continue;  // the FP64 pair pass has one launch shape
 			t.ul_block = bs;
 			t.ul_persistent = 0;
 			t.ul_chunk = 1;
 			t.ul_split = 1;
 			cands.push_back(t);
-			if (c->mixed)
-				for (uint32_t sp : {4u, 8u}) {
-					t.ul_split = sp;
-					cands.push_back(t);
-				}
+			if (!c->mixed) continue;
+			for (uint32_t sp : {4u, 8u}) {
+				t.ul_split = sp;
+				cands.push_back(t);
+			}
 			t.ul_split = 1;
 			for (uint32_t ch : {1u, 4u}) {
 				t.ul_persistent = 1;

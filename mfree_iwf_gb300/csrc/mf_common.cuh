@@ -143,6 +143,40 @@ MF_DEV KR32 cubic_spline_f(float xij, float yij, float h1, float fac) {
 	return w;
 }
 
+// Reciprocal and reciprocal square root in FP64 by one third-order step from an FP32
+// seed (Householder's iteration: with e = 1 - d r, 1/d = r (1 + e + e^2 + ...), and with
+// e = 1 - d y^2, 1/sqrt(d) = y (1 + e/2 + 3 e^2 / 8 + ...)).  The seed takes the leading
+// 24 bits of d, so |e| < 1e-6 and the terms left out are below 1e-18: results within an
+// ulp or two, in 3 and 5 FP64 instructions where the division and the square root take
+// several times that on the narrow FP64 pipe (the seeds and their conversions run on the
+// integer and FP32 pipes).  Zeros, subnormals, infinities, NaNs and exponents beyond
+// 2^+-123 take the plain operations.
+MF_DEV bool seed_range(int hi) { return (((uint32_t)hi >> 20) & 0x7ffu) - 900u < 246u; }
+MF_DEV float seed_f32(double d) {
+	const uint32_t h = (uint32_t)__double2hiint(d), l = (uint32_t)__double2loint(d);
+	return __uint_as_float((h & 0x80000000u) | ((((h >> 20) & 0x7ffu) - 896u) << 23) | ((h & 0xfffffu) << 3) | (l >> 29));
+}
+MF_DEV double seed_f64(float f) {  // f normal
+	const uint32_t u = __float_as_uint(f);
+	return __hiloint2double((int)((u & 0x80000000u) | ((((u >> 23) & 0xffu) + 896u) << 20) | ((u & 0x7fffffu) >> 3)),
+	                        (int)(u << 29));
+}
+MF_DEV double rcp64(double d) {
+	if (!seed_range(__double2hiint(d))) return 1. / d;
+	const double r = seed_f64(__fdividef(1.f, seed_f32(d)));
+	const double e = fma(-d, r, 1.);
+	return fma(r, fma(e, e, e), r);
+}
+MF_DEV double rsqrt64(double d) {
+	const int h = __double2hiint(d);
+	if (h < 0 || !seed_range(h)) return 1. / sqrt(d);
+	const double y = seed_f64(rsqrtf(seed_f32(d)));
+	const double e = fma(-d * y, y, 1.);
+	return fma(y * e, fma(0.375, e, 0.5), y);
+}
+// max(v, 0) by the sign bit (no FP64 compare); NaN stays NaN or becomes 0 by its sign
+MF_DEV double clamp0(double v) { return __double2hiint(v) < 0 ? 0. : v; }
+
 // Column-major 2x2 matrix: c[col][row], GLM's convention, used to restate the
 // reference's glm::dmat2x2 expressions with the same operation order.
 template <class T>
@@ -194,6 +228,15 @@ MF_DEV void jaumann(T vx_x, T vx_y, T vy_x, T vy_y, T Sxx, T Sxy, T Syy, T G, T&
 	dSxx = S_t.c[0][0];
 	dSxy = S_t.c[0][1];
 	dSyy = S_t.c[1][1];
+}
+
+// The same rate with the products by zero written out (fast FP64 forms).
+MF_DEV void jaumann_plane(double vx_x, double vx_y, double vy_x, double vy_y, double Sxx, double Sxy, double Syy,
+                          double G, double& dSxx, double& dSxy, double& dSyy) {
+	const double third = (vx_x + vy_y) * (1. / 3.), G2 = 2. * G, spin = vx_y - vy_x;
+	dSxx = fma(spin, Sxy, G2 * (vx_x - third));
+	dSyy = fma(-spin, Sxy, G2 * (vy_y - third));
+	dSxy = fma(0.5 * spin, Syy - Sxx, G * (vx_y + vy_x));
 }
 
 // Cauchy -> nominal stress P = J F^-1 sigma (cont_mech.h:154-169); F from the

@@ -69,6 +69,7 @@ struct ULArgs {
 	uint32_t max_nbh;                     // neighbour capacity (0 = unchecked)
 	uint32_t strict_grid;                 // 1: rebuild the reference grid at this stage
 	double nbh_eps;
+	float nbh_eps_f;                      // its FP32 copy
 	const BodyParams* params;             // device
 	Geom* geom;                           // device, per body
 	unsigned long long* bbox;             // device, 6 per body
@@ -80,6 +81,7 @@ struct ULArgs {
 	uint32_t* cell_start;                 // capacity cell_cap + 1
 	uint32_t cell_cap;                    // most cells over all bodies (0: n_total + 1)
 	void* rec;                            // cell-ordered gathered records
+	void* pos;                            // FP64 forms: cell-ordered float-float positions (float4 per row)
 	uint32_t* rec_body;                   // body of each cell-ordered row
 	void* sort_tmp;
 	size_t sort_tmp_bytes;

@@ -57,7 +57,8 @@ constexpr size_t OFF_FC = align_up(OFF_REC_BODY + 4ull * kMaxN);          // fcx
 constexpr size_t OFF_ACC = align_up(OFF_FC + 2 * 8ull * kMaxN);           // 8 fields
 constexpr size_t OFF_ST = align_up(OFF_ACC + 8 * 8ull * kMaxN);           // 8 fields
 constexpr size_t OFF_REC = align_up(OFF_ST + 8 * 8ull * kMaxN);           // 128 B per row
-constexpr size_t OFF_SORT_TMP = align_up(OFF_REC + 128ull * kMaxN);
+constexpr size_t OFF_POS = align_up(OFF_REC + 128ull * kMaxN);             // 16 B per row
+constexpr size_t OFF_SORT_TMP = align_up(OFF_POS + 16ull * kMaxN);
 constexpr size_t SORT_TMP_BYTES = 1u << 20;
 constexpr size_t SCRATCH_BYTES = OFF_SORT_TMP + SORT_TMP_BYTES;
 
@@ -155,6 +156,7 @@ extern "C" MF_API mf_status mf_ul_step_noalloc(const mf_device_body* body, const
 	a.max_nbh = 200;  // MAX_NBH, particle.h:31
 	a.strict_grid = 1;
 	a.nbh_eps = 1e-6;  // grid.h:157
+	a.nbh_eps_f = (float)a.nbh_eps;
 	a.params = reinterpret_cast<const BodyParams*>(B + OFF_PARAMS);
 	a.geom = reinterpret_cast<Geom*>(B + OFF_GEOM);
 	a.bbox = reinterpret_cast<unsigned long long*>(B + OFF_BBOX);
@@ -177,6 +179,7 @@ extern "C" MF_API mf_status mf_ul_step_noalloc(const mf_device_body* body, const
 	a.perm = reinterpret_cast<uint32_t*>(B + OFF_PERM);
 	a.cell_start = reinterpret_cast<uint32_t*>(B + OFF_CELLS);
 	a.rec = B + OFF_REC;
+	a.pos = B + OFF_POS;
 	a.rec_body = reinterpret_cast<uint32_t*>(B + OFF_REC_BODY);
 	a.sort_tmp = B + OFF_SORT_TMP;
 	a.sort_tmp_bytes = S->sort_tmp_needed;

@@ -409,6 +409,35 @@ __device__ __forceinline__ void per_particle32(uint32_t flags, const BodyParams&
 	rho21 = 1.f / (rho * rho);
 }
 
+#if !MF_STRICT_FORM
+// The same for the fast FP64 gather, which the narrow FP64 pipe bounds: the principal
+// stresses from the stress circle, cos 2 theta and sin 2 theta as its components over its
+// radius, in place of atan2, cos and sin of the angle (337k rows: 100 -> 41 us).
+__device__ __forceinline__ void per_particle64(uint32_t flags, const BodyParams& pr, double m, double rho, double qw0,
+                                               double Sxx, double Sxy, double Syy, Rec64& r) {
+	const double p = (flags & A_EOS) ? pr.c0sq * (rho - pr.rho0) : 0.;
+	const double rho1 = rcp64(rho);
+	r.sxx = Sxx - p;
+	r.syy = Syy - p;
+	r.sxy = Sxy;
+	r.rho21 = rho1 * rho1;
+	r.qw = (flags & A_RIEMANN) ? m * rho1 : qw0;
+	r.c = sqrt(pr.K * rho1);
+	r.Rxx = r.Rxy = r.Ryy = 0.;
+	if (flags & A_ART_STRESS) {
+		const double dev = r.sxx - r.syy, twice = 2. * Sxy, mean = 0.5 * (r.sxx + r.syy);
+		const double R2 = fma(dev, dev, twice * twice);
+		const double R1 = R2 > 0. ? rsqrt64(R2) : 0., radius = 0.5 * R2 * R1;
+		const double c2 = R2 > 0. ? 0.5 * dev * R1 : 0.5, s2 = 0.5 * twice * R1;  // halves of cos, sin 2 theta
+		const double eps = -pr.mghn_eps * r.rho21;
+		const double ra = eps * clamp0(mean + radius), rb = eps * clamp0(mean - radius);
+		r.Rxx = (0.5 + c2) * ra + (0.5 - c2) * rb;
+		r.Ryy = (0.5 - c2) * ra + (0.5 + c2) * rb;
+		r.Rxy = s2 * (ra - rb);
+	}
+}
+#endif
+
 __global__ void k_gather64(ULArgs a, const BodyParams* __restrict__ P) {
 	uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
 	if (k >= a.n_total) return;
@@ -420,13 +449,28 @@ __global__ void k_gather64(ULArgs a, const BodyParams* __restrict__ P) {
 	Rec64 r;
 	r.x = x; r.y = y; r.vx = vx; r.vy = vy;
 	r.m = a.m[i]; r.h = a.h[i]; r.rho = rho;
+#if MF_STRICT_FORM
 	per_particle<double>(a.flags, P[b], r.m, rho, a.qw0[i], Sxx, Sxy, Syy, r.sxx, r.syy, r.Rxx, r.Rxy, r.Ryy, r.c, r.qw,
 	                     r.rho21);
 	r.sxy = Sxy;
+#else
+	per_particle64(a.flags, P[b], r.m, rho, a.qw0[i], Sxx, Sxy, Syy, r);
+#endif
 	if (a.flags & (A_GOD_CONT | A_GOD_MOM)) {
 		r.Rxx = (a.flags & A_EOS) ? P[b].c0sq * (rho - P[b].rho0) : 0.;
 		r.Rxy = Syy;
 	}
+#if !MF_STRICT_FORM
+	else {  // pair64_fast takes the stresses times 1/rho^2 and c times alpha / 2
+		r.c *= 0.5 * P[b].alpha;
+		r.sxx *= r.rho21;
+		r.sxy *= r.rho21;
+		r.syy *= r.rho21;
+	}
+#endif
+	// float-float positions for the candidate tests
+	const FF fx = ff_split_bits(x), fy = ff_split_bits(y);
+	reinterpret_cast<float4*>(a.pos)[k] = make_float4(fx.hi, fx.lo, fy.hi, fy.lo);
 	Rec64* out = reinterpret_cast<Rec64*>(a.rec) + k;
 	const double2* s = reinterpret_cast<const double2*>(&r);
 	double2* d = reinterpret_cast<double2*>(out);
@@ -469,60 +513,6 @@ __global__ void k_gather32(ULArgs a, const BodyParams* __restrict__ P) {
 	a.rec_body[k] = b;
 }
 
-// --------------------------------------------------------------- RK update
-// rk4.h:52-69 (stage state = particles + c*dt*derivative) and :94-103 (final
-// combine with weights 1,2,2,1 / 6).  d[] = x_t, y_t, vx_t, vy_t, rho_t, Sxx_t, Sxy_t, Syy_t.
-template <class T>
-__device__ __forceinline__ void rk_update_f64(const ULArgs& a, uint32_t i, double dt, const double d[8]) {
-	double* bp[8] = {a.base.x, a.base.y, a.base.vx, a.base.vy, a.base.rho, a.base.Sxx, a.base.Sxy, a.base.Syy};
-	double* ap[8] = {a.acc.x, a.acc.y, a.acc.vx, a.acc.vy, a.acc.rho, a.acc.Sxx, a.acc.Sxy, a.acc.Syy};
-	double* sp[8] = {a.st.x, a.st.y, a.st.vx, a.st.vy, a.st.rho, a.st.Sxx, a.st.Sxy, a.st.Syy};
-	uint32_t s = a.stage;
-	if (s < 3) {
-		double dts = (s == 2 ? 1.0 : 0.5) * dt;
-#pragma unroll
-		for (int q = 0; q < 8; q++) {
-			double accv = (s == 0) ? d[q] : ap[q][i] + 2 * d[q];
-			ap[q][i] = accv;
-			sp[q][i] = bp[q][i] + d[q] * dts;
-		}
-	} else {
-		double w6 = dt * 1. / 6.;
-#pragma unroll
-		for (int q = 0; q < 8; q++) bp[q][i] = bp[q][i] + w6 * (ap[q][i] + d[q]);
-	}
-}
-
-// Mixed form: x, y, vx, vy accumulate in FP64, rho and the stresses in FP32.
-__device__ __forceinline__ void rk_update_mixed(const ULArgs& a, uint32_t i, double dt, const float d[8]) {
-	double* bp[4] = {a.base.x, a.base.y, a.base.vx, a.base.vy};
-	double* ap[4] = {a.acc.x, a.acc.y, a.acc.vx, a.acc.vy};
-	double* sp[4] = {a.st.x, a.st.y, a.st.vx, a.st.vy};
-	float* bq[4] = {a.base.rho_f, a.base.Sxx_f, a.base.Sxy_f, a.base.Syy_f};
-	float* aq[4] = {a.acc.rho_f, a.acc.Sxx_f, a.acc.Sxy_f, a.acc.Syy_f};
-	float* sq[4] = {a.st.rho_f, a.st.Sxx_f, a.st.Sxy_f, a.st.Syy_f};
-	uint32_t s = a.stage;
-	if (s < 3) {
-		double dts = (s == 2 ? 1.0 : 0.5) * dt;
-#pragma unroll
-		for (int q = 0; q < 4; q++) {
-			double dq = (double)d[q];
-			ap[q][i] = (s == 0) ? dq : ap[q][i] + 2 * dq;
-			sp[q][i] = bp[q][i] + dq * dts;
-			float dr = d[4 + q];
-			aq[q][i] = (s == 0) ? dr : aq[q][i] + 2.f * dr;
-			sq[q][i] = bq[q][i] + dr * (float)dts;
-		}
-	} else {
-		double w6 = dt * 1. / 6.;
-#pragma unroll
-		for (int q = 0; q < 4; q++) {
-			bp[q][i] = bp[q][i] + w6 * (ap[q][i] + (double)d[q]);
-			bq[q][i] = bq[q][i] + (float)w6 * (aq[q][i] + d[4 + q]);
-		}
-	}
-}
-
 __device__ __forceinline__ void stencil(const Geom& g, uint32_t key, int& lo_i, int& hi_i, int& lo_j, int& hi_j) {
 	uint32_t b = key - g.cell_off;
 	uint32_t gi = b / g.ny;
@@ -535,169 +525,454 @@ __device__ __forceinline__ void stencil(const Geom& g, uint32_t key, int& lo_i, 
 }
 
 // ----------------------------------------------------------- pair kernel FP64
-__device__ __forceinline__ void pair64_row(const ULArgs& a, const BodyParams* __restrict__ P,
-                                           const Geom* __restrict__ G, DevStatus* st, uint32_t k) {
-	uint32_t b = a.rec_body[k];
-	if (is_failed(a.failed, b)) return;  // a failed body stays as it was
-	const Rec64* rec = reinterpret_cast<const Rec64*>(a.rec);
-	const Rec64 ri = load_rec(rec + k);
-	const BodyParams& pr = P[b];
-	Geom g = G[b];
-	uint32_t i = a.perm[k];
-	uint32_t flags = a.flags;
-	int lo_i, hi_i, lo_j, hi_j;
-	stencil(g, a.keys_sorted[k], lo_i, hi_i, lo_j, hi_j);
-	const uint32_t tot = *a.total_cells;
+// GB300 issues FP64 at 2 lanes a clock and SM: a warp instruction holds the pipe for 16
+// clocks however few of its lanes are active, so these kernels' time is their FP64 warp
+// instructions.  Three things keep them low.
+//
+// 1. Four lanes share a row (P64_L).  They test the row's candidates in FP32, from the
+//    float-float positions the gather writes, and list the ones within reach in shared
+//    memory; then lane l takes the listed pairs l, l + 4, ...  A warp's eight rows finish
+//    in ceil(most neighbours / 4) pair evaluations with nearly every lane at work, where
+//    one thread a row ran the pair terms for every candidate that some lane accepted.
+//    The split depends on the row's own candidates alone, never on the launch, so a body
+//    gets the same bits in any batch.
+// 2. The FP32 test decides only what it can: the offsets' error is at most
+//    2^-23 |d| + 2^-46 |x| (the split keeps 48 bits), under 2e-6 of the squared distance
+//    while |x| <= 2^26 h; a candidate within 2e-5 of the reference's limit, and every
+//    candidate of a row outside those ranges, is decided by the reference's FP64
+//    predicate, so the counts and the neighbour sets are the reference's.
+// 3. The fast form rearranges the Gray-Monaghan pair terms (pair64_fast).
+//
+// Ensemble of 16 ring impacts (337k rows), per stage: 4.89 ms with one thread a row and
+// the FP64 test, 1.27 ms now (503 FP64 instructions a warp of eight rows, the FP64 pipe
+// 87 % busy); rings at dx = 1 mm (4,408 rows), parity form, per step: 1.76 ms -> 0.42 ms
+// (there the 35 blocks of 128 rows had also left 117 of the 152 SMs empty).
+constexpr uint32_t P64_L = 4;        // lanes per row
+constexpr uint32_t P64_CAP = 96;    // listed pairs per row before they are worked off
+constexpr uint32_t P64_THREADS = 128;
+constexpr uint32_t P64_ROWS = P64_THREADS / P64_L;
 
-	double hi = ri.h;
-	double radius2 = __dmul_rn(__dmul_rn(__dmul_rn(hi, hi), 2.), 2.);
-	double lim = __dadd_rn(radius2, a.nbh_eps);
-	double reach2 = 4.0000001 * hi * hi;  // pairs beyond q = 2 contribute exactly zero
-	double rhoi21 = ri.rho21;
-	double wdeltap = pr.wdeltap, corr_exp = pr.corr_exp;
-	double alpha = pr.alpha, beta = pr.beta, eta = pr.eta, xeps = pr.xsph_eps;
-
+// The pair sums of one row (a lane's share of them)
+struct Acc64 {
 	double Sxx_x = 0., Sxy_y = 0., Sxy_x = 0., Syy_y = 0.;
 	double vx_x = 0., vx_y = 0., vy_x = 0., vy_y = 0.;
 	double av_x = 0., av_y = 0., xs_x = 0., xs_y = 0.;
 	double god_rho = 0., god_vx = 0., god_vy = 0.;
-	const double two_rhoi = 2. / ri.rho;  // godunov.h:127-133's 2./rhoi, the same per pair
-	uint32_t cnt = 0;
-	for (int ni = lo_i; ni < hi_i; ni++) {
-		uint32_t c0 = min(g.cell_off + (uint32_t)ni * g.ny + (uint32_t)lo_j, tot);
-		uint32_t c1 = min(g.cell_off + (uint32_t)ni * g.ny + (uint32_t)hi_j, tot);
-		uint32_t j0 = a.cell_start[c0], j1 = a.cell_start[c1];
-		for (uint32_t kj = j0; kj < j1; kj++) {
-			const Rec64 rj = load_rec(rec + kj);
-			double xij = __dsub_rn(ri.x, rj.x);
-			double yij = __dsub_rn(ri.y, rj.y);
-			double r2 = __dadd_rn(__dmul_rn(xij, xij), __dmul_rn(yij, yij));
-			cnt += (r2 <= lim) ? 1u : 0u;
-			if (r2 > reach2) continue;
-			KR64 w = cubic_spline(xij, yij, hi);
-			if (flags & A_STRESS_MGHN) {
-				double Rxx = 0., Rxy = 0., Ryy = 0.;
-				if (wdeltap > 0) {
-					double fab = w.w / wdeltap;
-					if (corr_exp == 4.) {
-						double f2 = fab * fab;
-						fab = f2 * f2;
-					} else {
-						fab = pow(fab, corr_exp);
-					}
-					Rxx = fab * (ri.Rxx + rj.Rxx);
-					Rxy = fab * (ri.Rxy + rj.Rxy);
-					Ryy = fab * (ri.Ryy + rj.Ryy);
-				}
-				Sxx_x += rj.m * (ri.sxx * rhoi21 + rj.sxx * rj.rho21 + Rxx) * w.w_x;
-				Sxy_y += rj.m * (ri.sxy * rhoi21 + rj.sxy * rj.rho21 + Rxy) * w.w_y;
-				Sxy_x += rj.m * (ri.sxy * rhoi21 + rj.sxy * rj.rho21 + Rxy) * w.w_x;
-				Syy_y += rj.m * (ri.syy * rhoi21 + rj.syy * rj.rho21 + Ryy) * w.w_y;
+};
+
+// All pair terms in the reference's expressions.  rho21: whether the records hold the
+// stress itself (1/rho^2 applied here) or already times 1/rho^2 (the fast gather).
+template <bool GOD>
+__device__ __forceinline__ void pair64_ref(uint32_t flags, const BodyParams& pr, const Rec64& ri, const Rec64& rj,
+                                           Acc64& s) {
+	const double hi = ri.h;
+	double xij = __dsub_rn(ri.x, rj.x);
+	double yij = __dsub_rn(ri.y, rj.y);
+	double r2 = __dadd_rn(__dmul_rn(xij, xij), __dmul_rn(yij, yij));
+	KR64 w = cubic_spline(xij, yij, hi);
+	if (flags & A_STRESS_MGHN) {
+		double Rxx = 0., Rxy = 0., Ryy = 0.;
+		if (pr.wdeltap > 0) {
+			double fab = w.w / pr.wdeltap;
+			if (pr.corr_exp == 4.) {
+				double f2 = fab * fab;
+				fab = f2 * f2;
+			} else {
+				fab = pow(fab, pr.corr_exp);
 			}
-			if (flags & A_DERIVE_VEL) {
-				vx_x += (rj.vx - ri.vx) * w.w_x * rj.qw;
-				vx_y += (rj.vx - ri.vx) * w.w_y * rj.qw;
-				vy_x += (rj.vy - ri.vy) * w.w_x * rj.qw;
-				vy_y += (rj.vy - ri.vy) * w.w_y * rj.qw;
-			}
-			double vijx = ri.vx - rj.vx, vijy = ri.vy - rj.vy;
-			if (flags & A_ART_VISC) {
-				double vijposij = vijx * xij + vijy * yij;
-				if (vijposij < 0.) {
-					double cij = 0.5 * (ri.c + rj.c);
-					double hij = 0.5 * (hi + rj.h);
-					double rhoij = 0.5 * (ri.rho + rj.rho);
-					double r2ij = xij * xij + yij * yij;
-					double muij = (hij * vijposij) / (r2ij + eta * eta * hij * hij);
-					double piij = (-alpha * cij * muij + beta * muij * muij) / rhoij;
-					av_x += -rj.m * piij * w.w_x;
-					av_y += -rj.m * piij * w.w_y;
-				}
-			}
-			if (flags & A_XSPH) {
-				double rhoij = 0.5 * (ri.rho + rj.rho);
-				double fac = -xeps * w.w * ri.m / rhoij;
-				xs_x += fac * vijx;
-				xs_y += fac * vijy;
-			}
-			if ((flags & (A_GOD_CONT | A_GOD_MOM)) && kj != k) {
-				// |x_j - x_i| from the predicate's own sum (the same value as the
-				// reference's sqrt(dx*dx + dy*dy) and sqrt(dot(R, R)))
-				const double mag_r = sqrt(r2);
-				// the acoustic Riemann denominator, the same expression in both actions
-				const double frac = 1. / (ri.rho * ri.c + rj.rho * rj.c);
+			Rxx = fab * (ri.Rxx + rj.Rxx);
+			Rxy = fab * (ri.Rxy + rj.Rxy);
+			Ryy = fab * (ri.Ryy + rj.Ryy);
+		}
+		const double rhoi21 = ri.rho21;
+		s.Sxx_x += rj.m * (ri.sxx * rhoi21 + rj.sxx * rj.rho21 + Rxx) * w.w_x;
+		s.Sxy_y += rj.m * (ri.sxy * rhoi21 + rj.sxy * rj.rho21 + Rxy) * w.w_y;
+		s.Sxy_x += rj.m * (ri.sxy * rhoi21 + rj.sxy * rj.rho21 + Rxy) * w.w_x;
+		s.Syy_y += rj.m * (ri.syy * rhoi21 + rj.syy * rj.rho21 + Ryy) * w.w_y;
+	}
+	if (flags & A_DERIVE_VEL) {
+		s.vx_x += (rj.vx - ri.vx) * w.w_x * rj.qw;
+		s.vx_y += (rj.vx - ri.vx) * w.w_y * rj.qw;
+		s.vy_x += (rj.vy - ri.vy) * w.w_x * rj.qw;
+		s.vy_y += (rj.vy - ri.vy) * w.w_y * rj.qw;
+	}
+	double vijx = ri.vx - rj.vx, vijy = ri.vy - rj.vy;
+	if (flags & A_ART_VISC) {
+		double vijposij = vijx * xij + vijy * yij;
+		if (vijposij < 0.) {
+			double cij = 0.5 * (ri.c + rj.c);
+			double hij = 0.5 * (hi + rj.h);
+			double rhoij = 0.5 * (ri.rho + rj.rho);
+			double r2ij = xij * xij + yij * yij;
+			double muij = (hij * vijposij) / (r2ij + pr.eta * pr.eta * hij * hij);
+			double piij = (-pr.alpha * cij * muij + pr.beta * muij * muij) / rhoij;
+			s.av_x += -rj.m * piij * w.w_x;
+			s.av_y += -rj.m * piij * w.w_y;
+		}
+	}
+	if (flags & A_XSPH) {
+		double rhoij = 0.5 * (ri.rho + rj.rho);
+		double fac = -pr.xsph_eps * w.w * ri.m / rhoij;
+		s.xs_x += fac * vijx;
+		s.xs_y += fac * vijy;
+	}
+	if (GOD) {
+		// |x_j - x_i| from the predicate's own sum (the same value as the
+		// reference's sqrt(dx*dx + dy*dy) and sqrt(dot(R, R)))
+		const double mag_r = sqrt(r2);
+		// the acoustic Riemann denominator, the same expression in both actions
+		const double frac = 1. / (ri.rho * ri.c + rj.rho * rj.c);
 #if !MF_STRICT_FORM
-				const double inv_r = 1. / mag_r;
+		const double inv_r = 1. / mag_r;
 #endif
-				if (flags & A_GOD_CONT) {  // godunov_continuity, godunov.h:144-187
+		if (flags & A_GOD_CONT) {  // godunov_continuity, godunov.h:144-187
 #if MF_STRICT_FORM
-					double nx = xij / mag_r, ny = yij / mag_r;
+			double nx = xij / mag_r, ny = yij / mag_r;
 #else
-					double nx = xij * inv_r, ny = yij * inv_r;
+			double nx = xij * inv_r, ny = yij * inv_r;
 #endif
-					double vir = ri.vx * nx + ri.vy * ny;
-					double vjr = rj.vx * nx + rj.vy * ny;
-					// riemann_solver_acoustic (godunov.h:41-54); Rxx = p
-					double ustar = frac * (vir * ri.rho * ri.c + vjr * rj.rho * rj.c - ri.Rxx + rj.Rxx);
-					god_rho += 2 * ri.rho * (vir - ustar) * (w.w_x * nx + w.w_y * ny) * rj.qw;
-				}
-				if (flags & A_GOD_MOM) {  // godunov_get_trafo + godunov_momentum, godunov.h:56-142
-					double rx = rj.x - ri.x, ry = rj.y - ri.y;
+			double vir = ri.vx * nx + ri.vy * ny;
+			double vjr = rj.vx * nx + rj.vy * ny;
+			// riemann_solver_acoustic (godunov.h:41-54); Rxx = p
+			double ustar = frac * (vir * ri.rho * ri.c + vjr * rj.rho * rj.c - ri.Rxx + rj.Rxx);
+			s.god_rho += 2 * ri.rho * (vir - ustar) * (w.w_x * nx + w.w_y * ny) * rj.qw;
+		}
+		if (flags & A_GOD_MOM) {  // godunov_get_trafo + godunov_momentum, godunov.h:56-142
+			const double two_rhoi = 2. / ri.rho;  // godunov.h:127-133's 2./rhoi, the same per pair
+			double rx = rj.x - ri.x, ry = rj.y - ri.y;
 #if MF_STRICT_FORM
-					double inv = 1. / mag_r;  // glm::normalize: v * (1 / sqrt(dot(v, v)))
+			double inv = 1. / mag_r;  // glm::normalize: v * (1 / sqrt(dot(v, v)))
 #else
-					double inv = inv_r;
+			double inv = inv_r;
 #endif
-					double Rx = rx * inv, Ry = ry * inv, Sx = ry * inv, Sy = -rx * inv;
-					// the frame matrix is single precision (a glm::mat2x2 of the unit vectors)
-					double lRx = (double)__double2float_rn(Rx), lRy = (double)__double2float_rn(Ry);
-					double lSx = (double)__double2float_rn(Sx), lSy = (double)__double2float_rn(Sy);
-					// stress times R: (Sxx - p, Sxy; Sxy, Syy), Rxy = Syy
-					double siR0 = ri.sxx * Rx + ri.sxy * Ry, siR1 = ri.sxy * Rx + ri.Rxy * Ry;
-					double sjR0 = rj.sxx * Rx + rj.sxy * Ry, sjR1 = rj.sxy * Rx + rj.Rxy * Ry;
-					double si0 = lRx * siR0 + lSx * siR1;
-					double sj0 = lRx * sjR0 + lSx * sjR1, sj1 = lRy * sjR0 + lSy * sjR1;
-					double vi0 = lRx * ri.vx + lSx * ri.vy, vi1 = lRy * ri.vx + lSy * ri.vy;
-					double vj0 = lRx * rj.vx + lSx * rj.vy, vj1 = lRy * rj.vx + lSy * rj.vy;
-					// the second component takes sigma_j twice (godunov.h:116), as the reference does
-					double S0 = frac * (sj0 * ri.rho * ri.c + si0 * rj.rho * rj.c + ri.rho * ri.c * rj.rho * rj.c * (vj0 - vi0));
-					double S1 = frac * (sj1 * ri.rho * ri.c + sj1 * rj.rho * rj.c + ri.rho * ri.c * rj.rho * rj.c * (vj1 - vi1));
-					double SR0 = lRx * S0 + lRy * S1, SR1 = lSx * S0 + lSy * S1;
-					if (fabs(rx) > 0.) god_vx += two_rhoi * w.w_x * mag_r / rx * SR0 * rj.qw;
-					if (fabs(ry) > 0.) god_vy += two_rhoi * w.w_y * mag_r / ry * SR1 * rj.qw;
+			double Rx = rx * inv, Ry = ry * inv, Sx = ry * inv, Sy = -rx * inv;
+			// the frame matrix is single precision (a glm::mat2x2 of the unit vectors)
+			double lRx = (double)__double2float_rn(Rx), lRy = (double)__double2float_rn(Ry);
+			double lSx = (double)__double2float_rn(Sx), lSy = (double)__double2float_rn(Sy);
+			// stress times R: (Sxx - p, Sxy; Sxy, Syy), Rxy = Syy
+			double siR0 = ri.sxx * Rx + ri.sxy * Ry, siR1 = ri.sxy * Rx + ri.Rxy * Ry;
+			double sjR0 = rj.sxx * Rx + rj.sxy * Ry, sjR1 = rj.sxy * Rx + rj.Rxy * Ry;
+			double si0 = lRx * siR0 + lSx * siR1;
+			double sj0 = lRx * sjR0 + lSx * sjR1, sj1 = lRy * sjR0 + lSy * sjR1;
+			double vi0 = lRx * ri.vx + lSx * ri.vy, vi1 = lRy * ri.vx + lSy * ri.vy;
+			double vj0 = lRx * rj.vx + lSx * rj.vy, vj1 = lRy * rj.vx + lSy * rj.vy;
+			// the second component takes sigma_j twice (godunov.h:116), as the reference does
+			double S0 = frac * (sj0 * ri.rho * ri.c + si0 * rj.rho * rj.c + ri.rho * ri.c * rj.rho * rj.c * (vj0 - vi0));
+			double S1 = frac * (sj1 * ri.rho * ri.c + sj1 * rj.rho * rj.c + ri.rho * ri.c * rj.rho * rj.c * (vj1 - vi1));
+			double SR0 = lRx * S0 + lRy * S1, SR1 = lSx * S0 + lSy * S1;
+			if (fabs(rx) > 0.) s.god_vx += two_rhoi * w.w_x * mag_r / rx * SR0 * rj.qw;
+			if (fabs(ry) > 0.) s.god_vy += two_rhoi * w.w_y * mag_r / ry * SR1 * rj.qw;
+		}
+	}
+}
+
+#if !MF_STRICT_FORM
+// The Gray-Monaghan pair terms for the fast form: the same sums in ~70 FP64 instructions
+// a pair against ~150 (square root and five divisions included).
+//  * the spline through t = 2 - q and u = max(1 - q, 0): W = fac (t^3 / 4 - u^3) and
+//    dW/dq = 3 fac (u^2 - t^2 / 4), one expression for both pieces (t clamped at 0 beyond
+//    2h); the factor 3 fac is applied to the row's gradient sums at the end;
+//  * 1/r, 1/(r^2 + eta^2 h^2) and 1/(rho_i + rho_j) by one third-order step from an FP32
+//    seed (rsqrt64, rcp64);
+//  * stress and viscosity share one gradient sum, (s_i + s_j + R - Pi) grad W, since the
+//    momentum equation takes only the sums' totals and its rho_i / rho_i cancels; they
+//    collect in av_x, av_y;
+//  * mu and Pi with the factors 1/2 of the pair means folded into the constants, the
+//    records' stresses already times 1/rho^2 and their c times alpha / 2 (k_gather64).
+struct Row64 {
+	double h1, w_wdp, eta2q, half_beta, xs_c;
+	bool stress, art;
+};
+__device__ __forceinline__ void pair64_fast(uint32_t flags, const Row64& k, double corr_exp, const Rec64& ri,
+                                            const Rec64& rj, Acc64& s) {
+	const double xij = ri.x - rj.x, yij = ri.y - rj.y;
+	const double r2 = fma(yij, yij, xij * xij);
+	const bool apart = __double_as_longlong(r2) > __double_as_longlong(1e-24);  // kernel.cpp's r > 1e-12
+	const double sr = apart ? rsqrt64(r2) * k.h1 : 0.;  // 1 / (r h)
+	const double q = r2 * sr;
+	const double t = clamp0(2. - q), u = clamp0(1. - q);
+	const double u2 = u * u, t2q = 0.25 * t * t;
+	const double w = fma(t2q, t, -u2 * u);  // W / fac
+	const double g = (u2 - t2q) * sr;       // |grad W| / (3 fac r)
+	const double gx = xij * g, gy = yij * g;
+	const double dvx = rj.vx - ri.vx, dvy = rj.vy - ri.vy;
+	const double inv_rs = rcp64(ri.rho + rj.rho);
+	double piij = 0.;
+	if (flags & A_ART_VISC) {
+		const double dot = fma(dvy, yij, dvx * xij);  // -v_ij . x_ij
+		const bool approach = __double2hiint(dot) > 0;  // dot > 0 by its bits
+		const double hs = ri.h + rj.h;
+		const double D = approach ? fma(k.eta2q * hs, hs, r2) : 1.;
+		const double mu2 = hs * dot * rcp64(D);  // -2 mu_ij
+		const double p = mu2 * fma(k.half_beta, mu2, ri.c + rj.c) * inv_rs;
+		piij = approach ? p : 0.;
+	}
+	if (k.stress) {
+		double txx = ri.sxx + rj.sxx, txy = ri.sxy + rj.sxy, tyy = ri.syy + rj.syy;
+		if (k.art) {
+			double fab = w * k.w_wdp;
+			if (corr_exp == 4.) {
+				fab *= fab;
+				fab *= fab;
+			} else {
+				fab = pow(fab, corr_exp);
+			}
+			txx = fma(fab, ri.Rxx + rj.Rxx, txx);
+			txy = fma(fab, ri.Rxy + rj.Rxy, txy);
+			tyy = fma(fab, ri.Ryy + rj.Ryy, tyy);
+		}
+		const double mx = rj.m * gx, my = rj.m * gy;
+		s.av_x = fma(txx - piij, mx, fma(txy, my, s.av_x));
+		s.av_y = fma(txy, mx, fma(tyy - piij, my, s.av_y));
+	} else if (flags & A_ART_VISC) {
+		const double mp = rj.m * piij;
+		s.av_x = fma(-mp, gx, s.av_x);
+		s.av_y = fma(-mp, gy, s.av_y);
+	}
+	if (flags & A_DERIVE_VEL) {
+		const double qx = rj.qw * gx, qy = rj.qw * gy;
+		s.vx_x = fma(dvx, qx, s.vx_x);
+		s.vx_y = fma(dvx, qy, s.vx_y);
+		s.vy_x = fma(dvy, qx, s.vy_x);
+		s.vy_y = fma(dvy, qy, s.vy_y);
+	}
+	if (flags & A_XSPH) {
+		const double f = w * inv_rs;
+		s.xs_x = fma(f, dvx, s.xs_x);
+		s.xs_y = fma(f, dvy, s.xs_y);
+	}
+}
+#endif
+
+// The row's totals of N sums (N a multiple of its four lanes) into every lane: each lane
+// adds up a quarter of them, N / 2 + N / 4 additions where a butterfly per sum takes 2 N,
+// and reads the others' (the shuffles do not use the FP64 pipe).
+template <int N>
+__device__ __forceinline__ void row_sums64(double (&v)[N], uint32_t lane) {
+	double h[N / 2], t[N / 4];
+#pragma unroll
+	for (int i = 0; i < N / 2; i++) {
+		const double keep = (lane & 2u) ? v[N / 2 + i] : v[i], give = (lane & 2u) ? v[i] : v[N / 2 + i];
+		h[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+	}
+#pragma unroll
+	for (int i = 0; i < N / 4; i++) {
+		const double keep = (lane & 1u) ? h[N / 4 + i] : h[i], give = (lane & 1u) ? h[i] : h[N / 4 + i];
+		t[i] = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+	}
+#pragma unroll
+	for (int l = 0; l < 4; l++)
+#pragma unroll
+		for (int i = 0; i < N / 4; i++) v[(l >> 1) * (N / 2) + (l & 1) * (N / 4) + i] = __shfl_sync(0xffffffffu, t[i], l, P64_L);
+}
+
+// Every lane of a warp stays to the end (a row past the last, or of a failed body, lists
+// no pairs and writes nothing), so the shuffles take the whole warp.
+template <bool GOD>
+__global__ void __launch_bounds__(P64_THREADS) k_pair64(ULArgs a, const BodyParams* __restrict__ P,
+                                                        const Geom* __restrict__ G, DevStatus* st) {
+	__shared__ uint32_t s_list[P64_ROWS][P64_CAP + 1];  // (+ 1: rows start in different banks)
+	constexpr unsigned FULL = 0xffffffffu;
+	const uint32_t lane = threadIdx.x % P64_L;
+	const uint32_t k = (blockIdx.x * P64_THREADS + threadIdx.x) / P64_L;
+	const bool in_range = k < a.n_total;
+	const uint32_t kk = in_range ? k : a.n_total - 1;
+	uint32_t* list = s_list[threadIdx.x / P64_L];
+	const uint32_t b = a.rec_body[kk];
+	// the row's four lanes must agree on a word that other rows may set meanwhile
+	bool live = in_range && !is_failed(a.failed, b);
+	live = __shfl_sync(FULL, live, 0, P64_L);
+	const Rec64* rec = reinterpret_cast<const Rec64*>(a.rec);
+	const float4* pos = reinterpret_cast<const float4*>(a.pos);
+	const Rec64 ri = load_rec(rec + kk);
+	const float4 pi = __ldg(pos + kk);
+	const BodyParams& pr = P[b];
+	const Geom g = G[b];
+	const uint32_t i = a.perm[kk];
+	const uint32_t flags = a.flags;
+	int lo_i, hi_i, lo_j, hi_j;
+	stencil(g, a.keys_sorted[kk], lo_i, hi_i, lo_j, hi_j);
+	if (!live) hi_i = lo_i;
+	const uint32_t tot = *a.total_cells;
+
+	// the FP32 test's bands: beyond `far` a pair cannot contribute (q >= 2 gives exactly
+	// zero); below `sure_in` / above `sure_out` it is certainly within / beyond the
+	// reference's limit 4 h^2 + eps.  In FP32 from h's leading bits, out of the FP64 pipe's way.
+	const int he = __double2hiint(ri.h), eexp = ((__double2hiint(ri.h) >> 20) & 0x7ff) + 26;  // |x| < 2^26 h
+	const float hf = seed_f32(ri.h), limf = 4.f * hf * hf + a.nbh_eps_f;
+	const bool fp32 = he >= 0x3cd203af && he < 0x430c6bf5 /* 1e-15 <= h < 1e15 */ && limf < 1e30f && a.nbh_eps_f >= 0.f &&
+	                  ((__double2hiint(ri.x) >> 20) & 0x7ff) < eexp && ((__double2hiint(ri.y) >> 20) & 0x7ff) < eexp;
+	const float far = 4.f * hf * hf * 1.00002f, sure_in = limf * 0.99998f, sure_out = limf * 1.00002f;
+	Acc64 s;
+#if !MF_STRICT_FORM
+	Row64 rk;
+	rk.h1 = rcp64(ri.h);
+	const double fac = 10 * (K_1_PI) / 7.0 * rk.h1 * rk.h1;
+	rk.art = pr.wdeltap > 0;
+	rk.w_wdp = rk.art ? fac * rcp64(pr.wdeltap) : 0.;
+	rk.eta2q = 0.25 * pr.eta * pr.eta;
+	rk.half_beta = 0.5 * pr.beta;
+	rk.stress = (flags & A_MOMENTUM_UL) != 0;
+#endif
+	auto pairs = [&](uint32_t n) {
+		for (uint32_t e = lane; e < n; e += P64_L) {
+			const uint32_t kj = list[e];
+			const Rec64 rj = load_rec(rec + kj);
+#if MF_STRICT_FORM
+			pair64_ref<GOD>(flags, pr, ri, rj, s);
+#else
+			if (GOD) pair64_ref<GOD>(flags, pr, ri, rj, s);
+			else pair64_fast(flags, rk, pr.corr_exp, ri, rj, s);
+#endif
+		}
+	};
+	uint32_t cnt = 0, listed = 0;
+	const int cols = __reduce_max_sync(FULL, hi_i - lo_i);
+	for (int c = 0; c < cols; c++) {
+		uint32_t j0 = 0, j1 = 0;
+		if (lo_i + c < hi_i) {
+			const uint32_t row = g.cell_off + (uint32_t)(lo_i + c) * g.ny;
+			j0 = a.cell_start[min(row + (uint32_t)lo_j, tot)];
+			j1 = a.cell_start[min(row + (uint32_t)hi_j, tot)];
+		}
+		for (uint32_t base = j0; __any_sync(FULL, base < j1); base += 32) {
+			uint32_t mask = 0u;  // of the 32 candidates from base on, those to list
+#pragma unroll
+			for (uint32_t t = 0; t < 32; t += P64_L) {
+				const uint32_t kj = base + t + lane;
+				if (base >= j1 || kj >= j1) break;
+				const float4 pj = __ldg(pos + kj);
+				const float dx = (pi.x - pj.x) + (pi.y - pj.y), dy = (pi.z - pj.z) + (pi.w - pj.w);
+				const float r2 = dx * dx + dy * dy;
+				bool list_it = !(r2 > far), in = r2 <= sure_in;
+				if (!fp32 || !(in || r2 > sure_out)) {  // the reference's predicate decides
+					const double2 xy = __ldg(reinterpret_cast<const double2*>(rec + kj));
+					const double xij = __dsub_rn(ri.x, xy.x), yij = __dsub_rn(ri.y, xy.y);
+					const double d2 = __dadd_rn(__dmul_rn(xij, xij), __dmul_rn(yij, yij));
+					const double h2 = __dmul_rn(ri.h, ri.h);
+					in = d2 <= __dadd_rn(__dmul_rn(__dmul_rn(h2, 2.), 2.), a.nbh_eps);
+					if (!fp32) list_it = !(d2 > 4.0000001 * h2);
 				}
+				cnt += in ? 1u : 0u;
+				// (the row itself counts, but adds nothing to any sum)
+				if (list_it && kj != k) mask |= 1u << (t + lane);
+			}
+			uint32_t own = mask;
+#pragma unroll
+			for (uint32_t o = P64_L / 2; o > 0; o >>= 1) mask |= __shfl_xor_sync(FULL, mask, o);
+			while (own) {
+				const uint32_t bit = (uint32_t)__ffs(own) - 1u;
+				own &= own - 1u;
+				list[listed + __popc(mask & ((1u << bit) - 1u))] = base + bit;
+			}
+			listed += __popc(mask);
+			const bool full = listed > P64_CAP - 32;
+			if (__any_sync(FULL, full)) {  // a full row works its list off now (the others go on listing)
+				__syncwarp();
+				pairs(full ? listed : 0u);
+				if (full) listed = 0u;
+				__syncwarp();
 			}
 		}
 	}
-	if (a.max_nbh && cnt >= a.max_nbh) fail_body(a.failed, st, ERR_NBH_OVERFLOW, i, b);
-	if (cnt == 0) fail_body(a.failed, st, ERR_NO_NEIGHBOR, i, b);
+	__syncwarp();
+	pairs(listed);
+	for (uint32_t o = P64_L / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(FULL, cnt, o);
 
-	// per-particle actions, in the reference's list order
+	// per-particle actions, in the reference's list order; every lane of the row holds the
+	// totals, and lane q then updates the state components q and q + 4
 	double d[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
-	double rhoi = ri.rho;
-	if (flags & A_STRESS_MGHN) { Sxx_x *= rhoi; Sxy_y *= rhoi; Sxy_x *= rhoi; Syy_y *= rhoi; }
-	if (flags & A_ART_VISC) { d[2] = av_x; d[3] = av_y; }
-	if (flags & A_XSPH) { d[0] = xs_x; d[1] = xs_y; }
+	const double rhoi = ri.rho;
+#if MF_STRICT_FORM
+	constexpr bool SUMS = true;
+#else
+	constexpr bool SUMS = GOD;  // (pair64_fast adds the stress forces to av)
+#endif
+	constexpr int NS = GOD ? 16 : SUMS ? 12 : 8;
+	double v[NS] = {s.av_x, s.av_y, s.vx_x, s.vx_y, s.vy_x, s.vy_y, s.xs_x, s.xs_y};
+	if (SUMS) {
+		v[8 % NS] = s.Sxx_x; v[9 % NS] = s.Sxy_y; v[10 % NS] = s.Sxy_x; v[11 % NS] = s.Syy_y;
+	}
+	if (GOD) {
+		v[12 % NS] = s.god_rho; v[13 % NS] = s.god_vx; v[14 % NS] = s.god_vy; v[15 % NS] = 0.;
+	}
+	row_sums64<NS>(v, lane);
+	double vx_x = v[2], vx_y = v[3], vy_x = v[4], vy_y = v[5];
+#if !MF_STRICT_FORM
+	if (!GOD) {  // the factors that pair64_fast left out
+		const double gsc = 3. * fac, xsc = 2. * pr.xsph_eps * ri.m * fac;
+		v[0] *= gsc; v[1] *= gsc; v[6] *= xsc; v[7] *= xsc;
+		vx_x *= gsc; vx_y *= gsc; vy_x *= gsc; vy_y *= gsc;
+	}
+	const bool av = (flags & A_ART_VISC) || (!GOD && rk.stress);
+#else
+	const bool av = (flags & A_ART_VISC) != 0;
+#endif
+	if (av) { d[2] = v[0]; d[3] = v[1]; }
+	if (flags & A_XSPH) { d[0] = v[6]; d[1] = v[7]; }
 	if (flags & A_JAUMANN) {
 		// the Jaumann rate uses the stage stress itself (not S - p)
 		const mfk_host::StateSoA& sv = a.stage == 0 ? a.base : a.st;
+#if MF_STRICT_FORM
 		jaumann<double>(vx_x, vx_y, vy_x, vy_y, sv.Sxx[i], sv.Sxy[i], sv.Syy[i], pr.G, d[5], d[6], d[7]);
+#else
+		jaumann_plane(vx_x, vx_y, vy_x, vy_y, sv.Sxx[i], sv.Sxy[i], sv.Syy[i], pr.G, d[5], d[6], d[7]);
+#endif
 	}
 	if (flags & A_CONTINUITY) d[4] = -(rhoi * (vx_x + vy_y));
-	if (flags & A_GOD_CONT) d[4] = god_rho;
-	if (flags & A_GOD_MOM) {
-		d[2] += god_vx + a.fcx[i] / ri.m;
-		d[3] += god_vy + a.fcy[i] / ri.m;
+	if (GOD) {
+		if (flags & A_GOD_CONT) d[4] = v[12 % NS];
+		if (flags & A_GOD_MOM) {
+			d[2] += v[13 % NS] + a.fcx[i] / ri.m;
+			d[3] += v[14 % NS] + a.fcy[i] / ri.m;
+		}
 	}
 	if (flags & A_MOMENTUM_UL) {
-		d[2] += 1. / rhoi * (Sxx_x + Sxy_y) + a.fcx[i] / ri.m;
-		d[3] += 1. / rhoi * (Sxy_x + Syy_y) + a.fcy[i] / ri.m;
+#if MF_STRICT_FORM
+		const double fmx = a.fcx[i] / ri.m, fmy = a.fcy[i] / ri.m;
+#else
+		const double m1 = rcp64(ri.m), fmx = a.fcx[i] * m1, fmy = a.fcy[i] * m1;
+#endif
+		if (SUMS) {
+			d[2] += 1. / rhoi * (v[8 % NS] * rhoi + v[9 % NS] * rhoi) + fmx;
+			d[3] += 1. / rhoi * (v[10 % NS] * rhoi + v[11 % NS] * rhoi) + fmy;
+		} else {
+			d[2] += fmx;
+			d[3] += fmy;
+		}
 	}
 	if (flags & A_ADVECTION) { d[0] += ri.vx; d[1] += ri.vy; }
-	rk_update_f64<double>(a, i, pr.dt, d);
-	if (a.stage == 3 && !(isfinite(a.base.x[i]) && isfinite(a.base.y[i]) && isfinite(a.base.vx[i]) &&
-	                      isfinite(a.base.vy[i]) && isfinite(a.base.rho[i])))
-		fail_body(a.failed, st, ERR_NONFINITE, i, b);
+	if (!live) return;
+	if (lane == 0) {
+		if (a.max_nbh && cnt >= a.max_nbh) fail_body(a.failed, st, ERR_NBH_OVERFLOW, i, b);
+		if (cnt == 0) fail_body(a.failed, st, ERR_NO_NEIGHBOR, i, b);
+	}
+	// rk4.h:52-69 (stage state = particles + c*dt*derivative) and :94-103 (final combine
+	// with weights 1,2,2,1 / 6); d[] = x_t, y_t, vx_t, vy_t, rho_t, Sxx_t, Sxy_t, Syy_t
+	double* bp[8] = {a.base.x, a.base.y, a.base.vx, a.base.vy, a.base.rho, a.base.Sxx, a.base.Sxy, a.base.Syy};
+	double* ap[8] = {a.acc.x, a.acc.y, a.acc.vx, a.acc.vy, a.acc.rho, a.acc.Sxx, a.acc.Sxy, a.acc.Syy};
+	double* sp[8] = {a.st.x, a.st.y, a.st.vx, a.st.vy, a.st.rho, a.st.Sxx, a.st.Sxy, a.st.Syy};
+	const double dt = pr.dt;
+	bool ok = true;
+#pragma unroll
+	for (uint32_t half = 0; half < 2; half++) {
+		double dq = d[4 * half];
+		double *B = bp[4 * half], *A = ap[4 * half], *S = sp[4 * half];
+#pragma unroll
+		for (uint32_t q = 1; q < 4; q++)
+			if (lane == q) { dq = d[4 * half + q]; B = bp[4 * half + q]; A = ap[4 * half + q]; S = sp[4 * half + q]; }
+		if (a.stage < 3) {
+			const double dts = (a.stage == 2 ? 1.0 : 0.5) * dt;
+			A[i] = (a.stage == 0) ? dq : A[i] + 2 * dq;
+			S[i] = B[i] + dq * dts;
+		} else {
+			const double w6 = dt * 1. / 6.;
+			const double v = B[i] + w6 * (A[i] + dq);
+			B[i] = v;
+			if (half == 0 || lane == 0) ok = ok && isfinite(v);  // x, y, vx, vy, rho
+		}
+	}
+	if (!ok) fail_body(a.failed, st, ERR_NONFINITE, i, b);
 }
 
 // ---------------------------------------------------------- pair kernel mixed
@@ -954,18 +1229,17 @@ __global__ void __launch_bounds__(256, 3) k_pair_split(ULArgs a, const BodyParam
 	pair32_row<GOD, L>(a, P, G, st, k, t % L);
 }
 
-// The pair kernels.  Plain form: one thread per cell-ordered row.  Persistent form
+// The mixed pair kernel.  Plain form: one thread per cell-ordered row.  Persistent form
 // (one launch per stage over all bodies): a fixed grid whose blocks take chunks of
 // rows -- consecutive cell-ordered rows, so a chunk is a run of cells of one body --
 // from an atomic counter until the rows run out; no block ever waits on another.
-template <bool MIXED, bool GOD = false>
-__global__ void __launch_bounds__(256, MIXED ? 3 : 1) k_pair(ULArgs a, const BodyParams* __restrict__ P, const Geom* __restrict__ G,
-                                              DevStatus* st) {
+template <bool GOD>
+__global__ void __launch_bounds__(256, 3) k_pair(ULArgs a, const BodyParams* __restrict__ P, const Geom* __restrict__ G,
+                                                 DevStatus* st) {
 	if (!a.persistent) {
 		uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
 		if (k >= a.n_total) return;
-		if (MIXED) pair32_row<GOD>(a, P, G, st, k);
-		else pair64_row(a, P, G, st, k);
+		pair32_row<GOD>(a, P, G, st, k);
 		return;
 	}
 	__shared__ uint32_t s_chunk;
@@ -978,10 +1252,7 @@ __global__ void __launch_bounds__(256, MIXED ? 3 : 1) k_pair(ULArgs a, const Bod
 		if (base >= a.n_total) break;
 		for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) {
 			uint64_t k = base + r;
-			if (k < a.n_total) {
-				if (MIXED) pair32_row<GOD>(a, P, G, st, (uint32_t)k);
-				else pair64_row(a, P, G, st, (uint32_t)k);
-			}
+			if (k < a.n_total) pair32_row<GOD>(a, P, G, st, (uint32_t)k);
 		}
 	}
 }
@@ -1065,7 +1336,7 @@ cudaError_t ul_stage(const ULArgs& a, bool mixed, cudaStream_t s) {
 	}
 	unsigned bs = a.block ? a.block : 128;
 	unsigned grid = a.persistent ? a.grid : grid1(a.n_total, bs);
-	if (a.persistent) {
+	if (mixed && a.persistent) {
 		cudaError_t e = cudaMemsetAsync(a.work, 0, sizeof(uint32_t), s);
 		if (e != cudaSuccess) return e;
 	}
@@ -1081,11 +1352,13 @@ cudaError_t ul_stage(const ULArgs& a, bool mixed, cudaStream_t s) {
 			else k_pair_split<false, 8><<<g2, bs, 0, s>>>(a, a.params, a.geom, st);
 		}
 	} else if (mixed && god) {
-		k_pair<true, true><<<grid, bs, 0, s>>>(a, a.params, a.geom, st);
-	} else if (mixed) {
 		k_pair<true><<<grid, bs, 0, s>>>(a, a.params, a.geom, st);
-	} else {
+	} else if (mixed) {
 		k_pair<false><<<grid, bs, 0, s>>>(a, a.params, a.geom, st);
+	} else {
+		const unsigned g64 = grid1(a.n_total, P64_ROWS);
+		if (god) k_pair64<true><<<g64, P64_THREADS, 0, s>>>(a, a.params, a.geom, st);
+		else k_pair64<false><<<g64, P64_THREADS, 0, s>>>(a, a.params, a.geom, st);
 	}
 	if (a.ev_pair1) cudaEventRecord(a.ev_pair1, s);
 	return cudaGetLastError();
