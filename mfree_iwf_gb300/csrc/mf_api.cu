@@ -245,7 +245,7 @@ struct mf_ctx {
 	DevBuf<uint32_t> nbr_off, nbr, bc_rows, sl_off, snbr;
 	DevBuf<uint16_t> scnt;
 	DevBuf<double> wx64, wy64, P64, dA64, c64, bc_v;
-	DevBuf<double2> sw64;
+	DevBuf<double2> sw64, swA64, w_sum64;
 	DevBuf<float2> sw32, swA32;
 	// mixed TL halo tiles (TLArgs::t_*)
 	DevBuf<uint32_t> tt_rows, tt_halo_off, tt_halo, tt_sl;
@@ -944,7 +944,8 @@ TLArgs tl_args(mf_ctx* c) {
 	a.cnt = c->scnt.p;
 	a.snbr = c->snbr.p;
 	a.sw = c->mixed ? (const void*)c->sw32.p : (const void*)c->sw64.p;
-	a.swA = c->swA32.p;
+	a.swA = c->mixed ? (const void*)c->swA32.p : (const void*)c->swA64.p;
+	a.w_sum = c->w_sum64.p;
 	a.P = c->P64.p;
 	a.dA = c->dA64.p;
 	a.c = c->c64.p;
@@ -1265,11 +1266,15 @@ mf_status tl_setup(mf_ctx* c) {
 		CK(c->swA32.alloc(ent));
 	} else {
 		CK(c->sw64.alloc(ent));
+		if (!c->strict && !fam) {  // the fast FP64 passes' weights
+			CK(c->swA64.alloc(ent));
+			CK(c->w_sum64.alloc(n));
+		}
 	}
 	e = c->strict ? mf_strict::tl_to_sell(n, c->nbr_off.p, c->nbr.p, c->wx64.p, c->wy64.p, c->sl_off.p, c->scnt.p,
-	                                      c->snbr.p, c->sw64.p, nullptr, nullptr, c->qw0.p, c->m.p, c->stream)
+	                                      c->snbr.p, c->sw64.p, nullptr, nullptr, nullptr, nullptr, c->qw0.p, c->m.p, c->stream)
 	              : mf_fast::tl_to_sell(n, c->nbr_off.p, c->nbr.p, c->wx64.p, c->wy64.p, c->sl_off.p, c->scnt.p,
-	                                    c->snbr.p, tl_mixed_lists ? nullptr : (void*)c->sw64.p,
+	                                    c->snbr.p, tl_mixed_lists ? nullptr : (void*)c->sw64.p, c->swA64.p, c->w_sum64.p,
 	                                    tl_mixed_lists ? (void*)c->sw32.p : nullptr,
 	                                    tl_mixed_lists ? (void*)c->swA32.p : nullptr, c->qw0.p, c->m.p, c->stream);
 	if (e != cudaSuccess) return cuda_fail(c, e, "tl_to_sell");
@@ -2319,7 +2324,7 @@ mf_ctx::~mf_ctx() {
 			for (int q = 0; q < 4; q++) { gsd[k][q].free(); gsf[k][q].free(); }
 		g_w64.free(); t_w64.free(); p_w64.free(); g_w32.free(); t_w32.free(); p_w32.free();
 	}
-	sl_off.free(); snbr.free(); scnt.free(); sw64.free(); sw32.free(); swA32.free(); recA.free(); recB.free(); dA32.free();
+	sl_off.free(); snbr.free(); scnt.free(); sw64.free(); swA64.free(); w_sum64.free(); sw32.free(); swA32.free(); recA.free(); recB.free(); dA32.free();
 	recB2.free(); sW64.free(); R64.free(); av64.free();
 	cm_sw.free(); cm_swA.free(); cm_sX.free(); cm_swji.free(); cm_sW.free();
 	cm_U.free(); cm_X.free(); cm_V.free(); cm_P.free(); cm_R.free(); cm_H.free();

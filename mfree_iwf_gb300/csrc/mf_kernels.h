@@ -139,8 +139,9 @@ struct TLArgs {
 	const uint32_t* sl_off;
 	const uint16_t* cnt;
 	const uint32_t* snbr;
-	const void* sw;                      // corrected gradient per pair: double2 (FP64 forms) / float2 times m_j (mixed)
-	const void* swA;                     // mixed: the gradient times the neighbour's quad weight (pass A)
+	const void* sw;                      // corrected gradient per pair: double2 (FP64; the fast TL form times m_j) / float2 times m_j (mixed)
+	const void* swA;                     // mixed and fast FP64 TL: the gradient times the neighbour's quad weight (pass A)
+	const void* w_sum;                   // fast FP64 TL: per row the sum of sw (double2)
 	void *P, *dA, *c;                    // per-stage scratch (FP64 forms)
 	const void* sW;                      // corotational: kernel value W per pair (double, sliced ELL);
 	                                     // potential: grad W of the reverse pair (double2, sliced ELL)
@@ -294,8 +295,8 @@ struct ContactArgs {
 	cudaError_t tl_ref_positions(uint32_t n, const double* X, const double* Y, void* XF, cudaStream_t s);     \
 	cudaError_t to_float(uint64_t n, const double* a, float* b, cudaStream_t s);                             \
 	cudaError_t tl_to_sell(uint32_t n, const uint32_t* off, const uint32_t* nbr, const double* wx, const double* wy, \
-	                       const uint32_t* sl_off, uint16_t* cnt, uint32_t* snbr, void* sw64, void* sw32,     \
-	                       void* swA32, const double* qw, const double* mass, cudaStream_t s);                \
+	                       const uint32_t* sl_off, uint16_t* cnt, uint32_t* snbr, void* sw64, void* swA64,    \
+	                       void* w_sum, void* sw32, void* swA32, const double* qw, const double* mass, cudaStream_t s);     \
 	cudaError_t tl_stage(const mfk_host::TLArgs& a, bool mixed, int part, cudaStream_t s);                   \
 	cudaError_t tl_tile_sell(uint32_t n, const uint32_t* t_rows, const uint32_t* sl_off, const uint16_t* cnt, \
 	                         const void* sw, const void* swA, const uint32_t* t_sl, uint16_t* t_cnt, void* t_sw, \

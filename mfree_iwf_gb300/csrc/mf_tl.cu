@@ -195,7 +195,8 @@ __global__ void k_tl_bc(TLArgs a, int on_base) {
 	s.vy[i] = 0.;
 }
 
-// The per-particle part of pass A, shared by both forms (T = double).
+#if MF_STRICT_FORM
+// The per-particle part of the FP64 pass A in the reference's expressions.
 __device__ __forceinline__ void tl_particle(uint32_t flags, const BodyParams& pr, double Hxx, double Hxy, double Hyx,
                                             double Hyy, double Fxx, double Fxy, double Fyx, double Fyy, double rho,
                                             double Sxx, double Sxy, double Syy, double& Pxx, double& Pxy, double& Pyx,
@@ -212,6 +213,7 @@ __device__ __forceinline__ void tl_particle(uint32_t flags, const BodyParams& pr
 	Pxx = Pxy = Pyx = Pyy = 0.;
 	if (flags & A_C2N) cauchy_to_nominal<double>(Hxx, Hxy, Hyx, Hyy, Sxx - p, Sxy, Syy - p, Pxx, Pxy, Pyx, Pyy);
 }
+#endif
 
 // The per-row part of the mixed pass A in FP32.  GB300 issues FP64 at a small fraction
 // of its FP32 rate, and in FP64 this part kept the FP64 pipe ~70 % busy, the pass's
@@ -239,7 +241,183 @@ __device__ __forceinline__ void tl_particle32(uint32_t flags, const BodyParams& 
 // consecutive slots, so every per-pair load of the warp is one coalesced request.
 __device__ __forceinline__ uint32_t sell_base(const TLArgs& a, uint32_t i) { return a.sl_off[i >> 5] + (i & 31u); }
 
-// ---- FP64 pass A
+// RK4 update of row i (rk4.h:52-108) from its rates d[]; the next stage's state goes to
+// the other stage set.
+__device__ __forceinline__ void tlB_rk64(const TLArgs& a, uint32_t i, double dt, const double d[8]) {
+	double* bp[8] = {a.base.x, a.base.y, a.base.vx, a.base.vy, a.base.rho, a.base.Sxx, a.base.Sxy, a.base.Syy};
+	double* ap[8] = {a.acc.x, a.acc.y, a.acc.vx, a.acc.vy, a.acc.rho, a.acc.Sxx, a.acc.Sxy, a.acc.Syy};
+	double* np[8] = {a.nxt.x, a.nxt.y, a.nxt.vx, a.nxt.vy, a.nxt.rho, a.nxt.Sxx, a.nxt.Sxy, a.nxt.Syy};
+	uint32_t stg = a.stage;
+	if (stg < 3) {
+		double dts = (stg == 2 ? 1.0 : 0.5) * dt;
+#pragma unroll
+		for (int q2 = 0; q2 < 8; q2++) {
+			ap[q2][i] = (stg == 0) ? d[q2] : ap[q2][i] + 2 * d[q2];
+			np[q2][i] = bp[q2][i] + d[q2] * dts;  // the next stage state (ping-pong set)
+		}
+	} else {
+		double w6 = dt * 1. / 6.;
+#pragma unroll
+		for (int q2 = 0; q2 < 8; q2++) {
+			double v = bp[q2][i] + w6 * (ap[q2][i] + d[q2]);
+			bp[q2][i] = v;
+			np[q2][i] = v;  // the next step's first stage starts from a copy of the particles
+		}
+		if (!(isfinite(bp[0][i]) && isfinite(bp[1][i]) && isfinite(bp[2][i]) && isfinite(bp[3][i])))
+			raise(reinterpret_cast<DevStatus*>(a.status), ERR_NONFINITE, i);
+	}
+}
+
+// ---- FP64 passes, fast form.  GB300's FP64 pipe (2 lanes a clock and SM) bounds both,
+// so they are written for few FP64 instructions: per-pair weights already times the
+// neighbour's quad weight (pass A) and mass (pass B), P as the adjugate of F times sigma
+// (no inverse), Green-St Venant from H, stress and viscosity in one gradient sum,
+// reciprocals by rcp64.  Ring impact at dx = 0.1 mm (439,860 rows), per launch: pass A
+// 268 -> 191 us, pass B 901 -> 422 us (FP64 pipe 86-88 % busy in both).
+#if !MF_STRICT_FORM
+// The per-particle part of pass A (tl_particle) in fewer instructions.
+__device__ __forceinline__ void tl_particle_fast(uint32_t flags, const BodyParams& pr, double Hxx, double Hxy,
+                                                 double Hyx, double Hyy, double Fxx, double Fxy, double Fyx, double Fyy,
+                                                 double rho, double Sxx, double Sxy, double Syy, double P[4],
+                                                 double dA[4]) {
+	const double a = 1. + Hxx, b = Hxy, c = Hyx, d = 1. + Hyy;  // F = (a b; c d)
+	const double J = a * d - b * c;
+	double vx_x = 0., vx_y = 0., vy_x = 0., vy_y = 0.;
+	if (flags & A_VGRAD_TL) {  // Fdot F^-1
+		const double iJ = rcp64(J);
+		vx_x = (Fxx * d - Fxy * c) * iJ;
+		vx_y = (Fxy * a - Fxx * b) * iJ;
+		vy_x = (Fyx * d - Fyy * c) * iJ;
+		vy_y = (Fyy * a - Fyx * b) * iJ;
+	}
+	dA[0] = dA[1] = dA[2] = dA[3] = 0.;
+	if (flags & A_CONTINUITY) dA[0] = -(rho * (vx_x + vy_y));
+	const double p = (flags & A_EOS) ? pr.c0sq * (rho - pr.rho0) : 0.;
+	if (flags & A_JAUMANN) jaumann_plane(vx_x, vx_y, vy_x, vy_y, Sxx, Sxy, Syy, pr.G, dA[1], dA[2], dA[3]);
+	if (flags & A_GREEN) green_stvenant_h<double>(Hxx, Hxy, Hyx, Hyy, pr.D, pr.nu, Sxx, Sxy, Syy);
+	P[0] = P[1] = P[2] = P[3] = 0.;
+	if (flags & A_C2N) {  // J F^-1 sigma = adj(F) sigma (a singular F is not finite, as with the inverse)
+		const double sxx = Sxx - p, syy = Syy - p;
+		const bool singular = J == 0.;
+		const double bad = __longlong_as_double(0x7ff8000000000000ll);
+		P[0] = singular ? bad : d * sxx - b * Sxy;
+		P[1] = singular ? bad : d * Sxy - b * syy;
+		P[2] = singular ? bad : a * Sxy - c * sxx;
+		P[3] = singular ? bad : a * syy - c * Sxy;
+	}
+}
+
+__global__ void __launch_bounds__(256) k_tlA64(TLArgs a) {
+	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= a.n_total) return;
+	const mfk_host::StateSoA& s = a.st;
+	const double2* swA = (const double2*)a.swA;  // gradient times the neighbour's quad weight
+	const uint32_t flags = a.flags;
+	const double uxi = s.x[i] - a.X[i], uyi = s.y[i] - a.Y[i];
+	const double vxi = s.vx[i], vyi = s.vy[i];
+	double Hxx = 0., Hxy = 0., Hyx = 0., Hyy = 0.;
+	double Fxx = 0., Fxy = 0., Fyx = 0., Fyy = 0.;
+	uint32_t q = sell_base(a, i), c = a.cnt[i];
+#pragma unroll 2
+	for (uint32_t k = 0; k < c; k++, q += 32) {
+		const uint32_t j = a.snbr[q];
+		const double2 w = swA[q];
+		if (flags & A_DISP) {
+			const double ux = (s.x[j] - a.X[j]) - uxi, uy = (s.y[j] - a.Y[j]) - uyi;
+			Hxx = fma(ux, w.x, Hxx);
+			Hxy = fma(ux, w.y, Hxy);
+			Hyx = fma(uy, w.x, Hyx);
+			Hyy = fma(uy, w.y, Hyy);
+		}
+		if (flags & A_VEL_TL) {
+			const double vx = s.vx[j] - vxi, vy = s.vy[j] - vyi;
+			Fxx = fma(vx, w.x, Fxx);
+			Fxy = fma(vx, w.y, Fxy);
+			Fyx = fma(vy, w.x, Fyx);
+			Fyy = fma(vy, w.y, Fyy);
+		}
+	}
+	const BodyParams& pr = a.params[a.body_of[i]];
+	const double rho = s.rho[i];
+	double P[4], dA[4];
+	tl_particle_fast(flags, pr, Hxx, Hxy, Hyx, Hyy, Fxx, Fxy, Fyx, Fyy, rho, s.Sxx[i], s.Sxy[i], s.Syy[i], P, dA);
+	const size_t n = a.n_total;
+#pragma unroll
+	for (int k = 0; k < 4; k++) {
+		((double*)a.P)[k * n + i] = P[k];
+		((double*)a.dA)[k * n + i] = dA[k];
+	}
+	// the sound speed in pass B's units: times alpha / 2 rho0^2 (its viscosity constants)
+	if (flags & A_ART_VISC) ((double*)a.c)[i] = sqrt(pr.K * rcp64(rho)) * (0.5 * pr.alpha * pr.rho0 * pr.rho0);
+}
+
+__global__ void __launch_bounds__(256) k_tlB64(TLArgs a) {
+	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= a.n_total) return;
+	const mfk_host::StateSoA& s = a.st;
+	const double2* sw = (const double2*)a.sw;  // gradient times the neighbour's mass
+	const double* P = (const double*)a.P;
+	const double* cc = (const double*)a.c;
+	const size_t n = a.n_total;
+	const uint32_t flags = a.flags;
+	const BodyParams& pr = a.params[a.body_of[i]];
+	const bool stress = (flags & A_STRESS_TL) && (flags & A_MOMENTUM_TL);
+	const double xi = s.x[i], yi = s.y[i], vxi = s.vx[i], vyi = s.vy[i], hi = a.h[i], rhoi = s.rho[i];
+	const double rho02 = pr.rho0 * pr.rho0;
+	const double half_beta = 0.5 * pr.beta * rho02, eta2q = 0.25 * pr.eta * pr.eta;
+	const double ci = (flags & A_ART_VISC) ? cc[i] : 0.;
+	// sums of (P_i + P_j - rho0^2 Pi_ij I) times m_j grad w: the stress forces and the
+	// viscosity together, rho0^2 the common scale; P_i's share by the row's weight sum
+	double ax = 0., ay = 0.;
+	if (stress) {
+		const double2 ws = ((const double2*)a.w_sum)[i];
+		ax = fma(P[i], ws.x, P[2 * n + i] * ws.y);
+		ay = fma(P[n + i], ws.x, P[3 * n + i] * ws.y);
+	}
+	uint32_t q = sell_base(a, i), c = a.cnt[i];
+	for (uint32_t k = 0; k < c; k++, q += 32) {
+		const uint32_t j = a.snbr[q];
+		const double2 w = sw[q];
+		double pi2 = 0.;  // rho0^2 Pi_ij
+		if (flags & A_ART_VISC) {
+			const double dvx = s.vx[j] - vxi, dvy = s.vy[j] - vyi;
+			const double xij = xi - s.x[j], yij = yi - s.y[j];
+			const double dot = fma(dvy, yij, dvx * xij);  // -v_ij . x_ij
+			if (__double2hiint(dot) > 0) {  // approaching (dot > 0 by its bits)
+				// with n = 2 h_ij dot, D = r^2 + eta^2 h_ij^2, rs = rho_i + rho_j and
+				// A = 1 / (D rs): Pi = n A (alpha c_ij + beta / 2 n A rs)
+				const double hs = hi + a.h[j], rs = rhoi + s.rho[j];
+				const double D = fma(eta2q * hs, hs, fma(yij, yij, xij * xij));
+				const double nA = hs * dot * rcp64(D * rs);
+				pi2 = nA * fma(half_beta * rs, nA, ci + cc[j]);
+			}
+		}
+		if (stress) {
+			ax = fma(P[j] - pi2, w.x, fma(P[2 * n + j], w.y, ax));
+			ay = fma(P[n + j], w.x, fma(P[3 * n + j] - pi2, w.y, ay));
+		} else {
+			ax = fma(-pi2, w.x, ax);
+			ay = fma(-pi2, w.y, ay);
+		}
+	}
+	const double* dA = (const double*)a.dA;
+	const double r21 = rcp64(rho02);
+	double d[8];
+	d[0] = (flags & A_ADVECTION) ? vxi : 0.;
+	d[1] = (flags & A_ADVECTION) ? vyi : 0.;
+	d[2] = ax * r21;
+	d[3] = ay * r21;
+	if (flags & A_MOMENTUM_TL) {
+		const double m1 = rcp64(a.m[i]);
+		d[2] = fma(a.fcx[i], m1, d[2]);
+		d[3] = fma(a.fcy[i], m1, d[3]);
+	}
+	d[4] = dA[i]; d[5] = dA[n + i]; d[6] = dA[2 * n + i]; d[7] = dA[3 * n + i];
+	tlB_rk64(a, i, pr.dt, d);
+}
+
+#else
+// ---- FP64 pass A, parity form
 __global__ void __launch_bounds__(256) k_tlA64(TLArgs a) {
 	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= a.n_total) return;
@@ -283,7 +461,7 @@ __global__ void __launch_bounds__(256) k_tlA64(TLArgs a) {
 	((double*)a.c)[i] = sqrt(pr.K / rho);
 }
 
-// ---- FP64 pass B + RK update
+// ---- FP64 pass B + RK update, parity form
 __global__ void __launch_bounds__(256) k_tlB64(TLArgs a) {
 	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= a.n_total) return;
@@ -338,30 +516,9 @@ __global__ void __launch_bounds__(256) k_tlB64(TLArgs a) {
 		d[3] += 1. / rho0 * (Pxy_x + Pyy_y) + a.fcy[i] / a.m[i];
 	}
 	d[4] = dA[i]; d[5] = dA[n + i]; d[6] = dA[2 * n + i]; d[7] = dA[3 * n + i];
-	double* bp[8] = {a.base.x, a.base.y, a.base.vx, a.base.vy, a.base.rho, a.base.Sxx, a.base.Sxy, a.base.Syy};
-	double* ap[8] = {a.acc.x, a.acc.y, a.acc.vx, a.acc.vy, a.acc.rho, a.acc.Sxx, a.acc.Sxy, a.acc.Syy};
-	double* np[8] = {a.nxt.x, a.nxt.y, a.nxt.vx, a.nxt.vy, a.nxt.rho, a.nxt.Sxx, a.nxt.Sxy, a.nxt.Syy};
-	uint32_t stg = a.stage;
-	double dt = pr.dt;
-	if (stg < 3) {
-		double dts = (stg == 2 ? 1.0 : 0.5) * dt;
-#pragma unroll
-		for (int q2 = 0; q2 < 8; q2++) {
-			ap[q2][i] = (stg == 0) ? d[q2] : ap[q2][i] + 2 * d[q2];
-			np[q2][i] = bp[q2][i] + d[q2] * dts;  // the next stage state (ping-pong set)
-		}
-	} else {
-		double w6 = dt * 1. / 6.;
-#pragma unroll
-		for (int q2 = 0; q2 < 8; q2++) {
-			double v = bp[q2][i] + w6 * (ap[q2][i] + d[q2]);
-			bp[q2][i] = v;
-			np[q2][i] = v;  // the next step's first stage starts from a copy of the particles
-		}
-		if (!(isfinite(bp[0][i]) && isfinite(bp[1][i]) && isfinite(bp[2][i]) && isfinite(bp[3][i])))
-			raise(reinterpret_cast<DevStatus*>(a.status), ERR_NONFINITE, i);
-	}
+	tlB_rk64(a, i, pr.dt, d);
 }
+#endif
 
 // ---- mixed form
 // recA[i] = displacement u = x - X as float-float (16 B).
@@ -948,25 +1105,40 @@ __global__ void k_tile_sell(uint32_t n, const uint32_t* __restrict__ t_rows, con
 }
 
 // CSR (set-up order) -> sliced ELL; the mixed form gets FP32 gradients pre-multiplied
-// by the neighbour's mass (pass B) and by its quad weight (pass A), in FP64 then rounded.
+// by the neighbour's mass (pass B) and by its quad weight (pass A), in FP64 then rounded;
+// with swA64 (the fast FP64 form) the FP64 gradients are pre-multiplied alike, pairs whose
+// gradient is zero (the row itself, pairs beyond 2h) are left out, and w_sum receives the
+// row's sum of sw64.
 __global__ void k_to_sell(uint32_t n, const uint32_t* __restrict__ off, const uint32_t* __restrict__ nbr,
                           const double* __restrict__ wx, const double* __restrict__ wy, const uint32_t* __restrict__ sl_off,
-                          uint16_t* cnt, uint32_t* snbr, double2* sw64, float2* sw32, float2* swA32,
-                          const double* __restrict__ qw, const double* __restrict__ mass) {
+                          uint16_t* cnt, uint32_t* snbr, double2* sw64, double2* swA64, double2* w_sum,
+                          float2* sw32, float2* swA32, const double* __restrict__ qw, const double* __restrict__ mass) {
 	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	uint32_t base = sl_off[i >> 5] + (i & 31u);
 	uint32_t q0 = off[i], c = off[i + 1] - q0;
-	cnt[i] = (uint16_t)c;
+	double2 ws = make_double2(0., 0.);
+	uint32_t kept = 0;
 	for (uint32_t k = 0; k < c; k++) {
-		uint32_t q = base + 32 * k;
+		uint32_t q = base + 32 * kept;
 		uint32_t j = nbr[q0 + k];
-		snbr[q] = j;
 		double gx = wx[q0 + k], gy = wy[q0 + k];
-		if (sw64) sw64[q] = make_double2(gx, gy);
+		if (swA64 && gx == 0. && gy == 0.) continue;
+		kept++;
+		snbr[q] = j;
+		if (swA64) {
+			sw64[q] = make_double2(gx * mass[j], gy * mass[j]);
+			swA64[q] = make_double2(gx * qw[j], gy * qw[j]);
+			ws.x += sw64[q].x;
+			ws.y += sw64[q].y;
+		} else if (sw64) {
+			sw64[q] = make_double2(gx, gy);
+		}
 		if (sw32) sw32[q] = make_float2((float)(gx * mass[j]), (float)(gy * mass[j]));
 		if (swA32) swA32[q] = make_float2((float)(gx * qw[j]), (float)(gy * qw[j]));
 	}
+	cnt[i] = (uint16_t)kept;
+	if (w_sum) w_sum[i] = ws;
 }
 
 __global__ void k_advance_time(uint32_t nb, BodyParams* P) {
@@ -1016,10 +1188,10 @@ cudaError_t to_float(uint64_t n, const double* a, float* b, cudaStream_t s) {
 }
 
 cudaError_t tl_to_sell(uint32_t n, const uint32_t* off, const uint32_t* nbr, const double* wx, const double* wy,
-                       const uint32_t* sl_off, uint16_t* cnt, uint32_t* snbr, void* sw64, void* sw32, void* swA32,
+                       const uint32_t* sl_off, uint16_t* cnt, uint32_t* snbr, void* sw64, void* swA64, void* w_sum, void* sw32, void* swA32,
                        const double* qw, const double* mass, cudaStream_t s) {
-	k_to_sell<<<grid1(n, 128), 128, 0, s>>>(n, off, nbr, wx, wy, sl_off, cnt, snbr, (double2*)sw64, (float2*)sw32,
-	                                        (float2*)swA32, qw, mass);
+	k_to_sell<<<grid1(n, 128), 128, 0, s>>>(n, off, nbr, wx, wy, sl_off, cnt, snbr, (double2*)sw64, (double2*)swA64,
+	                                        (double2*)w_sum, (float2*)sw32, (float2*)swA32, qw, mass);
 	return cudaGetLastError();
 }
 
