@@ -1724,6 +1724,7 @@ mf_status weak_setup(mf_ctx* c) {
 		CK(c->wpack.alloc(2 * (size_t)n));
 	} else {
 		CK(c->gP64.alloc(4 * (size_t)ng));
+		if (!c->strict) CK(c->wpack.alloc(2 * (size_t)n));  // fast FP64: u and v as double2 pairs
 	}
 	// particles: stage 0 starts from a copy of the particles (set 2)
 	for (int q = 0; q < 8; q++) {
@@ -1784,7 +1785,7 @@ mf_status weak_step(mf_ctx* c) {
 		timing_begin(c, 2, slot);
 		if ((e = launch(3)) != cudaSuccess) return cuda_fail(c, e, "weak particle pass");
 		timing_end(c, slot, c->n_total);
-		c->launches += 2 + (c->n_bc ? 1 : 0) + (c->mixed ? 1 : 0);
+		c->launches += 2 + (c->n_bc ? 1 : 0) + (c->strict ? 0 : 1);
 	}
 	if ((e = launch(6)) != cudaSuccess || (e = launch(4)) != cudaSuccess) return cuda_fail(c, e, "weak step end");
 	c->launches += 1 + (c->n_bc ? 1 : 0);

@@ -291,6 +291,44 @@ MF_DEV void velocity_gradient_tl(T Hxx, T Hxy, T Hyx, T Hyy, T Fxx, T Fxy, T Fyx
 	vy_y = L.c[1][1];
 }
 
+// The total-Lagrangian per-point part (velocity gradient L = Fdot F^-1, continuity, EOS,
+// Jaumann rate, Green-St Venant, P = J F^-1 sigma) for the fast FP64 forms, in few FP64
+// instructions: P as the adjugate of F times sigma (no inverse), Green-St Venant from H,
+// one reciprocal for L.
+struct PointTerms {
+	bool vgrad, cont, eos, jaumann, green, nominal;
+};
+template <class Params>
+MF_DEV void tl_point_fast(PointTerms f, const Params& pr, double Hxx, double Hxy, double Hyx, double Hyy, double Fxx,
+                          double Fxy, double Fyx, double Fyy, double rho, double Sxx, double Sxy, double Syy,
+                          double P[4], double dA[4]) {
+	const double a = 1. + Hxx, b = Hxy, c = Hyx, d = 1. + Hyy;  // F = (a b; c d)
+	const double J = a * d - b * c;
+	double vx_x = 0., vx_y = 0., vy_x = 0., vy_y = 0.;
+	if (f.vgrad) {
+		const double iJ = rcp64(J);
+		vx_x = (Fxx * d - Fxy * c) * iJ;
+		vx_y = (Fxy * a - Fxx * b) * iJ;
+		vy_x = (Fyx * d - Fyy * c) * iJ;
+		vy_y = (Fyy * a - Fyx * b) * iJ;
+	}
+	dA[0] = dA[1] = dA[2] = dA[3] = 0.;
+	if (f.cont) dA[0] = -(rho * (vx_x + vy_y));
+	const double p = f.eos ? pr.c0sq * (rho - pr.rho0) : 0.;
+	if (f.jaumann) jaumann_plane(vx_x, vx_y, vy_x, vy_y, Sxx, Sxy, Syy, pr.G, dA[1], dA[2], dA[3]);
+	if (f.green) green_stvenant_h<double>(Hxx, Hxy, Hyx, Hyy, pr.D, pr.nu, Sxx, Sxy, Syy);
+	P[0] = P[1] = P[2] = P[3] = 0.;
+	if (f.nominal) {  // (a singular F is not finite, as with the inverse)
+		const double sxx = Sxx - p, syy = Syy - p;
+		const bool singular = J == 0.;
+		const double bad = __longlong_as_double(0x7ff8000000000000ll);
+		P[0] = singular ? bad : d * sxx - b * Sxy;
+		P[1] = singular ? bad : d * Sxy - b * syy;
+		P[2] = singular ? bad : a * Sxy - c * sxx;
+		P[3] = singular ? bad : a * syy - c * Sxy;
+	}
+}
+
 // Order-preserving map of doubles onto uint64 for atomicMin/atomicMax.
 MF_DEV unsigned long long ord_encode(double d) {
 	unsigned long long u = (unsigned long long)__double_as_longlong(d);

@@ -212,9 +212,9 @@ struct WeakArgs {
 	// (transposed, gradients), particle -> particles (shape-function values)
 	const uint32_t *g_sl, *g_snbr, *t_sl, *t_snbr, *p_sl, *p_snbr;
 	const uint16_t *g_cnt, *t_cnt, *p_cnt;
-	const void *g_w, *t_w, *p_w;  // double2 (FP64 forms) / float2 (mixed, pre-multiplied weights)
-	void* gP;                     // nominal stress per Gauss point
-	void* pack;                   // mixed: per particle u and v as float-float (2 x float4)
+	const void *g_w, *t_w, *p_w;  // double2 (FP64; pre-multiplied in the fast form) / float2 (mixed, pre-multiplied)
+	void* gP;                     // nominal stress per Gauss point (parity form: four arrays; else one record)
+	void* pack;                   // per particle u and v: float-float (mixed) or double2 pairs (fast FP64), 32 B
 	const uint32_t* bc_rows;
 	const double* bc_v;
 	uint32_t n_bc;

@@ -275,38 +275,6 @@ __device__ __forceinline__ void tlB_rk64(const TLArgs& a, uint32_t i, double dt,
 // reciprocals by rcp64.  Ring impact at dx = 0.1 mm (439,860 rows), per launch: pass A
 // 268 -> 191 us, pass B 901 -> 422 us (FP64 pipe 86-88 % busy in both).
 #if !MF_STRICT_FORM
-// The per-particle part of pass A (tl_particle) in fewer instructions.
-__device__ __forceinline__ void tl_particle_fast(uint32_t flags, const BodyParams& pr, double Hxx, double Hxy,
-                                                 double Hyx, double Hyy, double Fxx, double Fxy, double Fyx, double Fyy,
-                                                 double rho, double Sxx, double Sxy, double Syy, double P[4],
-                                                 double dA[4]) {
-	const double a = 1. + Hxx, b = Hxy, c = Hyx, d = 1. + Hyy;  // F = (a b; c d)
-	const double J = a * d - b * c;
-	double vx_x = 0., vx_y = 0., vy_x = 0., vy_y = 0.;
-	if (flags & A_VGRAD_TL) {  // Fdot F^-1
-		const double iJ = rcp64(J);
-		vx_x = (Fxx * d - Fxy * c) * iJ;
-		vx_y = (Fxy * a - Fxx * b) * iJ;
-		vy_x = (Fyx * d - Fyy * c) * iJ;
-		vy_y = (Fyy * a - Fyx * b) * iJ;
-	}
-	dA[0] = dA[1] = dA[2] = dA[3] = 0.;
-	if (flags & A_CONTINUITY) dA[0] = -(rho * (vx_x + vy_y));
-	const double p = (flags & A_EOS) ? pr.c0sq * (rho - pr.rho0) : 0.;
-	if (flags & A_JAUMANN) jaumann_plane(vx_x, vx_y, vy_x, vy_y, Sxx, Sxy, Syy, pr.G, dA[1], dA[2], dA[3]);
-	if (flags & A_GREEN) green_stvenant_h<double>(Hxx, Hxy, Hyx, Hyy, pr.D, pr.nu, Sxx, Sxy, Syy);
-	P[0] = P[1] = P[2] = P[3] = 0.;
-	if (flags & A_C2N) {  // J F^-1 sigma = adj(F) sigma (a singular F is not finite, as with the inverse)
-		const double sxx = Sxx - p, syy = Syy - p;
-		const bool singular = J == 0.;
-		const double bad = __longlong_as_double(0x7ff8000000000000ll);
-		P[0] = singular ? bad : d * sxx - b * Sxy;
-		P[1] = singular ? bad : d * Sxy - b * syy;
-		P[2] = singular ? bad : a * Sxy - c * sxx;
-		P[3] = singular ? bad : a * syy - c * Sxy;
-	}
-}
-
 __global__ void __launch_bounds__(256) k_tlA64(TLArgs a) {
 	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= a.n_total) return;
@@ -340,7 +308,9 @@ __global__ void __launch_bounds__(256) k_tlA64(TLArgs a) {
 	const BodyParams& pr = a.params[a.body_of[i]];
 	const double rho = s.rho[i];
 	double P[4], dA[4];
-	tl_particle_fast(flags, pr, Hxx, Hxy, Hyx, Hyy, Fxx, Fxy, Fyx, Fyy, rho, s.Sxx[i], s.Sxy[i], s.Syy[i], P, dA);
+	const PointTerms terms = {(flags & A_VGRAD_TL) != 0, (flags & A_CONTINUITY) != 0, (flags & A_EOS) != 0,
+	                          (flags & A_JAUMANN) != 0, (flags & A_GREEN) != 0, (flags & A_C2N) != 0};
+	tl_point_fast(terms, pr, Hxx, Hxy, Hyx, Hyy, Fxx, Fxy, Fyx, Fyy, rho, s.Sxx[i], s.Sxy[i], s.Syy[i], P, dA);
 	const size_t n = a.n_total;
 #pragma unroll
 	for (int k = 0; k < 4; k++) {

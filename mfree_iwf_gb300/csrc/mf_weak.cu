@@ -178,7 +178,8 @@ __global__ void k_transpose_w(uint32_t n_p, const uint32_t* __restrict__ toff, c
 	}
 }
 
-// CSR -> sliced ELL for the weak lists; values optionally pre-multiplied (mixed form).
+// CSR -> sliced ELL for the weak lists; the values pre-multiplied by the quad weights
+// (mixed and fast FP64 forms).
 __global__ void k_weak_sell(uint32_t n, const uint32_t* __restrict__ off, const uint32_t* __restrict__ nbr,
                             const double* __restrict__ a, const double* __restrict__ b, const uint32_t* __restrict__ sl_off,
                             uint16_t* cnt, uint32_t* snbr, double2* out64, float2* out32,
@@ -193,9 +194,13 @@ __global__ void k_weak_sell(uint32_t n, const uint32_t* __restrict__ off, const 
 		uint32_t j = nbr[q0 + k];
 		snbr[q] = j;
 		double va = a ? a[q0 + k] : 0., vb = b ? b[q0 + k] : 0.;
-		if (out64) out64[q] = make_double2(va, vb);
+		double s = 1.;
+#if MF_STRICT_FORM
+		if (out32)  // (the parity form multiplies in its passes, in the reference's order)
+#endif
+			s = (mul_row ? mul_row[i] : 1.) * (mul_nbr ? mul_nbr[j] : 1.);
+		if (out64) out64[q] = make_double2(va * s, vb * s);
 		if (out32) {
-			double s = (mul_row ? mul_row[i] : 1.) * (mul_nbr ? mul_nbr[j] : 1.);
 			out32[q] = make_float2((float)(va * s), (float)(vb * s));
 		}
 	}
@@ -217,7 +222,8 @@ __global__ void k_weak_bc(WeakArgs a, int on_base) {
 	s.vy[i] = 0.;
 }
 
-// per-Gauss-point part shared by both forms
+#if MF_STRICT_FORM
+// The per-Gauss-point part of the FP64 pass in the reference's expressions
 __device__ __forceinline__ void gp_point(uint32_t flags, const BodyParams& pr, double Hxx, double Hxy, double Hyx,
                                          double Hyy, double Fxx, double Fxy, double Fyx, double Fyy, double rho,
                                          double Sxx, double Sxy, double Syy, double& Pxx, double& Pxy, double& Pyx,
@@ -233,6 +239,7 @@ __device__ __forceinline__ void gp_point(uint32_t flags, const BodyParams& pr, d
 	Pxx = Pxy = Pyx = Pyy = 0.;
 	if (flags & A_C2N_GP) cauchy_to_nominal<double>(Hxx, Hxy, Hyx, Hyy, Sxx - p, Sxy, Syy - p, Pxx, Pxy, Pyx, Pyy);
 }
+#endif
 
 // The per-Gauss-point part of the mixed pass in FP32: GB300 runs FP64 (and every
 // conversion from it) on a narrow pipe, and in FP64 this part bounded the pass.  The
@@ -298,6 +305,138 @@ __device__ __forceinline__ void gp_rk(const WeakArgs& a, uint32_t i, double dt, 
 	}
 }
 
+// RK4 update of one component of particle j (rk4.h:140-183) from its rate d, own row
+// only: in place; false when the step ends in a value that is not finite
+__device__ __forceinline__ bool p_rk64_one(const WeakArgs& a, double* bp, double* ap, double* sp, uint32_t j, double dt,
+                                           double d) {
+	const uint32_t stg = a.stage;
+	if (stg < 3) {
+		const double dts = (stg == 2 ? 1.0 : 0.5) * dt;
+		ap[j] = (stg == 0) ? d : ap[j] + 2 * d;
+		sp[j] = bp[j] + d * dts;
+		return true;
+	}
+	const double w6 = dt * 1. / 6.;
+	const double v = bp[j] + w6 * (ap[j] + d);
+	bp[j] = v;
+	sp[j] = v;
+	return isfinite(v);
+}
+
+#if !MF_STRICT_FORM
+// The FP64 passes, fast form: GB300's narrow FP64 pipe bounds them, so the lists carry the
+// gradients already times the quad weights, the particles' displacement and velocity come
+// packed, and a Gauss point's stress is one 32-byte record: 8 FP64 instructions a list
+// entry in the Gauss-point pass and 4 in the particle pass (24 and 16 in the reference's
+// expressions).  Plate at dx = 0.2 mm (50k particles, 200k Gauss points), per launch:
+// Gauss points 219 -> 99 us (FP64 pipe 89 % busy), particles 139 -> 48 us (80 %).
+__global__ void k_weak_pack64(WeakArgs a) {
+	uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+	if (j >= a.n_p) return;
+	const mfk_host::StateSoA& s = a.st;
+	double2* pk = (double2*)a.pack;
+	pk[2 * (size_t)j] = make_double2(s.x[j] - a.X[j], s.y[j] - a.Y[j]);
+	pk[2 * (size_t)j + 1] = make_double2(s.vx[j], s.vy[j]);
+}
+
+// Displacement and velocity gradient sums of Gauss point i; MOVED: the point has a
+// displacement of its own (its body was moved after the points were placed).
+template <bool MOVED>
+__device__ __forceinline__ void gp_sums64(const WeakArgs& a, uint32_t i, double ux, double uy, double H[4], double F[4]) {
+	const double2 *gw = (const double2*)a.g_w, *pk = (const double2*)a.pack;
+	const uint32_t flags = a.flags;
+	uint32_t q = sbase(a.g_sl, i), c = a.g_cnt[i];
+#pragma unroll 4
+	for (uint32_t k = 0; k < c; k++, q += 32) {
+		const size_t j = a.g_snbr[q];
+		const double2 w = gw[q];
+		if (flags & A_DISP_W) {
+			double2 u = __ldg(pk + 2 * j);
+			if (MOVED) {
+				u.x -= ux;
+				u.y -= uy;
+			}
+			H[0] = fma(u.x, w.x, H[0]);
+			H[1] = fma(u.x, w.y, H[1]);
+			H[2] = fma(u.y, w.x, H[2]);
+			H[3] = fma(u.y, w.y, H[3]);
+		}
+		if (flags & A_VEL_W) {
+			const double2 v = __ldg(pk + 2 * j + 1);
+			F[0] = fma(v.x, w.x, F[0]);
+			F[1] = fma(v.x, w.y, F[1]);
+			F[2] = fma(v.y, w.x, F[2]);
+			F[3] = fma(v.y, w.y, F[3]);
+		}
+	}
+}
+
+__global__ void __launch_bounds__(256) k_gp_pass64(WeakArgs a) {
+	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= a.n_g) return;
+	const uint32_t flags = a.flags;
+	const double ux = a.gp_ux[i], uy = a.gp_uy[i];
+	double H[4] = {0., 0., 0., 0.}, F[4] = {0., 0., 0., 0.};
+	// (the points of a launch usually all have, or all lack, a displacement of their own)
+	const bool moved = ((__double_as_longlong(ux) | __double_as_longlong(uy)) << 1) != 0;
+	if (moved) gp_sums64<true>(a, i, ux, uy, H, F);
+	else gp_sums64<false>(a, i, ux, uy, H, F);
+	const BodyParams& pr = a.params[a.gp_body[i]];
+	double* gs[4] = {a.gst.rho, a.gst.Sxx, a.gst.Sxy, a.gst.Syy};
+	double* gb[4] = {a.gbase.rho, a.gbase.Sxx, a.gbase.Sxy, a.gbase.Syy};
+	double* ga[4] = {a.gacc.rho, a.gacc.Sxx, a.gacc.Sxy, a.gacc.Syy};
+	const PointTerms terms = {(flags & A_VGRAD_GP) != 0, (flags & A_CONT_GP) != 0, (flags & A_EOS_GP) != 0,
+	                          (flags & A_JAUMANN_GP) != 0, false, (flags & A_C2N_GP) != 0};
+	double P[4], e[4];
+	tl_point_fast(terms, pr, H[0], H[1], H[2], H[3], F[0], F[1], F[2], F[3], gs[0][i], gs[1][i], gs[2][i], gs[3][i], P, e);
+	double2* gP = (double2*)a.gP + 2 * (size_t)i;
+	gP[0] = make_double2(P[0], P[1]);
+	gP[1] = make_double2(P[2], P[3]);
+	gp_rk<double>(a, i, pr.dt, e, gb, ga, gs);
+}
+
+// Four lanes share a particle: its ~84 transposed entries would be a serial chain of
+// gathers with too few warps to hide them (one thread a particle: 79 us), and each lane
+// then updates one of x, y, vx, vy.
+constexpr uint32_t PP64_L = 4;
+__global__ void __launch_bounds__(256) k_p_pass64(WeakArgs a) {
+	const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, lane = t % PP64_L;
+	const bool live = t / PP64_L < a.n_p;
+	const uint32_t j = live ? t / PP64_L : a.n_p - 1;  // (every lane stays for the shuffles)
+	const uint32_t flags = a.flags;
+	double fx = 0., fy = 0.;
+	if (flags & A_STRESS_W) {
+		const double2 *tw = (const double2*)a.t_w, *gP = (const double2*)a.gP;
+		uint32_t q = sbase(a.t_sl, j) + 32 * lane, c = a.t_cnt[j];
+#pragma unroll 4
+		for (uint32_t k = lane; k < c; k += PP64_L, q += 32 * PP64_L) {
+			const size_t i = a.t_snbr[q];
+			const double2 w = tw[q], p = __ldg(gP + 2 * i), r = __ldg(gP + 2 * i + 1);  // Pxx Pxy, Pyx Pyy
+			fx = fma(p.x, w.x, fma(r.x, w.y, fx));
+			fy = fma(p.y, w.x, fma(r.y, w.y, fy));
+		}
+#pragma unroll
+		for (uint32_t o = PP64_L / 2; o > 0; o >>= 1) {
+			fx += __shfl_xor_sync(0xffffffffu, fx, o);
+			fy += __shfl_xor_sync(0xffffffffu, fy, o);
+		}
+	}
+	if (!live) return;
+	const mfk_host::StateSoA& s = a.st;
+	double d = 0.;  // the rate of component `lane`
+	if (lane < 2) {
+		if (flags & A_ADVECTION) d = (lane == 0 ? s.vx : s.vy)[j];
+	} else if (flags & A_MOMENTUM_W) {
+		d = ((lane == 2 ? a.fcx : a.fcy)[j] - (lane == 2 ? fx : fy)) * rcp64(a.m[j]);
+	}
+	const bool ok = p_rk64_one(a, lane == 0 ? a.base.x : lane == 1 ? a.base.y : lane == 2 ? a.base.vx : a.base.vy,
+	                           lane == 0 ? a.acc.x : lane == 1 ? a.acc.y : lane == 2 ? a.acc.vx : a.acc.vy,
+	                           lane == 0 ? a.st.x : lane == 1 ? a.st.y : lane == 2 ? a.st.vx : a.st.vy, j,
+	                           a.params[a.body_of[j]].dt, d);
+	if (!ok) raise(reinterpret_cast<DevStatus*>(a.status), ERR_NONFINITE, j);
+}
+
+#else
 __global__ void __launch_bounds__(256) k_gp_pass64(WeakArgs a) {
 	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= a.n_g) return;
@@ -377,27 +516,12 @@ __global__ void __launch_bounds__(256) k_p_pass64(WeakArgs a) {
 	double* bp[4] = {a.base.x, a.base.y, a.base.vx, a.base.vy};
 	double* ap[4] = {a.acc.x, a.acc.y, a.acc.vx, a.acc.vy};
 	double* sp[4] = {a.st.x, a.st.y, a.st.vx, a.st.vy};
-	uint32_t stg = a.stage;
-	double dt = pr.dt;
-	if (stg < 3) {
-		double dts = (stg == 2 ? 1.0 : 0.5) * dt;
+	bool ok = true;
 #pragma unroll
-		for (int q = 0; q < 4; q++) {
-			ap[q][j] = (stg == 0) ? d[q] : ap[q][j] + 2 * d[q];
-			sp[q][j] = bp[q][j] + d[q] * dts;  // own row only: in place
-		}
-	} else {
-		double w6 = dt * 1. / 6.;
-#pragma unroll
-		for (int q = 0; q < 4; q++) {
-			double v = bp[q][j] + w6 * (ap[q][j] + d[q]);
-			bp[q][j] = v;
-			sp[q][j] = v;
-		}
-		if (!(isfinite(bp[0][j]) && isfinite(bp[1][j]) && isfinite(bp[2][j]) && isfinite(bp[3][j])))
-			raise(reinterpret_cast<DevStatus*>(a.status), ERR_NONFINITE, j);
-	}
+	for (int q = 0; q < 4; q++) ok = p_rk64_one(a, bp[q], ap[q], sp[q], j, pr.dt, d[q]) && ok;
+	if (!ok) raise(reinterpret_cast<DevStatus*>(a.status), ERR_NONFINITE, j);
 }
+#endif
 
 // ---- mixed form: particle displacement and velocity as float-float, FP32 sums
 __global__ void k_weak_pack(WeakArgs a) {
@@ -521,9 +645,15 @@ __global__ void k_smooth(WeakArgs a, int mixed) {
 		double vsx = 0., vsy = 0.;
 		for (uint32_t k = 0; k < c; k++, q += 32) {
 			uint32_t j = a.p_snbr[q];
+#if MF_STRICT_FORM
 			double w = pw[q].x, qwj = a.qw_p[j];
 			vsx += a.base.vx[j] * w * qwj;
 			vsy += a.base.vy[j] * w * qwj;
+#else
+			const double w = pw[q].x;  // already times qw_j
+			vsx = fma(a.base.vx[j], w, vsx);
+			vsy = fma(a.base.vy[j], w, vsy);
+#endif
 		}
 		a.st.vx[i] = vsx;
 		a.st.vy[i] = vsy;
@@ -604,6 +734,9 @@ cudaError_t weak_stage(const WeakArgs& a, bool mixed, int part, cudaStream_t s) 
 		break;
 	case 1:
 		if (mixed) k_weak_pack<<<grid1(a.n_p, 256), 256, 0, s>>>(a);
+#if !MF_STRICT_FORM
+		else k_weak_pack64<<<grid1(a.n_p, 256), 256, 0, s>>>(a);
+#endif
 		break;
 	case 2:
 		if (mixed) k_gp_pass32<<<grid1(a.n_g, bs), bs, 0, s>>>(a);
@@ -611,7 +744,11 @@ cudaError_t weak_stage(const WeakArgs& a, bool mixed, int part, cudaStream_t s) 
 		break;
 	case 3:
 		if (mixed) k_p_pass32<<<grid1(a.n_p, bs), bs, 0, s>>>(a);
+#if MF_STRICT_FORM
 		else k_p_pass64<<<grid1(a.n_p, bs), bs, 0, s>>>(a);
+#else
+		else k_p_pass64<<<grid1((uint64_t)a.n_p * PP64_L, bs), bs, 0, s>>>(a);
+#endif
 		break;
 	case 4:
 		if (a.n_bc) k_weak_bc<<<grid1(a.n_bc, 128), 128, 0, s>>>(a, 1);

@@ -1,5 +1,6 @@
 """The fast FP64 passes against the CPU oracle where their branches change: with and
-without the velocity gradient, viscosity and contact, row counts that do not fill a warp or a block."""
+without the velocity gradient, viscosity and contact, moving and resting Gauss points,
+row counts that do not fill a warp or a block."""
 import numpy as np
 import pytest
 
@@ -8,7 +9,8 @@ from mfree_iwf_gb300 import scenarios as S
 
 pytestmark = pytest.mark.gpu
 
-CASES = [S.tensile_tl(7), S.tensile_tl(21), S.rings_tl_contact(13), S.rings_tl_contact(21)]
+CASES = [S.tensile_tl(7), S.tensile_tl(21), S.rings_tl_contact(13), S.rings_tl_contact(21), S.tensile_tl_weak(7),
+         S.tensile_tl_weak(17), S.rotation_tl_weak(15), S.rotation_tl_fem(15), S.rings_tl_weak_contact(21)]
 
 
 # 1e-8: the fast FP64 form's bound against the reference (contraction and reciprocals by
