@@ -4,13 +4,12 @@
 // stress and contact-force history (mfree_iwf_gb300/surrogate.py).  No counterpart in
 // the reference: this is a learned screen placed in front of the solver.
 //
-// The forward products go through a pipelined tensor-core GEMM (k_gemm_nt: 128x64
-// tiles, cp.async double buffering, ldmatrix fragments); the backward products, whose
-// operands are transposed, through a simpler tiled one (k_gemm: 64x64 tiles staged
-// element-wise).  Both issue mma.sync m16n8k16 (BF16 inputs, FP32 accumulators) with
-// gridDim.z over the ensemble members, and fuse the bias and ReLU into the epilogue,
-// which stores FP32 and/or BF16.  The layers (6 -> 256 -> 256 -> 256 -> 66, a few hundred rows per
-// training batch) are too small for a TMA/tcgen05 pipeline to pay off.
+// Inference runs the whole network in one tcgen05 kernel (namespace fz).  Per-layer
+// forward products run on tcgen05 (namespace tc) where K is a multiple of 64, else on a
+// pipelined mma.sync kernel (k_gemm_nt).  The backward products of a training step, a few
+// hundred rows per member and a few microseconds each, are 64x64 mma.sync tiles
+// (namespace tr) that fill the SMs with small blocks; a layer's weight gradient, its bias
+// gradient and the gradient of its input (with the ReLU mask) share one launch.
 //
 // Training keeps the whole data set on the device.  One training step -- bootstrap
 // minibatch gather (each member draws its own rows), forward, MSE, backward, Adam --
@@ -51,108 +50,8 @@ struct GemmArgs {
 	long long sBias;
 	int relu;
 	int n_store;  // tcgen05 path: FP32 output columns stored (0: all N), any ldc
+	int n_slice;  // tcgen05 path: columns per block when N is split over gridDim.z
 };
-
-constexpr int BM = 64, BN = 64, BK = 32, PADK = BK + 8;  // 80-byte rows: conflict-free fragment loads
-
-__device__ __forceinline__ uint32_t ld_pair(const bf16* p) { return *reinterpret_cast<const uint32_t*>(p); }
-
-// C[M x N] = op(A)[M x K] op(B)[K x N]
-//   TA = false: A(m, k) = A[m*lda + k]   TA = true: A(m, k) = A[k*lda + m]
-//   TB = false: B(k, n) = B[k*ldb + n]   TB = true: B(k, n) = B[n*ldb + k]
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(128) k_gemm(GemmArgs g) {
-	__shared__ __align__(16) bf16 As[BM][PADK];  // [m][k]
-	__shared__ __align__(16) bf16 Bs[BN][PADK];  // [n][k]
-	const int z = blockIdx.z;
-	const bf16* A = g.A + z * g.sA;
-	const bf16* B = g.B + z * g.sB;
-	const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-	const int wm = warp >> 1, wn = warp & 1;
-	const int gid = lane >> 2, tig = lane & 3;
-	float acc[2][4][4];
-#pragma unroll
-	for (int a = 0; a < 2; a++)
-#pragma unroll
-		for (int b = 0; b < 4; b++)
-#pragma unroll
-			for (int c = 0; c < 4; c++) acc[a][b][c] = 0.f;
-	const bf16 zero = __float2bfloat16(0.f);
-	for (int k0 = 0; k0 < g.K; k0 += BK) {
-		// stage the tiles; consecutive threads walk the contiguous dimension
-#pragma unroll 4
-		for (int e = tid; e < BM * BK; e += 128) {
-			const int mm = TA ? (e % BM) : (e / BK), kk = TA ? (e / BM) : (e % BK);
-			const int m = m0 + mm, k = k0 + kk;
-			bf16 v = zero;
-			if (m < g.M && k < g.K) v = TA ? A[(long long)k * g.lda + m] : A[(long long)m * g.lda + k];
-			As[mm][kk] = v;
-		}
-#pragma unroll 4
-		for (int e = tid; e < BN * BK; e += 128) {
-			const int nn = TB ? (e / BK) : (e % BN), kk = TB ? (e % BK) : (e / BN);
-			const int n = n0 + nn, k = k0 + kk;
-			bf16 v = zero;
-			if (n < g.N && k < g.K) v = TB ? B[(long long)n * g.ldb + k] : B[(long long)k * g.ldb + n];
-			Bs[nn][kk] = v;
-		}
-		__syncthreads();
-#pragma unroll
-		for (int ks = 0; ks < BK; ks += 16) {
-			uint32_t af[2][4], bfr[4][2];
-			const int c = ks + tig * 2;
-#pragma unroll
-			for (int mt = 0; mt < 2; mt++) {
-				const int r = wm * 32 + mt * 16 + gid;
-				af[mt][0] = ld_pair(&As[r][c]);
-				af[mt][1] = ld_pair(&As[r + 8][c]);
-				af[mt][2] = ld_pair(&As[r][c + 8]);
-				af[mt][3] = ld_pair(&As[r + 8][c + 8]);
-			}
-#pragma unroll
-			for (int nt = 0; nt < 4; nt++) {
-				const int n = wn * 32 + nt * 8 + gid;
-				bfr[nt][0] = ld_pair(&Bs[n][c]);
-				bfr[nt][1] = ld_pair(&Bs[n][c + 8]);
-			}
-#pragma unroll
-			for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-				for (int nt = 0; nt < 4; nt++) {
-					float* d = acc[mt][nt];
-					asm volatile(
-					    "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-					    "{%0,%1,%2,%3};\n"
-					    : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-					    : "r"(af[mt][0]), "r"(af[mt][1]), "r"(af[mt][2]), "r"(af[mt][3]), "r"(bfr[nt][0]),
-					      "r"(bfr[nt][1]));
-				}
-		}
-		__syncthreads();
-	}
-	float* C = g.C ? g.C + z * g.sC : nullptr;
-	bf16* Cb = g.Cb ? g.Cb + z * g.sCb : nullptr;
-	const float* bias = g.bias ? g.bias + z * g.sBias : nullptr;
-#pragma unroll
-	for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-		for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-			for (int h = 0; h < 2; h++)
-#pragma unroll
-				for (int q = 0; q < 2; q++) {
-					const int m = m0 + wm * 32 + mt * 16 + gid + 8 * h;
-					const int n = n0 + wn * 32 + nt * 8 + tig * 2 + q;
-					if (m >= g.M || n >= g.N) continue;
-					float v = acc[mt][nt][2 * h + q];
-					if (bias) v += bias[n];
-					if (g.relu) v = fmaxf(v, 0.f);
-					if (C) C[(long long)m * g.ldc + n] = v;
-					if (Cb) Cb[(long long)m * g.ldcb + n] = __float2bfloat16(v);
-				}
-}
-
 
 // The forward product Z = H W^T (A row-major [M][K], B = W row-major [N][K], both
 // contiguous in k) as a pipelined kernel: 128x64 output tiles, 8 warps of 32x32,
@@ -389,7 +288,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, GemmArgs g,
               int rows_per_member, uint32_t* err) {
 	extern __shared__ uint8_t smem_raw[];
-	const int N = g.N, KB = g.K / BK, G = gridDim.x, z = blockIdx.y;
+	// gridDim.z > 1: each block takes n_slice of the N columns (rows of W past N are zero)
+	const int n0 = blockIdx.z * g.n_slice, N = gridDim.z > 1 ? g.n_slice : g.N;
+	const int KB = g.K / BK, G = gridDim.x, z = blockIdx.y;
 	const uint32_t raw = saddr(smem_raw);
 	uint8_t* sW = smem_raw + (((raw + 1023u) & ~1023u) - raw);
 	uint8_t* sA = sW + (size_t)KB * N * 128;
@@ -431,7 +332,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 	if (warp == 0) {
 		if (lane == 0) {  // TMA producer
 			mbar_expect_tx(w_full, (uint32_t)(KB * N * 128));
-			for (int kb = 0; kb < KB; kb++) tma_load_3d(sW + (size_t)kb * N * 128, &tmW, kb * BK, 0, z, w_full);
+			for (int kb = 0; kb < KB; kb++) tma_load_3d(sW + (size_t)kb * N * 128, &tmW, kb * BK, n0, z, w_full);
 			uint32_t it = 0;
 			for (int t = blockIdx.x; t < tiles && ok; t += G)
 				for (int kb = 0; kb < KB; kb++, it++) {
@@ -472,10 +373,11 @@ __global__ void __launch_bounds__(THREADS, 1)
 		// instruction; FP32: one row of up to 128 bytes per instruction, any ldc
 		const int q = warp & 3, grp = (warp - 2) >> 2;  // lane quarter; column group (chunks grp, grp + 2, ...)
 		uint8_t* stg = sStg + (size_t)(warp - 2) * 32 * STG_ROW;
-		const float* bias = g.bias ? g.bias + z * g.sBias : nullptr;
-		float* C = g.C ? g.C + z * g.sC : nullptr;
-		bf16* Cb = g.Cb ? g.Cb + z * g.sCb : nullptr;
-		const int nst = g.n_store > 0 ? g.n_store : N;
+		const float* bias = g.bias ? g.bias + z * g.sBias + n0 : nullptr;
+		float* C = g.C ? g.C + z * g.sC + n0 : nullptr;
+		bf16* Cb = g.Cb ? g.Cb + z * g.sCb + n0 : nullptr;
+		const int n_end = g.N - n0;  // columns of this block that exist
+		const int nst = (g.n_store > 0 ? g.n_store : g.N) - n0;
 		uint32_t i = 0;
 		for (int t = blockIdx.x; t < tiles && ok; t += G, i++) {
 			const uint32_t ab = i & 1u;
@@ -490,7 +392,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
 				for (int j = 0; j < 32; j++) {
 					float x = __uint_as_float(r[j]);
-					if (bias && c0 + j < N) x += bias[c0 + j];
+					if (bias && c0 + j < n_end) x += bias[c0 + j];
 					if (g.relu) x = fmaxf(x, 0.f);
 					v[j] = x;
 				}
@@ -509,7 +411,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
 					for (int k = 0; k < 4; k++) {
 						const int e = lane + 32 * k, rr = e >> 2, ch = e & 3, m = row0 + rr;
-						if (m < g.M && c0 + 8 * ch < N)
+						if (m < g.M && c0 + 8 * ch < n_end)
 							*reinterpret_cast<uint4*>(Cb + (long long)m * g.ldcb + c0 + 8 * ch) =
 							    *reinterpret_cast<const uint4*>(stg + rr * STG_ROW + 16 * ch);
 					}
@@ -906,9 +808,213 @@ __global__ void k_pack_layer(int members, int N, int K, int Kp, const bf16* src,
 
 }  // namespace fz
 
+// ---- The backward products of a training step: 64x64 tiles of mma.sync m16n8k16 (BF16
+// inputs, FP32 accumulators, K ascending in steps of 16), four warps of 32x32, K in slices
+// of 64 through a 3-stage cp.async ring (zero-filled past M, N and K), fragments by
+// ldmatrix (transposed where the operand's K does not run along its rows).  At 512 rows
+// and five members a 256-wide layer is 80 + 160 tiles: one or two waves of small blocks,
+// bound by the latency of their four to eight slices.  Per step of 512 rows and five
+// members of 6-256-256-256-66: 428 us with element-wise staged tiles and a launch for
+// each product, ReLU mask and bias gradient; 69 us now (this launch 54 + 19 + 19 + 4 -> 7.6 us a layer).
+namespace tr {
+
+constexpr int T = 64, LD = T + 8, STAGES = 3, THREADS = 128;  // 144-byte rows: ldmatrix conflict-free
+constexpr size_t SMEM = (size_t)STAGES * 2 * T * LD * sizeof(bf16);
+
+__device__ __forceinline__ void ldsm_x4_t(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* p) {
+	uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+	             : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+	             : "r"(a));
+}
+
+// 64x64 elements from row r0, column c0 of a row-major matrix of R x C elements
+__device__ __forceinline__ void load_tile(bf16* s, const bf16* g, int ld, int r0, int c0, int R, int C) {
+#pragma unroll
+	for (int e = threadIdx.x; e < T * T / 8; e += THREADS) {
+		const int row = e >> 3, col = (e & 7) * 8;
+		const bool ok = r0 + row < R && c0 + col < C;  // (C is a multiple of 8)
+		cp16z(s + row * LD + col, ok ? (const void*)(g + (long long)(r0 + row) * ld + c0 + col) : (const void*)g, ok ? 16u : 0u);
+	}
+}
+
+// acc += A(m0.., k) B(k, n0..) over k < K.  AT: A is stored [k][m], else [m][k];
+// BT: B is stored [n][k], else [k][n].
+template <bool AT, bool BT>
+__device__ __forceinline__ void product(const bf16* A, int lda, const bf16* B, int ldb, int m0, int n0, int M, int N, int K,
+                                        bf16* smem, float (&acc)[2][4][4]) {
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+	const int nk = (K + T - 1) / T;
+	auto load = [&](int kt) {
+		if (kt < nk) {
+			bf16 *As = smem + (kt % STAGES) * 2 * T * LD, *Bs = As + T * LD;
+			if (AT) load_tile(As, A, lda, kt * T, m0, K, M);
+			else load_tile(As, A, lda, m0, kt * T, M, K);
+			if (BT) load_tile(Bs, B, ldb, n0, kt * T, N, K);
+			else load_tile(Bs, B, ldb, kt * T, n0, K, N);
+		}
+		asm volatile("cp.async.commit_group;\n" ::: "memory");  // (empty past the last slice: the waits count groups)
+	};
+#pragma unroll
+	for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+		for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+			for (int c = 0; c < 4; c++) acc[mt][nt][c] = 0.f;
+#pragma unroll
+	for (int kt = 0; kt < STAGES - 1; kt++) load(kt);
+	for (int kt = 0; kt < nk; kt++) {
+		asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+		__syncthreads();  // slice kt has landed, and every warp is done with the slot the next load takes
+		load(kt + STAGES - 1);
+		const bf16 *As = smem + (kt % STAGES) * 2 * T * LD, *Bs = As + T * LD;
+#pragma unroll
+		for (int ks = 0; ks < T; ks += 16) {
+			uint32_t af[2][4], bq[4][2];
+#pragma unroll
+			for (int mt = 0; mt < 2; mt++) {
+				const int m = wm + mt * 16;
+				if (AT)
+					ldsm_x4_t(af[mt][0], af[mt][1], af[mt][2], af[mt][3],
+					          As + (ks + (lane >> 4) * 8 + (lane & 7)) * LD + m + ((lane >> 3) & 1) * 8);
+				else
+					ldsm_x4(af[mt][0], af[mt][1], af[mt][2], af[mt][3], As + (m + (lane & 15)) * LD + ks + (lane >> 4) * 8);
+			}
+#pragma unroll
+			for (int np = 0; np < 2; np++) {  // two n-tiles of 8 per ldmatrix.x4
+				const int n = wn + np * 16;
+				if (BT)
+					ldsm_x4(bq[2 * np][0], bq[2 * np][1], bq[2 * np + 1][0], bq[2 * np + 1][1],
+					        Bs + (n + (lane & 7) + ((lane >> 4) << 3)) * LD + ks + ((lane >> 3) & 1) * 8);
+				else
+					ldsm_x4_t(bq[2 * np][0], bq[2 * np][1], bq[2 * np + 1][0], bq[2 * np + 1][1],
+					          Bs + (ks + ((lane >> 3) & 1) * 8 + (lane & 7)) * LD + n + (lane >> 4) * 8);
+			}
+#pragma unroll
+			for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+				for (int nt = 0; nt < 4; nt++) {
+					float* d = acc[mt][nt];
+					asm volatile(
+					    "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+					    "{%0,%1,%2,%3};\n"
+					    : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+					    : "r"(af[mt][0]), "r"(af[mt][1]), "r"(af[mt][2]), "r"(af[mt][3]), "r"(bq[nt][0]), "r"(bq[nt][1]));
+				}
+		}
+	}
+}
+
+// f(m, n, v0, v1) for every element pair (n, n + 1) that this thread holds
+template <class F>
+__device__ __forceinline__ void each_pair(int m0, int n0, const float (&acc)[2][4][4], F f) {
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+	for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+		for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+			for (int h = 0; h < 2; h++)
+				f(m0 + (warp >> 1) * 32 + mt * 16 + (lane >> 2) + 8 * h, n0 + (warp & 1) * 32 + nt * 8 + (lane & 3) * 2,
+				  acc[mt][nt][2 * h], acc[mt][nt][2 * h + 1]);
+}
+
+// Sums of 64 columns over `rows` rows of FP32, added row by row: 64-row tiles through a
+// cp.async ring, one thread a column.
+__device__ __forceinline__ void column_sums(const float* g, int ld, int n0, int N, int rows, float* smem, float* out) {
+	constexpr int ROWS = 32;
+	const int nt = (rows + ROWS - 1) / ROWS;
+	auto load = [&](int t) {
+		if (t < nt) {
+			float* s = smem + (t % STAGES) * ROWS * T;
+#pragma unroll
+			for (int e = threadIdx.x; e < ROWS * T / 4; e += THREADS) {
+				const int row = e / (T / 4), col = e % (T / 4) * 4;
+				const bool ok = t * ROWS + row < rows && n0 + col < N;
+				cp16z(s + row * T + col, ok ? (const void*)(g + (long long)(t * ROWS + row) * ld + n0 + col) : (const void*)g,
+				      ok ? 16u : 0u);
+			}
+		}
+		asm volatile("cp.async.commit_group;\n" ::: "memory");
+	};
+#pragma unroll
+	for (int t = 0; t < STAGES - 1; t++) load(t);
+	float sum = 0.f;
+	for (int t = 0; t < nt; t++) {
+		asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+		__syncthreads();
+		load(t + STAGES - 1);
+		if (threadIdx.x < T) {
+			const float* s = smem + (t % STAGES) * ROWS * T + threadIdx.x;
+			const int r1 = min(ROWS, rows - t * ROWS);
+			if (r1 == ROWS) {
+#pragma unroll
+				for (int r = 0; r < ROWS; r++) sum += s[r * T];
+			} else {
+				for (int r = 0; r < r1; r++) sum += s[r * T];
+			}
+		}
+	}
+	if (threadIdx.x < T && n0 + (int)threadIdx.x < N) out[n0 + threadIdx.x] = sum;
+}
+
+// One layer backward over a batch, three roles by block: dW = dZ^T H (w_tiles blocks); the
+// bias gradient, dZ's column sums (b_tiles blocks); the previous layer's dZ = dZ W where
+// its ReLU output H > 0 (the rest).  dZ comes and goes as BF16 (the products' operand)
+// and FP32 (the bias gradient's).
+struct Bwd {
+	int batch, out_p, in_p;
+	const bf16 *dz, *H, *W;
+	const float* dzf;
+	long long sDz, sHin, sW;
+	float *gW, *gB;
+	long long sGw, sGb;
+	bf16* dz_prev;
+	float* dzf_prev;
+	int w_tiles, b_tiles;
+};
+__global__ void __launch_bounds__(THREADS) k_backward(Bwd g) {
+	extern __shared__ __align__(16) bf16 smem[];
+	const int z = blockIdx.y, nx = (g.in_p + T - 1) / T;
+	const bf16 *dz = g.dz + z * g.sDz, *H = g.H + z * g.sHin;
+	float acc[2][4][4];
+	int t = blockIdx.x;
+	if (t < g.w_tiles) {
+		const int m0 = t / nx * T, n0 = t % nx * T;
+		product<true, false>(dz, g.out_p, H, g.in_p, m0, n0, g.out_p, g.in_p, g.batch, smem, acc);
+		float* gW = g.gW + z * g.sGw;
+		each_pair(m0, n0, acc, [&](int m, int n, float v0, float v1) {
+			if (m < g.out_p && n < g.in_p) *reinterpret_cast<float2*>(gW + (long long)m * g.in_p + n) = make_float2(v0, v1);
+		});
+		return;
+	}
+	t -= g.w_tiles;
+	if (t < g.b_tiles) {
+		column_sums(g.dzf + z * g.sDz, g.out_p, t * T, g.out_p, g.batch, reinterpret_cast<float*>(smem), g.gB + z * g.sGb);
+		return;
+	}
+	t -= g.b_tiles;
+	const int m0 = t / nx * T, n0 = t % nx * T;
+	product<false, false>(dz, g.out_p, g.W + z * g.sW, g.in_p, m0, n0, g.batch, g.in_p, g.out_p, smem, acc);
+	bf16* prev = g.dz_prev + z * g.sDz;
+	float* prevf = g.dzf_prev + z * g.sDz;
+	each_pair(m0, n0, acc, [&](int m, int n, float v0, float v1) {
+		if (m < g.batch && n < g.in_p) {
+			const long long e = (long long)m * g.in_p + n;
+			const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(H + e);
+			v0 = __low2float(h) > 0.f ? v0 : 0.f;
+			v1 = __high2float(h) > 0.f ? v1 : 0.f;
+			*reinterpret_cast<__nv_bfloat162*>(prev + e) = __floats2bfloat162_rn(v0, v1);
+			*reinterpret_cast<float2*>(prevf + e) = make_float2(v0, v1);
+		}
+	});
+}
+
+}  // namespace tr
+
 // Training control block in device memory, read by the graph's kernels on every replay.
 struct TrainCtl {
-	uint32_t step;   // Adam steps taken so far (the current step's number inside a step)
+	uint32_t step;   // Adam steps taken so far (inside a step its number is step + 1)
 	uint32_t t0;     // step count when the current mf_mlp_train call began
 	uint32_t total;  // steps of the current call (cosine schedule length)
 	uint32_t n_data;
@@ -924,15 +1030,17 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
 	return x ^ (x >> 31);
 }
 
-// bootstrap minibatch: member z's row r takes data row splitmix(seed, step, z, r) mod n
-__global__ void k_gather(const TrainCtl* ctl, int in, int in_p, int out, long long sH0, long long sY, const float* X,
-                         const float* Y, bf16* H0, float* Yb) {
-	const int r = blockIdx.x, z = blockIdx.y;
-	const uint64_t key = ctl->seed ^ ((uint64_t)ctl->step << 20) ^ ((uint64_t)z << 52) ^ (uint64_t)r;
+// bootstrap minibatch: member z's row r takes data row splitmix(seed, step, z, r) mod n;
+// a warp per row
+__global__ void __launch_bounds__(128) k_gather(const TrainCtl* ctl, int rows, int in, int in_p, int out, long long sH0,
+                                                long long sY, const float* X, const float* Y, bf16* H0, float* Yb) {
+	const int r = blockIdx.x * 4 + threadIdx.x / 32, z = blockIdx.y, lane = threadIdx.x % 32;
+	if (r >= rows) return;
+	const uint64_t key = ctl->seed ^ ((uint64_t)(ctl->step + 1) << 20) ^ ((uint64_t)z << 52) ^ (uint64_t)r;
 	const uint32_t src = (uint32_t)(splitmix64(key) % ctl->n_data);
-	for (int c = threadIdx.x; c < in_p; c += blockDim.x)
+	for (int c = lane; c < in_p; c += 32)
 		H0[z * sH0 + (long long)r * in_p + c] = __float2bfloat16(c < in ? X[(long long)src * in + c] : 0.f);
-	for (int c = threadIdx.x; c < out; c += blockDim.x) Yb[z * sY + (long long)r * out + c] = Y[(long long)src * out + c];
+	for (int c = lane; c < out; c += 32) Yb[z * sY + (long long)r * out + c] = Y[(long long)src * out + c];
 }
 
 // x (FP32 [batch][in] per member, member stride sx; 0 = shared) -> BF16 [batch][in_p], zero padded
@@ -974,57 +1082,69 @@ __global__ void k_mse(int batch, int out, int out_p, const float* yp, long long 
 	if (threadIdx.x == 0) atomicAdd(&loss[z], red[0] * inv);
 }
 
-// dZ = dH where the layer's ReLU output H > 0, else 0 (FP32 and BF16 copies)
-__global__ void k_relu_bwd(int members, long long per, const float* dh, long long sdh, const bf16* h, long long sh,
-                           float* dz, bf16* dzb, long long sdz) {
-	const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-	if (e >= per * members) return;
-	const int z = (int)(e / per);
-	const long long w = e % per;
-	const float v = __bfloat162float(h[z * sh + w]) > 0.f ? dh[z * sdh + w] : 0.f;
-	dz[z * sdz + w] = v;
-	dzb[z * sdz + w] = __float2bfloat16(v);
-}
-
-// db[n] = sum over rows of dZ[r][n]
-__global__ void k_bias_grad(int batch, int out_p, const float* dz, long long sdz, float* db, long long sdb) {
-	const int n = blockIdx.x * blockDim.x + threadIdx.x, z = blockIdx.y;
-	if (n >= out_p) return;
-	const float* d = dz + z * sdz;
-	float s = 0.f;
-	for (int r = 0; r < batch; r++) s += d[(long long)r * out_p + n];
-	db[z * sdb + n] = s;
-}
-
 // Adam (Kingma & Ba 2015) on FP32 master parameters with a cosine learning-rate
-// schedule from lr0 to lr1 over the current call; refreshes the BF16 weight copy.
-__global__ void k_adam(const TrainCtl* ctl, long long n, float* w, const float* g, float* m, float* v, bf16* wb) {
-	const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-	if (e >= n) return;
+// schedule from lr0 to lr1 over the current call; refreshes the BF16 weight copy.  The
+// weights' blocks first, then the biases' (one launch); the schedule once per block.
+struct AdamSet {
+	long long n;
+	float* w;
+	const float* g;
+	float *m, *v;
+	bf16* wb;  // optional
+};
+__global__ void __launch_bounds__(256) k_adam(const TrainCtl* ctl, AdamSet weights, AdamSet biases, unsigned w_blocks) {
+	__shared__ float s_lr, s_c1, s_c2;
 	const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-	const uint32_t t = ctl->step;
-	const float frac = ctl->total > 1 ? (float)(t - 1 - ctl->t0) / (float)(ctl->total - 1) : 0.f;
-	const float lr = ctl->lr1 + 0.5f * (ctl->lr0 - ctl->lr1) * (1.f + cospif(fminf(fmaxf(frac, 0.f), 1.f)));
-	const float c1 = 1.f - powf(b1, (float)t), c2 = 1.f - powf(b2, (float)t);
-	const float gi = g[e];
-	const float mi = b1 * m[e] + (1.f - b1) * gi;
-	const float vi = b2 * v[e] + (1.f - b2) * gi * gi;
-	m[e] = mi;
-	v[e] = vi;
-	const float wi = w[e] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-	w[e] = wi;
-	if (wb) wb[e] = __float2bfloat16(wi);
+	const bool wts = blockIdx.x < w_blocks;
+	const AdamSet& p = wts ? weights : biases;
+	const long long q = (long long)(wts ? blockIdx.x : blockIdx.x - w_blocks) * 256 + threadIdx.x;
+	const bool in = 4 * q < p.n;  // (n is a multiple of 16, the arrays 16-byte aligned)
+	float4 w{}, m{}, v{}, g{};
+	if (in) {
+		w = ((float4*)p.w)[q];
+		m = ((float4*)p.m)[q];
+		v = ((float4*)p.v)[q];
+		g = ((const float4*)p.g)[q];
+	}
+	if (threadIdx.x == 0) {
+		const uint32_t t = ctl->step + 1;
+		const float frac = ctl->total > 1 ? (float)(t - 1 - ctl->t0) / (float)(ctl->total - 1) : 0.f;
+		s_lr = ctl->lr1 + 0.5f * (ctl->lr0 - ctl->lr1) * (1.f + cospif(fminf(fmaxf(frac, 0.f), 1.f)));
+		s_c1 = 1.f - powf(b1, (float)t);
+		s_c2 = 1.f - powf(b2, (float)t);
+	}
+	__syncthreads();
+	if (!in) return;
+	const float lr = s_lr, c1 = s_c1, c2 = s_c2;
+	auto one = [&](float& wi, float& mi, float& vi, float gi) {
+		// (the two contractions spelled out: any other rounding of them, amplified by the
+		// steps that follow, ends in other weights)
+		mi = __fmaf_rn(1.f - b1, gi, __fmul_rn(b1, mi));
+		vi = __fmaf_rn(__fmul_rn(1.f - b2, gi), gi, __fmul_rn(b2, vi));
+		wi = wi - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+	};
+	one(w.x, m.x, v.x, g.x);
+	one(w.y, m.y, v.y, g.y);
+	one(w.z, m.z, v.z, g.z);
+	one(w.w, m.w, v.w, g.w);
+	((float4*)p.m)[q] = m;
+	((float4*)p.v)[q] = v;
+	((float4*)p.w)[q] = w;
+	if (p.wb) {
+		((__nv_bfloat162*)p.wb)[2 * q] = __floats2bfloat162_rn(w.x, w.y);
+		((__nv_bfloat162*)p.wb)[2 * q + 1] = __floats2bfloat162_rn(w.z, w.w);
+	}
 }
 
-__global__ void k_step_begin(TrainCtl* ctl, float* loss, int members) {
+// the step's losses into the history, and the counters ready for the next step
+__global__ void k_step_end(TrainCtl* ctl, float* loss, int members) {
+	const uint32_t row = ctl->step - ctl->t0;
+	for (int z = threadIdx.x; z < members; z += blockDim.x) {
+		if (ctl->hist && row < ctl->total) ctl->hist[(size_t)row * members + z] = loss[z];
+		loss[z] = 0.f;
+	}
+	__syncthreads();
 	if (threadIdx.x == 0) ctl->step += 1;
-	for (int z = threadIdx.x; z < members; z += blockDim.x) loss[z] = 0.f;
-}
-
-__global__ void k_step_end(const TrainCtl* ctl, const float* loss, int members) {
-	const uint32_t row = ctl->step - 1 - ctl->t0;
-	if (!ctl->hist || row >= ctl->total) return;
-	for (int z = threadIdx.x; z < members; z += blockDim.x) ctl->hist[(size_t)row * members + z] = loss[z];
 }
 
 __global__ void k_to_bf16(long long n, const float* a, bf16* b) {
@@ -1087,8 +1207,8 @@ struct mf_mlp {
 	Buf<bf16> Wb;
 	std::vector<Buf<bf16>> H;  // H[l]: BF16 [members][rows][pd[l]], l = 0..L-1
 	Buf<float> Yp;             // FP32 [members][rows][pd[L]]
-	Buf<float> dz, dh;         // FP32 [members][rows][widest]
-	Buf<bf16> dzb;
+	Buf<float> dz[2];          // FP32 and
+	Buf<bf16> dzb[2];          // BF16 [members][rows][widest]: a layer's output gradient and the one before it
 	Buf<float> loss;           // [members]
 	Buf<float> Xin, Yin;       // batches from the host: [members][rows][in], [members][rows][out]
 	Buf<float> Xd, Yd;         // training set [n][in], [n][out]
@@ -1151,13 +1271,20 @@ constexpr size_t TC_SMEM_MAX = 227 * 1024;
 // The tcgen05 path takes the forward products Z = H W^T whose operands are contiguous
 // K-major rows with K a multiple of 64, N a multiple of 16 up to 256, and whose staged
 // operands fit the shared memory; H is [members][rows][K], W [N][K] per member.
-bool tc_eligible(const mf_mlp* m, bool ta, bool tb, const GemmArgs& g) {
-	return m->tc && !ta && tb && g.K % tc::BK == 0 && g.N % 16 == 0 && g.N <= 256 && g.lda == g.K && g.ldb == g.K &&
+bool tc_eligible(const mf_mlp* m, const GemmArgs& g) {
+	return m->tc && g.K % tc::BK == 0 && g.N % 16 == 0 && g.N <= 256 && g.lda == g.K && g.ldb == g.K &&
 	       g.sA == (long long)m->rows * g.K && g.M <= m->rows && tc::smem_bytes(g.N, g.K) <= TC_SMEM_MAX &&
 	       (!g.Cb || g.ldcb % 8 == 0) && g.sB % 8 == 0;
 }
 
-cudaError_t gemm_tc(mf_mlp* m, const GemmArgs& g) {
+cudaError_t gemm_tc(mf_mlp* m, GemmArgs g) {
+	// With few row tiles (a training batch: 4 a member) one block per tile leaves most SMs
+	// idle and loads all of W first; 64-column slices put four times the blocks to work on
+	// a quarter of W each (512 rows, 5 members, 256 x 256: 9.5 -> 6.1 us).  From half the
+	// SMs on, whole tiles keep W resident and read H once.
+	const int row_tiles = (g.M + tc::BM - 1) / tc::BM;
+	g.n_slice = row_tiles * m->members <= m->sm_count / 2 && g.N > 64 ? 64 : g.N;
+	const int slices = (g.N + g.n_slice - 1) / g.n_slice;
 	EncodeTiled enc = tensor_map_encoder();
 	CUtensorMap tA, tW;
 	// H as [members * rows][K]; boxes of 64 K x 128 rows, 128-byte swizzle, zero fill past the end
@@ -1167,7 +1294,7 @@ cudaError_t gemm_tc(mf_mlp* m, const GemmArgs& g) {
 	// W as [members][N][K] (member stride sB elements); boxes of 64 K x N rows x 1 member
 	const cuuint64_t dW[3] = {(cuuint64_t)g.K, (cuuint64_t)g.N, (cuuint64_t)m->members};
 	const cuuint64_t sW[2] = {(cuuint64_t)g.K * 2, (cuuint64_t)g.sB * 2};
-	const cuuint32_t bW[3] = {tc::BK, (cuuint32_t)g.N, 1};
+	const cuuint32_t bW[3] = {tc::BK, (cuuint32_t)g.n_slice, 1};
 	if (enc(&tA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16*>(g.A), dA, sA, bA, e1,
 	        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
 	        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
@@ -1175,26 +1302,18 @@ cudaError_t gemm_tc(mf_mlp* m, const GemmArgs& g) {
 	        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
 	        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
 		return cudaErrorInvalidValue;
-	const int tiles = (g.M + tc::BM - 1) / tc::BM;
-	const int G = std::max(1, std::min(tiles, m->sm_count / m->members));
-	tc::k_gemm_tc<<<dim3(G, m->members), tc::THREADS, tc::smem_bytes(g.N, g.K), m->stream>>>(tA, tW, g, m->rows,
-	                                                                                         m->dev_err.p);
+	const int G = std::max(1, std::min(row_tiles, m->sm_count / m->members));
+	tc::k_gemm_tc<<<dim3(G, m->members, slices), tc::THREADS, tc::smem_bytes(g.n_slice, g.K), m->stream>>>(
+	    tA, tW, g, m->rows, m->dev_err.p);
 	m->launches++;
 	return cudaGetLastError();
 }
 
-cudaError_t gemm(mf_mlp* m, bool ta, bool tb, GemmArgs g) {
-	dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, m->members);
-	cudaStream_t s = m->stream;
-	if (tc_eligible(m, ta, tb, g)) return gemm_tc(m, g);
-	if (!ta && tb && g.K % 8 == 0 && g.lda % 8 == 0 && g.ldb % 8 == 0 && g.N % 2 == 0 && (!g.C || g.ldc % 2 == 0) &&
-	    (!g.Cb || g.ldcb % 2 == 0)) {
-		dim3 gnt((g.N + NT_BN - 1) / NT_BN, (g.M + NT_BM - 1) / NT_BM, m->members);
-		k_gemm_nt<<<gnt, 256, 0, s>>>(g);
-	} else if (!ta && tb) k_gemm<false, true><<<grid, 128, 0, s>>>(g);
-	else if (!ta && !tb) k_gemm<false, false><<<grid, 128, 0, s>>>(g);
-	else if (ta && !tb) k_gemm<true, false><<<grid, 128, 0, s>>>(g);
-	else k_gemm<true, true><<<grid, 128, 0, s>>>(g);
+// Z = H W^T (the padded widths are multiples of 16, so k_gemm_nt takes what tcgen05 does not)
+cudaError_t gemm(mf_mlp* m, const GemmArgs& g) {
+	if (tc_eligible(m, g)) return gemm_tc(m, g);
+	dim3 gnt((g.N + NT_BN - 1) / NT_BN, (g.M + NT_BM - 1) / NT_BM, m->members);
+	k_gemm_nt<<<gnt, 256, 0, m->stream>>>(g);
 	m->launches++;
 	return cudaGetLastError();
 }
@@ -1316,13 +1435,13 @@ cudaError_t forward_layers(mf_mlp* m, int batch, bool direct_out = false, bool* 
 			g.relu = 1;
 		} else {
 			g.C = m->Yp.p; g.ldc = m->pd[l + 1]; g.sC = sH(m, l + 1);
-			if (direct_out && tc_eligible(m, false, true, g)) {
+			if (direct_out && tc_eligible(m, g)) {
 				g.C = m->Yin.p; g.ldc = m->dims[m->L]; g.sC = (long long)m->rows * m->dims[m->L];
 				g.n_store = m->dims[m->L];
 				if (wrote_direct) *wrote_direct = true;
 			}
 		}
-		cudaError_t e = gemm(m, false, true, g);
+		cudaError_t e = gemm(m, g);
 		if (e != cudaSuccess) return e;
 	}
 	return cudaSuccess;
@@ -1333,44 +1452,36 @@ cudaError_t forward_layers(mf_mlp* m, int batch, bool direct_out = false, bool* 
 cudaError_t backward_layers(mf_mlp* m, const float* y, int batch) {
 	cudaStream_t s = m->stream;
 	const int L = m->L;
-	const long long sdz = (long long)m->rows * m->widest;  // member stride of dz, dh, dzb
+	const long long sdz = (long long)m->rows * m->widest;  // member stride of dz, dzb
+	auto tiles = [](int n) { return (n + tr::T - 1) / tr::T; };
 	k_mse<<<dim3(32, m->members), 256, 0, s>>>(batch, m->dims[L], m->pd[L], m->Yp.p, sH(m, L), y,
-	                                           (long long)m->rows * m->dims[L], m->dz.p, m->dzb.p, sdz, m->loss.p);
+	                                           (long long)m->rows * m->dims[L], m->dz[L & 1].p, m->dzb[L & 1].p, sdz,
+	                                           m->loss.p);
 	m->launches++;
 	for (int l = L - 1; l >= 0; l--) {
-		const int out_p = m->pd[l + 1], in_p = m->pd[l];
-		k_bias_grad<<<dim3(nblk(out_p, 128), m->members), 128, 0, s>>>(batch, out_p, m->dz.p, sdz, m->gB.p + m->b_off[l],
-		                                                               m->b_per);
-		m->launches++;
-		// dW [out x in] = dZ^T [out x batch] . H[l] [batch x in]
-		GemmArgs gw{};
-		gw.M = out_p; gw.N = in_p; gw.K = batch;
-		gw.A = m->dzb.p; gw.lda = out_p; gw.sA = sdz;
-		gw.B = m->H[l].p; gw.ldb = in_p; gw.sB = sH(m, l);
-		gw.C = m->gW.p + m->w_off[l]; gw.ldc = in_p; gw.sC = m->w_per;
-		cudaError_t e = gemm(m, true, false, gw);
-		if (e != cudaSuccess) return e;
-		if (l == 0) break;
-		// dH [batch x in] = dZ [batch x out] . W [out x in]
-		GemmArgs gx{};
-		gx.M = batch; gx.N = in_p; gx.K = out_p;
-		gx.A = m->dzb.p; gx.lda = out_p; gx.sA = sdz;
-		gx.B = m->Wb.p + m->w_off[l]; gx.ldb = in_p; gx.sB = m->w_per;
-		gx.C = m->dh.p; gx.ldc = in_p; gx.sC = sdz;
-		if ((e = gemm(m, false, false, gx)) != cudaSuccess) return e;
-		const long long per = (long long)batch * in_p;
-		k_relu_bwd<<<nblk(per * m->members, 256), 256, 0, s>>>(m->members, per, m->dh.p, sdz, m->H[l].p, sH(m, l), m->dz.p,
-		                                                      m->dzb.p, sdz);
+		tr::Bwd g{};
+		g.batch = batch; g.out_p = m->pd[l + 1]; g.in_p = m->pd[l];
+		g.dz = m->dzb[(l + 1) & 1].p; g.dzf = m->dz[(l + 1) & 1].p; g.sDz = sdz;
+		g.H = m->H[l].p; g.sHin = sH(m, l);
+		g.W = m->Wb.p + m->w_off[l]; g.sW = m->w_per;
+		g.gW = m->gW.p + m->w_off[l]; g.sGw = m->w_per;
+		g.gB = m->gB.p + m->b_off[l]; g.sGb = m->b_per;
+		g.dz_prev = m->dzb[l & 1].p; g.dzf_prev = m->dz[l & 1].p;
+		g.w_tiles = tiles(g.out_p) * tiles(g.in_p);
+		g.b_tiles = tiles(g.out_p);
+		const int x_tiles = l > 0 ? tiles(batch) * tiles(g.in_p) : 0;
+		tr::k_backward<<<dim3(g.w_tiles + g.b_tiles + x_tiles, m->members), tr::THREADS, tr::SMEM, s>>>(g);
 		m->launches++;
 	}
 	return cudaGetLastError();
 }
 
 cudaError_t adam_update(mf_mlp* m) {
-	const long long nw = m->w_per * m->members, nb = m->b_per * m->members;
-	k_adam<<<nblk(nw, 256), 256, 0, m->stream>>>(m->ctl.p, nw, m->W.p, m->gW.p, m->mW.p, m->vW.p, m->Wb.p);
-	k_adam<<<nblk(nb, 256), 256, 0, m->stream>>>(m->ctl.p, nb, m->Bias.p, m->gB.p, m->mB.p, m->vB.p, nullptr);
-	m->launches += 2;
+	const AdamSet w{m->w_per * m->members, m->W.p, m->gW.p, m->mW.p, m->vW.p, m->Wb.p};
+	const AdamSet b{m->b_per * m->members, m->Bias.p, m->gB.p, m->mB.p, m->vB.p, nullptr};
+	const unsigned wb = nblk(w.n, 1024);
+	k_adam<<<wb + nblk(b.n, 1024), 256, 0, m->stream>>>(m->ctl.p, w, b, wb);
+	m->launches++;
 	return cudaGetLastError();
 }
 
@@ -1378,10 +1489,10 @@ cudaError_t adam_update(mf_mlp* m) {
 cudaError_t train_step_launches(mf_mlp* m) {
 	cudaStream_t s = m->stream;
 	const int out = m->dims[m->L];
-	k_step_begin<<<1, 64, 0, s>>>(m->ctl.p, m->loss.p, m->members);
-	k_gather<<<dim3(m->rows, m->members), 32, 0, s>>>(m->ctl.p, m->dims[0], m->pd[0], out, sH(m, 0),
-	                                                  (long long)m->rows * out, m->Xd.p, m->Yd.p, m->H[0].p, m->Yin.p);
-	m->launches += 2;
+	k_gather<<<dim3((m->rows + 3) / 4, m->members), 128, 0, s>>>(m->ctl.p, m->rows, m->dims[0], m->pd[0], out, sH(m, 0),
+	                                                             (long long)m->rows * out, m->Xd.p, m->Yd.p, m->H[0].p,
+	                                                             m->Yin.p);
+	m->launches++;
 	cudaError_t e;
 	if ((e = forward_layers(m, m->rows)) != cudaSuccess) return e;
 	if ((e = backward_layers(m, m->Yin.p, m->rows)) != cudaSuccess) return e;
@@ -1495,9 +1606,11 @@ MF_API mf_status mf_mlp_create(const mf_mlp_config* cfg, mf_mlp** out) {
 		for (int l = 0; l < m->L; l++) MCK(m->H[l].alloc((size_t)m->members * sH(m, l)));
 		const size_t act = (size_t)m->members * m->rows * m->widest;
 		MCK(m->Yp.alloc((size_t)m->members * sH(m, m->L)));
-		MCK(m->dz.alloc(act));
-		MCK(m->dh.alloc(act));
-		MCK(m->dzb.alloc(act));
+		for (int k = 0; k < 2; k++) {
+			MCK(m->dz[k].alloc(act));
+			MCK(m->dzb[k].alloc(act));
+		}
+		MCK(cudaFuncSetAttribute(tr::k_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tr::SMEM));
 		MCK(m->loss.alloc(m->members));
 		MCK(m->Xin.alloc((size_t)m->members * m->rows * m->dims[0]));
 		MCK(m->Yin.alloc((size_t)m->members * m->rows * m->dims[m->L]));
@@ -1656,6 +1769,7 @@ MF_API mf_status mf_mlp_train(mf_mlp* m, int32_t steps, float lr0, float lr1, fl
 		}
 	}
 	m->wf_dirty = true;
+	MCK(cudaMemsetAsync(m->loss.p, 0, m->members * 4, s));  // (each step leaves it zero for the next)
 	for (int t = 0; t < steps; t++) MCK(cudaGraphLaunch(m->graph, s));
 	m->launches += m->step_launches * (uint64_t)steps;
 	if (loss_history)
