@@ -51,6 +51,10 @@ enum : uint32_t {
 	A_ADVECTION = 1u << 11,
 	A_GOD_CONT = mfk_host::FLAG_GODUNOV_CONTINUITY,
 	A_GOD_MOM = mfk_host::FLAG_GODUNOV_MOMENTUM,
+	// the whole Gray-Monaghan list (rings.cpp:86-96): the mixed pair pass is compiled for it,
+	// so that no pair tests a flag
+	A_MONAGHAN = A_RIEMANN | A_EOS | A_ART_STRESS | A_STRESS_MGHN | A_DERIVE_VEL | A_ART_VISC | A_XSPH | A_JAUMANN |
+	             A_CONTINUITY | A_MOMENTUM_UL | A_ADVECTION,
 };
 
 // Cell-ordered record of one particle's stage state plus per-particle derived
@@ -63,7 +67,7 @@ struct __align__(16) Rec64 {
 	double sxy, syy, Rxx, Rxy;
 	double Ryy, c, qw, rho21;  // c = sqrt(K/rho), qw = m/rho (or the stored weight), rho21 = 1/rho^2
 };
-// Mixed form: positions and velocities as float-float, the rest FP32: 80 bytes.
+// Mixed form: positions and velocities as float-float, the rest FP32: five 16-byte parts.
 struct __align__(16) Rec32 {
 	FF x, y, vx, vy;
 	float m, h, rho, sxx;
@@ -79,23 +83,22 @@ __device__ __forceinline__ Rec64 load_rec(const Rec64* p) {
 	for (int i = 0; i < 8; i++) d[i] = __ldg(s + i);
 	return r;
 }
-__device__ __forceinline__ Rec32 load_rec(const Rec32* p) {
+// The mixed records are stored as five float4 arrays of n rows (16-byte part f of row k at
+// rec[f * n + k]): the 32 lanes of a warp reach the same part of mostly consecutive rows,
+// 4 cache lines an access where 80-byte records spread it over 20 (with them the L1 data
+// pipe was 60 % busy in the pair pass).
+__device__ __forceinline__ Rec32 load_rec(const float4* rec, size_t n, uint32_t k, float4 head) {
 	Rec32 r;
-	const float4* s = reinterpret_cast<const float4*>(p);
 	float4* d = reinterpret_cast<float4*>(&r);
+	d[0] = head;  // (x, y: already loaded)
 #pragma unroll
-	for (int i = 0; i < 5; i++) d[i] = __ldg(s + i);
+	for (int f = 1; f < 5; f++) d[f] = __ldg(rec + f * n + k);
 	return r;
 }
-// the rest of a record whose first 16 bytes (x, y) are already loaded
-__device__ __forceinline__ Rec32 load_rec_tail(const Rec32* p, float4 head) {
-	Rec32 r;
-	const float4* s = reinterpret_cast<const float4*>(p);
-	float4* d = reinterpret_cast<float4*>(&r);
-	d[0] = head;
+__device__ __forceinline__ void store_rec(float4* rec, size_t n, uint32_t k, const Rec32& r) {
+	const float4* s = reinterpret_cast<const float4*>(&r);
 #pragma unroll
-	for (int i = 1; i < 5; i++) d[i] = __ldg(s + i);
-	return r;
+	for (int f = 0; f < 5; f++) rec[f * n + k] = s[f];
 }
 
 // ------------------------------------------------------- per-body failures
@@ -389,18 +392,17 @@ __device__ __forceinline__ void per_particle32(uint32_t flags, const BodyParams&
 	float sxx = Sxx - p, syy = Syy - p, sxy = Sxy;
 	Rxx = Rxy = Ryy = 0.f;
 	if (flags & A_ART_STRESS) {
-		float eps = pr.fmghn_eps;
-		float theta = 0.5f * atan2f(2.f * sxy, sxx - syy + 0.f);
-		float cs = cosf(theta), sn = sinf(theta);
-		float cs2 = cs * cs, sn2 = sn * sn;
-		float rot_sxx = cs2 * sxx + 2.f * cs * sn * sxy + sn2 * syy;
-		float rot_syy = sn2 * sxx - 2.f * cs * sn * sxy + cs2 * syy;
-		float rot_rxx = 0.f, rot_ryy = 0.f;
-		if (rot_sxx > 0.f) rot_rxx = -eps * rot_sxx / (rho * rho);
-		if (rot_syy > 0.f) rot_ryy = -eps * rot_syy / (rho * rho);
-		Rxx = cs2 * rot_rxx + sn2 * rot_ryy;
-		Rxy = cs * sn * (rot_rxx - rot_ryy);
-		Ryy = sn2 * rot_rxx + cs2 * rot_ryy;
+		// principal stresses from the stress circle; cos 2 theta and sin 2 theta (halved) as
+		// its components over its radius, in place of atan2f, cosf and sinf of the angle
+		const float dev = sxx - syy, twice = 2.f * sxy, mean = 0.5f * (sxx + syy);
+		const float R2 = dev * dev + twice * twice;
+		const float R1 = R2 > 1e-30f ? rsqrtf(R2) : 0.f, radius = 0.5f * R2 * R1;
+		const float c2 = R2 > 1e-30f ? 0.5f * dev * R1 : 0.5f, s2 = 0.5f * twice * R1;
+		const float eps = -pr.fmghn_eps / (rho * rho);
+		const float ra = eps * fmaxf(mean + radius, 0.f), rb = eps * fmaxf(mean - radius, 0.f);
+		Rxx = (0.5f + c2) * ra + (0.5f - c2) * rb;
+		Ryy = (0.5f - c2) * ra + (0.5f + c2) * rb;
+		Rxy = s2 * (ra - rb);
 	}
 	sxx_o = sxx;
 	syy_o = syy;
@@ -479,9 +481,9 @@ __global__ void k_gather64(ULArgs a, const BodyParams* __restrict__ P) {
 	a.rec_body[k] = b;
 }
 
-// The record of particle i (body parameters pr) from its stage state, into out.
-__device__ __forceinline__ void put_rec32(const ULArgs& a, const BodyParams& pr, uint32_t i, Rec32* out, double x,
-                                          double y, double vx, double vy, float rho_dev, float Sxx, float Sxy,
+// The record of particle i (body parameters pr) from its stage state, as row k of rec.
+__device__ __forceinline__ void put_rec32(const ULArgs& a, const BodyParams& pr, uint32_t i, void* rec, uint32_t k,
+                                          double x, double y, double vx, double vy, float rho_dev, float Sxx, float Sxy,
                                           float Syy) {
 	const float rho = rho_dev + pr.frho0;  // the mixed state holds rho - rho0
 	Rec32 r;
@@ -493,11 +495,13 @@ __device__ __forceinline__ void put_rec32(const ULArgs& a, const BodyParams& pr,
 	if (a.flags & (A_GOD_CONT | A_GOD_MOM)) {  // p from the stored deviation, the stress Syy itself
 		r.Rxx = (a.flags & A_EOS) ? pr.fc0sq * rho_dev : 0.f;
 		r.Rxy = Syy;
+	} else {  // pair32_fast takes the stresses times 1/rho^2 and c times alpha / 2
+		r.c *= 0.5f * pr.falpha;
+		r.sxx *= r.rho21;
+		r.sxy *= r.rho21;
+		r.syy *= r.rho21;
 	}
-	const float4* s = reinterpret_cast<const float4*>(&r);
-	float4* d = reinterpret_cast<float4*>(out);
-#pragma unroll
-	for (int q = 0; q < 5; q++) d[q] = s[q];
+	store_rec(reinterpret_cast<float4*>(rec), a.n_total, k, r);
 }
 
 __global__ void k_gather32(ULArgs a, const BodyParams* __restrict__ P) {
@@ -509,7 +513,7 @@ __global__ void k_gather32(ULArgs a, const BodyParams* __restrict__ P) {
 	float rho, Sxx, Sxy, Syy;
 	v.load(i, x, y, vx, vy, rho, Sxx, Sxy, Syy);
 	uint32_t b = a.body_of[i];
-	put_rec32(a, P[b], i, reinterpret_cast<Rec32*>(a.rec) + k, x, y, vx, vy, rho, Sxx, Sxy, Syy);
+	put_rec32(a, P[b], i, a.rec, k, x, y, vx, vy, rho, Sxx, Sxy, Syy);
 	a.rec_body[k] = b;
 }
 
@@ -976,124 +980,223 @@ __global__ void __launch_bounds__(P64_THREADS) k_pair64(ULArgs a, const BodyPara
 }
 
 // ---------------------------------------------------------- pair kernel mixed
+// Instruction issue (60 % of the slots), the L1 data pipe (60 %) and the L2 reads behind it
+// bound these kernels together, so the Gray-Monaghan pair terms are written for few
+// instructions, as in pair64_fast: ~75 FP32 operations a pair against ~120 in the
+// reference's expressions, no flag tests in the whole list's instance, the records as
+// arrays.  Ensemble of 64 ring impacts (1.35M rows), per stage: 373 -> 285 us.  Measured
+// and not kept: a list over all stencil columns in shared memory (fewer evaluations, 21
+// against 25 a row, but the lanes drift apart: 300 against 271 us alone), 8-byte relative
+// positions for the candidate tests (303: the tests on the records' own positions bring
+// the lines that the pair terms read next), cells in blocks of 8 x 16 (381), a warp's
+// records of the next column prefetched into L1 (285).
+
+// The pair sums of one row (or a lane's share of them)
+struct Acc32 {
+	float Sxx_x = 0.f, Sxy_y = 0.f, Sxy_x = 0.f, Syy_y = 0.f;
+	float vx_x = 0.f, vx_y = 0.f, vy_x = 0.f, vy_y = 0.f;
+	float av_x = 0.f, av_y = 0.f, xs_x = 0.f, xs_y = 0.f;
+	float god_rho = 0.f, god_vx = 0.f, god_vy = 0.f;
+};
+// Per-row constants of the pair terms (the parameters' FP32 copies: a conversion, let
+// alone a division, in FP64 would run on the narrow FP64 pipe for every row)
+struct Row32 {
+	float h1, fac;                          // 1 / h, 10 / (7 pi h^2)
+	float w_wdp, eta2q, half_beta, corr_exp;
+	bool stress, art;
+};
+
+// 1/x and 1/sqrt(x) by the special-function unit alone (2 ulp, no rescaling of
+// subnormals: r^2, eta^2 h^2 and densities are far above them)
+__device__ __forceinline__ float rcp_approx(float x) {
+	float y;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+	return y;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+	float y;
+	asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+	return y;
+}
+
+// The Gray-Monaghan pair terms at the offset (xij, yij) = x_i - x_j, r2 its square.
+__device__ __forceinline__ void pair32_fast(uint32_t flags, const Row32& k, const Rec32& ri, const Rec32& rj, float xij,
+                                            float yij, float r2, Acc32& s) {
+	// W = fac (t^3 / 4 - u^3), |grad W| = 3 fac (t^2 / 4 - u^2) / h with t = 2 - q,
+	// u = max(1 - q, 0) (t clamped at 0 beyond 2h); 3 fac is applied to the row's sums
+	const float sr = r2 > 1e-24f ? rsqrt_approx(r2) * k.h1 : 0.f;  // 1 / (r h); kernel.cpp's r > 1e-12
+	const float q = r2 * sr;
+	const float t = fmaxf(2.f - q, 0.f), u = fmaxf(1.f - q, 0.f);
+	const float u2 = u * u, t2q = 0.25f * t * t;
+	const float w = t2q * t - u2 * u;
+	const float g = (u2 - t2q) * sr;
+	const float gx = xij * g, gy = yij * g;
+	const float dvx = ff_diff(rj.vx, ri.vx), dvy = ff_diff(rj.vy, ri.vy);
+	const float inv_rs = rcp_approx(ri.rho + rj.rho);
+	float piij = 0.f;
+	if (flags & A_ART_VISC) {
+		const float dot = dvx * xij + dvy * yij;  // -v_ij . x_ij
+		const float hs = ri.h + rj.h;
+		const float mu2 = hs * dot * rcp_approx(r2 + k.eta2q * hs * hs);  // -2 mu_ij
+		const float p = mu2 * (k.half_beta * mu2 + (ri.c + rj.c)) * inv_rs;
+		piij = dot > 0.f ? p : 0.f;  // approaching
+	}
+	if (k.stress) {  // the records' stresses are already times 1/rho^2
+		float txx = ri.sxx + rj.sxx, txy = ri.sxy + rj.sxy, tyy = ri.syy + rj.syy;
+		if (k.art) {
+			float fab = w * k.w_wdp;
+			if (k.corr_exp == 4.f) {
+				fab *= fab;
+				fab *= fab;
+			} else {
+				fab = powf(fab, k.corr_exp);
+			}
+			txx += fab * (ri.Rxx + rj.Rxx);
+			txy += fab * (ri.Rxy + rj.Rxy);
+			tyy += fab * (ri.Ryy + rj.Ryy);
+		}
+		const float mx = rj.m * gx, my = rj.m * gy;
+		s.av_x += (txx - piij) * mx + txy * my;
+		s.av_y += txy * mx + (tyy - piij) * my;
+	} else if (flags & A_ART_VISC) {
+		const float mp = rj.m * piij;
+		s.av_x -= mp * gx;
+		s.av_y -= mp * gy;
+	}
+	if (flags & A_DERIVE_VEL) {
+		const float qx = rj.qw * gx, qy = rj.qw * gy;
+		s.vx_x += dvx * qx;
+		s.vx_y += dvx * qy;
+		s.vy_x += dvy * qx;
+		s.vy_y += dvy * qy;
+	}
+	if (flags & A_XSPH) {
+		const float f = w * inv_rs;
+		s.xs_x += f * dvx;
+		s.xs_y += f * dvy;
+	}
+}
+
+// The pair terms of a pipeline with Godunov actions, in the reference's expressions.
+__device__ __forceinline__ void pair32_godunov(uint32_t flags, const BodyParams& pr, const Row32& k, const Rec32& ri,
+                                               const Rec32& rj, float xij, float yij, float r2, Acc32& s) {
+	KR32 w = cubic_spline_f(xij, yij, k.h1, k.fac);
+	if (flags & A_STRESS_MGHN) {
+		float Rxx = 0.f, Rxy = 0.f, Ryy = 0.f;
+		if (pr.fwdp1 > 0.f) {
+			float fab = w.w * pr.fwdp1;
+			if (pr.fcorr_exp == 4.f) {
+				float f2 = fab * fab;
+				fab = f2 * f2;
+			} else {
+				fab = powf(fab, pr.fcorr_exp);
+			}
+			Rxx = fab * (ri.Rxx + rj.Rxx);
+			Rxy = fab * (ri.Rxy + rj.Rxy);
+			Ryy = fab * (ri.Ryy + rj.Ryy);
+		}
+		float tsx = rj.m * (ri.sxy * ri.rho21 + rj.sxy * rj.rho21 + Rxy);
+		s.Sxx_x += rj.m * (ri.sxx * ri.rho21 + rj.sxx * rj.rho21 + Rxx) * w.w_x;
+		s.Sxy_y += tsx * w.w_y;
+		s.Sxy_x += tsx * w.w_x;
+		s.Syy_y += rj.m * (ri.syy * ri.rho21 + rj.syy * rj.rho21 + Ryy) * w.w_y;
+	}
+	float dvx = ff_diff(rj.vx, ri.vx), dvy = ff_diff(rj.vy, ri.vy);
+	if (flags & A_DERIVE_VEL) {
+		float qx = w.w_x * rj.qw, qy = w.w_y * rj.qw;
+		s.vx_x += dvx * qx;
+		s.vx_y += dvx * qy;
+		s.vy_x += dvy * qx;
+		s.vy_y += dvy * qy;
+	}
+	if (flags & A_ART_VISC) {
+		float vijposij = -(dvx * xij + dvy * yij);
+		if (vijposij < 0.f) {
+			float cij = 0.5f * (ri.c + rj.c);
+			float hij = 0.5f * (ri.h + rj.h);
+			float rhoij = 0.5f * (ri.rho + rj.rho);
+			float muij = __fdividef(hij * vijposij, r2 + pr.feta2 * hij * hij);
+			float piij = __fdividef(-pr.falpha * cij * muij + pr.fbeta * muij * muij, rhoij);
+			s.av_x += -rj.m * piij * w.w_x;
+			s.av_y += -rj.m * piij * w.w_y;
+		}
+	}
+	if (flags & A_XSPH) {
+		float rhoij = 0.5f * (ri.rho + rj.rho);
+		float f = __fdividef(-pr.fxsph_eps * w.w * ri.m, rhoij);
+		s.xs_x -= f * dvx;
+		s.xs_y -= f * dvy;
+	}
+	{
+		// godunov_continuity / godunov_momentum (godunov.h:86-187) in FP32: velocity
+		// differences from the float-float records, the Riemann state in the form
+		// v_i - u* = (Z_j (v_i - v_j).n + p_i - p_j) / (Z_i + Z_j), Z = rho c;
+		// Rxx holds p, Rxy the stress Syy itself
+		const float mag_r = sqrtf(r2), inv = 1.f / mag_r;
+		const float Zi = ri.rho * ri.c, Zj = rj.rho * rj.c;
+		const float frac = 1.f / (Zi + Zj);
+		if (flags & A_GOD_CONT) {
+			float nx = xij * inv, ny = yij * inv;
+			float dvn = -(dvx * nx + dvy * ny);  // (v_i - v_j).n
+			float vi_us = frac * (Zj * dvn + (ri.Rxx - rj.Rxx));
+			s.god_rho += 2.f * ri.rho * vi_us * (w.w_x * nx + w.w_y * ny) * rj.qw;
+		}
+		if (flags & A_GOD_MOM) {
+			float rx = -xij, ry = -yij;
+			float Rx = rx * inv, Ry = ry * inv, Sx = ry * inv, Sy = -rx * inv;  // the float frame
+			float siR0 = ri.sxx * Rx + ri.sxy * Ry;
+			float sjR0 = rj.sxx * Rx + rj.sxy * Ry, sjR1 = rj.sxy * Rx + rj.Rxy * Ry;
+			float si0 = Rx * siR0 + Sx * (ri.sxy * Rx + ri.Rxy * Ry);
+			float sj0 = Rx * sjR0 + Sx * sjR1, sj1 = Ry * sjR0 + Sy * sjR1;
+			float dv0 = Rx * dvx + Sx * dvy, dv1 = Ry * dvx + Sy * dvy;  // frame (v_j - v_i)
+			// the second component takes sigma_j twice (godunov.h:116), as the reference does
+			float S0 = frac * (sj0 * Zi + si0 * Zj + Zi * Zj * dv0);
+			float S1 = frac * (sj1 * Zi + sj1 * Zj + Zi * Zj * dv1);
+			float SR0 = Rx * S0 + Ry * S1, SR1 = Sx * S0 + Sy * S1;
+			if (fabsf(rx) > 0.f) s.god_vx += (2.f / ri.rho) * __fdividef(w.w_x * mag_r, rx) * SR0 * rj.qw;
+			if (fabsf(ry) > 0.f) s.god_vy += (2.f / ri.rho) * __fdividef(w.w_y * mag_r, ry) * SR1 * rj.qw;
+		}
+	}
+}
+
 // L threads per row (L = 1: one thread walks the row's whole stencil): lane takes every
 // L-th candidate of each stencil row, the partial sums are added across the L lanes,
 // and lane 0 finishes the row.  L > 1 puts more rows' work in flight when the rows are
 // few (the launch would otherwise cover a handful of SMs); it changes the order of the
 // pair sums, not their terms.
-template <bool GOD, int L = 1>
+template <bool GOD, bool FULL, int L = 1>
 __device__ __forceinline__ void pair32_row(const ULArgs& a, const BodyParams* __restrict__ P,
                                            const Geom* __restrict__ G, DevStatus* st, uint32_t k,
                                            uint32_t lane = 0) {
 	uint32_t b = a.rec_body[k];
 	if (is_failed(a.failed, b)) return;  // a failed body stays as it was (all L lanes of the row)
-	const Rec32* rec = reinterpret_cast<const Rec32*>(a.rec);
-	const Rec32 ri = load_rec(rec + k);
+	const float4* rec = reinterpret_cast<const float4*>(a.rec);
+	const size_t n = a.n_total;
+	const Rec32 ri = load_rec(rec, n, k, __ldg(rec + k));
 	const BodyParams& pr = P[b];
 	Geom g = G[b];
 	uint32_t i = a.perm[k];
-	uint32_t flags = a.flags;
+	const uint32_t flags = FULL ? A_MONAGHAN : a.flags;
 	int lo_i, hi_i, lo_j, hi_j;
 	stencil(g, a.keys_sorted[k], lo_i, hi_i, lo_j, hi_j);
 	const uint32_t tot = *a.total_cells;
 
-	float hi = ri.h;
-	float h1 = 1.f / hi;
-	float fac = (float)(10 * (K_1_PI) / 7.0) * h1 * h1;
-	float reach2 = 4.0001f * hi * hi;
-	float rhoi21 = ri.rho21;
-	// the parameters' FP32 copies: a conversion (let alone a division) in FP64 would run
-	// on the narrow FP64 pipe for every row
-	float wdp1 = pr.fwdp1;
-	bool exp4 = pr.fcorr_exp == 4.f;
-	float corr_exp = pr.fcorr_exp;
-	float alpha = pr.falpha, beta = pr.fbeta, eta2 = pr.feta2, xeps = pr.fxsph_eps;
-
-	float Sxx_x = 0.f, Sxy_y = 0.f, Sxy_x = 0.f, Syy_y = 0.f;
-	float vx_x = 0.f, vx_y = 0.f, vy_x = 0.f, vy_y = 0.f;
-	float av_x = 0.f, av_y = 0.f, xs_x = 0.f, xs_y = 0.f;
-	float god_rho = 0.f, god_vx = 0.f, god_vy = 0.f;
-	const float two_rhoi = 2.f / ri.rho;
+	Row32 rk;
+	rk.h1 = 1.f / ri.h;
+	rk.fac = (float)(10 * (K_1_PI) / 7.0) * rk.h1 * rk.h1;
+	rk.art = pr.fwdp1 > 0.f;
+	rk.w_wdp = rk.fac * pr.fwdp1;
+	rk.eta2q = 0.25f * pr.feta2;
+	rk.half_beta = 0.5f * pr.fbeta;
+	rk.corr_exp = pr.fcorr_exp;
+	rk.stress = (flags & A_MOMENTUM_UL) != 0;
+	const float reach2 = 4.0001f * ri.h * ri.h;
+	Acc32 s;
 	// the pair terms of candidate kj within reach (xij, yij: x_i - x_j; r2 = |x_i - x_j|^2)
 	auto pair = [&](uint32_t kj, float4 head, float xij, float yij, float r2) {
-		const Rec32 rj = load_rec_tail(rec + kj, head);
-		KR32 w = cubic_spline_f(xij, yij, h1, fac);
-		if (flags & A_STRESS_MGHN) {
-			float Rxx = 0.f, Rxy = 0.f, Ryy = 0.f;
-			if (wdp1 > 0.f) {
-				float fab = w.w * wdp1;
-				if (exp4) {
-					float f2 = fab * fab;
-					fab = f2 * f2;
-				} else {
-					fab = powf(fab, corr_exp);
-				}
-				Rxx = fab * (ri.Rxx + rj.Rxx);
-				Rxy = fab * (ri.Rxy + rj.Rxy);
-				Ryy = fab * (ri.Ryy + rj.Ryy);
-			}
-			float tsx = rj.m * (ri.sxy * rhoi21 + rj.sxy * rj.rho21 + Rxy);
-			Sxx_x += rj.m * (ri.sxx * rhoi21 + rj.sxx * rj.rho21 + Rxx) * w.w_x;
-			Sxy_y += tsx * w.w_y;
-			Sxy_x += tsx * w.w_x;
-			Syy_y += rj.m * (ri.syy * rhoi21 + rj.syy * rj.rho21 + Ryy) * w.w_y;
-		}
-		float dvx = ff_diff(rj.vx, ri.vx), dvy = ff_diff(rj.vy, ri.vy);
-		if (flags & A_DERIVE_VEL) {
-			float qx = w.w_x * rj.qw, qy = w.w_y * rj.qw;
-			vx_x += dvx * qx;
-			vx_y += dvx * qy;
-			vy_x += dvy * qx;
-			vy_y += dvy * qy;
-		}
-		if (flags & A_ART_VISC) {
-			float vijposij = -(dvx * xij + dvy * yij);
-			if (vijposij < 0.f) {
-				float cij = 0.5f * (ri.c + rj.c);
-				float hij = 0.5f * (hi + rj.h);
-				float rhoij = 0.5f * (ri.rho + rj.rho);
-				float muij = __fdividef(hij * vijposij, r2 + eta2 * hij * hij);
-				float piij = __fdividef(-alpha * cij * muij + beta * muij * muij, rhoij);
-				av_x += -rj.m * piij * w.w_x;
-				av_y += -rj.m * piij * w.w_y;
-			}
-		}
-		if (flags & A_XSPH) {
-			float rhoij = 0.5f * (ri.rho + rj.rho);
-			float f = __fdividef(-xeps * w.w * ri.m, rhoij);
-			xs_x -= f * dvx;
-			xs_y -= f * dvy;
-		}
-		if (GOD && kj != k) {
-			// godunov_continuity / godunov_momentum (godunov.h:86-187) in FP32: velocity
-			// differences from the float-float records, the Riemann state in the form
-			// v_i - u* = (Z_j (v_i - v_j).n + p_i - p_j) / (Z_i + Z_j), Z = rho c;
-			// Rxx holds p, Rxy the stress Syy itself
-			const float mag_r = sqrtf(r2), inv = 1.f / mag_r;
-			const float Zi = ri.rho * ri.c, Zj = rj.rho * rj.c;
-			const float frac = 1.f / (Zi + Zj);
-			if (flags & A_GOD_CONT) {
-				float nx = xij * inv, ny = yij * inv;
-				float dvn = -(dvx * nx + dvy * ny);  // (v_i - v_j).n
-				float vi_us = frac * (Zj * dvn + (ri.Rxx - rj.Rxx));
-				god_rho += 2.f * ri.rho * vi_us * (w.w_x * nx + w.w_y * ny) * rj.qw;
-			}
-			if (flags & A_GOD_MOM) {
-				float rx = -xij, ry = -yij;
-				float Rx = rx * inv, Ry = ry * inv, Sx = ry * inv, Sy = -rx * inv;  // the float frame
-				float siR0 = ri.sxx * Rx + ri.sxy * Ry;
-				float sjR0 = rj.sxx * Rx + rj.sxy * Ry, sjR1 = rj.sxy * Rx + rj.Rxy * Ry;
-				float si0 = Rx * siR0 + Sx * (ri.sxy * Rx + ri.Rxy * Ry);
-				float sj0 = Rx * sjR0 + Sx * sjR1, sj1 = Ry * sjR0 + Sy * sjR1;
-				float dv0 = Rx * dvx + Sx * dvy, dv1 = Ry * dvx + Sy * dvy;  // frame (v_j - v_i)
-				// the second component takes sigma_j twice (godunov.h:116), as the reference does
-				float S0 = frac * (sj0 * Zi + si0 * Zj + Zi * Zj * dv0);
-				float S1 = frac * (sj1 * Zi + sj1 * Zj + Zi * Zj * dv1);
-				float SR0 = Rx * S0 + Ry * S1, SR1 = Sx * S0 + Sy * S1;
-				if (fabsf(rx) > 0.f) god_vx += two_rhoi * __fdividef(w.w_x * mag_r, rx) * SR0 * rj.qw;
-				if (fabsf(ry) > 0.f) god_vy += two_rhoi * __fdividef(w.w_y * mag_r, ry) * SR1 * rj.qw;
-			}
-		}
+		const Rec32 rj = load_rec(rec, n, kj, head);
+		if (GOD) pair32_godunov(flags, pr, rk, ri, rj, xij, yij, r2, s);
+		else pair32_fast(flags, rk, ri, rj, xij, yij, r2, s);
 	};
 	// candidate offsets and squared distance, one rounding each (the same values in both
 	// walks below)
@@ -1114,13 +1217,14 @@ __device__ __forceinline__ void pair32_row(const ULArgs& a, const BodyParams* __
 			uint32_t mask = 0u;
 			for (uint32_t kj = j0; kj < j1; kj++) {
 				float xij, yij;
-				const float r2 = offs(__ldg(reinterpret_cast<const float4*>(rec + kj)), xij, yij);
+				const float r2 = offs(__ldg(rec + kj), xij, yij);
 				if (!(r2 > reach2)) mask |= 1u << (kj - j0);
 			}
+			if (k - j0 < 32u) mask &= ~(1u << (k - j0));  // (the row itself adds nothing to any sum)
 			while (mask) {
 				const uint32_t kj = j0 + (uint32_t)(__ffs(mask) - 1);
 				mask &= mask - 1u;
-				const float4 head = __ldg(reinterpret_cast<const float4*>(rec + kj));
+				const float4 head = __ldg(rec + kj);
 				float xij, yij;
 				const float r2 = offs(head, xij, yij);
 				pair(kj, head, xij, yij, r2);
@@ -1128,43 +1232,52 @@ __device__ __forceinline__ void pair32_row(const ULArgs& a, const BodyParams* __
 		} else {
 			for (uint32_t kj = j0 + lane; kj < j1; kj += L) {
 				// positions first: most candidates of the stencil lie beyond the reach
-				const float4 head = __ldg(reinterpret_cast<const float4*>(rec + kj));
+				const float4 head = __ldg(rec + kj);
 				float xij, yij;
 				const float r2 = offs(head, xij, yij);
-				if (r2 > reach2) continue;
+				if (r2 > reach2 || kj == k) continue;
 				pair(kj, head, xij, yij, r2);
 			}
 		}
 	}
 	if (L > 1) {
 		const unsigned gmask = ((1u << L) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(L - 1));
-		float* acc[15] = {&Sxx_x, &Sxy_y, &Sxy_x, &Syy_y, &vx_x, &vx_y, &vy_x, &vy_y,
-		                  &av_x, &av_y, &xs_x, &xs_y, &god_rho, &god_vx, &god_vy};
+		constexpr int NS = GOD ? 15 : 8;
+		float* acc[15] = {&s.vx_x, &s.vx_y, &s.vy_x, &s.vy_y, &s.av_x, &s.av_y, &s.xs_x, &s.xs_y,
+		                  &s.Sxx_x, &s.Sxy_y, &s.Sxy_x, &s.Syy_y, &s.god_rho, &s.god_vx, &s.god_vy};
 #pragma unroll
-		for (int q = 0; q < 15; q++)
+		for (int q = 0; q < NS; q++)
 #pragma unroll
 			for (int o = L / 2; o > 0; o >>= 1) *acc[q] += __shfl_xor_sync(gmask, *acc[q], o, L);
 		if (lane != 0) return;
 	}
 	float d[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-	float rhoi = ri.rho;
-	if (flags & A_STRESS_MGHN) { Sxx_x *= rhoi; Sxy_y *= rhoi; Sxy_x *= rhoi; Syy_y *= rhoi; }
-	if (flags & A_ART_VISC) { d[2] = av_x; d[3] = av_y; }
-	if (flags & A_XSPH) { d[0] = xs_x; d[1] = xs_y; }
-	float vxi = ri.vx.hi + ri.vx.lo, vyi = ri.vy.hi + ri.vy.lo;
+	const float rhoi = ri.rho;
+	if (!GOD) {  // the factors that pair32_fast left out
+		const float gsc = 3.f * rk.fac, xsc = 2.f * pr.fxsph_eps * ri.m * rk.fac;
+		s.av_x *= gsc; s.av_y *= gsc;
+		s.vx_x *= gsc; s.vx_y *= gsc; s.vy_x *= gsc; s.vy_y *= gsc;
+		s.xs_x *= xsc; s.xs_y *= xsc;
+	}
+	if ((flags & A_ART_VISC) || (!GOD && rk.stress)) { d[2] = s.av_x; d[3] = s.av_y; }
+	if (flags & A_XSPH) { d[0] = s.xs_x; d[1] = s.xs_y; }
 	if (flags & A_JAUMANN) {
 		const mfk_host::StateSoA& sv = a.stage == 0 ? a.base : a.st;
-		jaumann<float>(vx_x, vx_y, vy_x, vy_y, sv.Sxx_f[i], sv.Sxy_f[i], sv.Syy_f[i], pr.fG, d[5], d[6], d[7]);
+		jaumann<float>(s.vx_x, s.vx_y, s.vy_x, s.vy_y, sv.Sxx_f[i], sv.Sxy_f[i], sv.Syy_f[i], pr.fG, d[5], d[6], d[7]);
 	}
-	if (flags & A_CONTINUITY) d[4] = -(rhoi * (vx_x + vy_y));
-	if (GOD && (flags & A_GOD_CONT)) d[4] = god_rho;
+	if (flags & A_CONTINUITY) d[4] = -(rhoi * (s.vx_x + s.vy_y));
+	if (GOD && (flags & A_GOD_CONT)) d[4] = s.god_rho;
 	if (GOD && (flags & A_GOD_MOM)) {
-		d[2] += god_vx + (float)a.fcx[i] / ri.m;
-		d[3] += god_vy + (float)a.fcy[i] / ri.m;
+		d[2] += s.god_vx + (float)a.fcx[i] / ri.m;
+		d[3] += s.god_vy + (float)a.fcy[i] / ri.m;
 	}
 	if (flags & A_MOMENTUM_UL) {
-		d[2] += 1.f / rhoi * (Sxx_x + Sxy_y) + (float)a.fcx[i] / ri.m;
-		d[3] += 1.f / rhoi * (Sxy_x + Syy_y) + (float)a.fcy[i] / ri.m;
+		if (GOD) {  // (pair32_fast added the stress forces to av, without rho / rho)
+			d[2] += 1.f / rhoi * (s.Sxx_x * rhoi + s.Sxy_y * rhoi);
+			d[3] += 1.f / rhoi * (s.Sxy_x * rhoi + s.Syy_y * rhoi);
+		}
+		d[2] += (float)a.fcx[i] / ri.m;
+		d[3] += (float)a.fcy[i] / ri.m;
 	}
 	if (a.stage > 0) {
 		// the cells were sized at stage 0 for moves up to g.slack; check that held
@@ -1174,13 +1287,12 @@ __device__ __forceinline__ void pair32_row(const ULArgs& a, const BodyParams* __
 	// advection: the FP64 velocity enters the FP64 position update below
 	double dd0 = (double)d[0], dd1 = (double)d[1];
 	if (flags & A_ADVECTION) {
-		const mfk_host::StateSoA& s = a.stage == 0 ? a.base : a.st;
-		dd0 += s.vx[i];
-		dd1 += s.vy[i];
+		const mfk_host::StateSoA& sv = a.stage == 0 ? a.base : a.st;
+		dd0 += sv.vx[i];
+		dd1 += sv.vy[i];
 	}
-	(void)vxi; (void)vyi;
 	// position/velocity in FP64, rho/S in FP32
-	uint32_t s = a.stage;
+	const uint32_t stg = a.stage;
 	double dt = pr.dt;
 	double dq[4] = {dd0, dd1, (double)d[2], (double)d[3]};
 	double* bp[4] = {a.base.x, a.base.y, a.base.vx, a.base.vy};
@@ -1189,23 +1301,22 @@ __device__ __forceinline__ void pair32_row(const ULArgs& a, const BodyParams* __
 	float* bq[4] = {a.base.rho_f, a.base.Sxx_f, a.base.Sxy_f, a.base.Syy_f};
 	float* aq[4] = {a.acc.rho_f, a.acc.Sxx_f, a.acc.Sxy_f, a.acc.Syy_f};
 	float* sq[4] = {a.st.rho_f, a.st.Sxx_f, a.st.Sxy_f, a.st.Syy_f};
-	if (s < 3) {
-		double dts = (s == 2 ? 1.0 : 0.5) * dt;
+	if (stg < 3) {
+		double dts = (stg == 2 ? 1.0 : 0.5) * dt;
 		double nv[4];  // the next stage's x, y, vx, vy
 		float nf[4];   // and its rho - rho0, Sxx, Sxy, Syy
 #pragma unroll
 		for (int q = 0; q < 4; q++) {
-			ap[q][i] = (s == 0) ? dq[q] : ap[q][i] + 2 * dq[q];
+			ap[q][i] = (stg == 0) ? dq[q] : ap[q][i] + 2 * dq[q];
 			nv[q] = bp[q][i] + dq[q] * dts;
 			sp[q][i] = nv[q];
 			float dr = d[4 + q];
-			aq[q][i] = (s == 0) ? dr : aq[q][i] + 2.f * dr;
+			aq[q][i] = (stg == 0) ? dr : aq[q][i] + 2.f * dr;
 			nf[q] = bq[q][i] + dr * (float)dts;
 			sq[q][i] = nf[q];
 		}
 		if (a.write_recs)
-			put_rec32(a, pr, i, reinterpret_cast<Rec32*>(a.rec_next) + k, nv[0], nv[1], nv[2], nv[3], nf[0], nf[1], nf[2],
-			          nf[3]);
+			put_rec32(a, pr, i, a.rec_next, k, nv[0], nv[1], nv[2], nv[3], nf[0], nf[1], nf[2], nf[3]);
 	} else {
 		double w6 = dt * 1. / 6.;
 #pragma unroll
@@ -1220,26 +1331,30 @@ __device__ __forceinline__ void pair32_row(const ULArgs& a, const BodyParams* __
 }
 
 // The mixed pair pass with L threads per row (plain grid)
-template <bool GOD, int L>
+template <bool GOD, bool FULL, int L>
 __global__ void __launch_bounds__(256, 3) k_pair_split(ULArgs a, const BodyParams* __restrict__ P,
                                                        const Geom* __restrict__ G, DevStatus* st) {
 	const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
 	const uint32_t k = t / L;
 	if (k >= a.n_total) return;  // a row's L lanes leave together (L divides the warp)
-	pair32_row<GOD, L>(a, P, G, st, k, t % L);
+	pair32_row<GOD, FULL, L>(a, P, G, st, k, t % L);
 }
+
+constexpr uint32_t PAIR_ROWS_MB4 = 1u << 19;
 
 // The mixed pair kernel.  Plain form: one thread per cell-ordered row.  Persistent form
 // (one launch per stage over all bodies): a fixed grid whose blocks take chunks of
 // rows -- consecutive cell-ordered rows, so a chunk is a run of cells of one body --
 // from an atomic counter until the rows run out; no block ever waits on another.
-template <bool GOD>
-__global__ void __launch_bounds__(256, 3) k_pair(ULArgs a, const BodyParams* __restrict__ P, const Geom* __restrict__ G,
+// MB: blocks of 256 per SM the register budget is cut for (3: 80 registers; 4: 64, with
+// some constants of a row spilled) -- the same arithmetic, so the same results.
+template <bool GOD, bool FULL, int MB>
+__global__ void __launch_bounds__(256, MB) k_pair(ULArgs a, const BodyParams* __restrict__ P, const Geom* __restrict__ G,
                                                  DevStatus* st) {
 	if (!a.persistent) {
 		uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
 		if (k >= a.n_total) return;
-		pair32_row<GOD>(a, P, G, st, k);
+		pair32_row<GOD, FULL>(a, P, G, st, k);
 		return;
 	}
 	__shared__ uint32_t s_chunk;
@@ -1252,7 +1367,7 @@ __global__ void __launch_bounds__(256, 3) k_pair(ULArgs a, const BodyParams* __r
 		if (base >= a.n_total) break;
 		for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) {
 			uint64_t k = base + r;
-			if (k < a.n_total) pair32_row<GOD>(a, P, G, st, (uint32_t)k);
+			if (k < a.n_total) pair32_row<GOD, FULL>(a, P, G, st, (uint32_t)k);
 		}
 	}
 }
@@ -1291,7 +1406,7 @@ __global__ void k_neighbors(ULArgs a, const Geom* __restrict__ G, uint32_t* coun
 	if (pass == 0) counts[i] = cnt;
 }
 
-inline unsigned grid1(uint32_t n, unsigned bs) { return (unsigned)((n + bs - 1) / bs); }
+inline unsigned grid1(uint64_t n, unsigned bs) { return (unsigned)((n + bs - 1) / bs); }
 
 cudaError_t build_grid(const ULArgs& a, bool mixed, cudaStream_t s) {
 	DevStatus* st = reinterpret_cast<DevStatus*>(a.status);
@@ -1342,19 +1457,19 @@ cudaError_t ul_stage(const ULArgs& a, bool mixed, cudaStream_t s) {
 	}
 	if (a.ev_pair0) cudaEventRecord(a.ev_pair0, s);
 	const bool god = a.flags & (A_GOD_CONT | A_GOD_MOM);
-	if (mixed && !a.persistent && (a.split == 4 || a.split == 8)) {
-		const unsigned g2 = grid1((uint64_t)a.n_total * a.split, bs);
-		if (a.split == 4) {
-			if (god) k_pair_split<true, 4><<<g2, bs, 0, s>>>(a, a.params, a.geom, st);
-			else k_pair_split<false, 4><<<g2, bs, 0, s>>>(a, a.params, a.geom, st);
-		} else {
-			if (god) k_pair_split<true, 8><<<g2, bs, 0, s>>>(a, a.params, a.geom, st);
-			else k_pair_split<false, 8><<<g2, bs, 0, s>>>(a, a.params, a.geom, st);
-		}
-	} else if (mixed && god) {
-		k_pair<true><<<grid, bs, 0, s>>>(a, a.params, a.geom, st);
-	} else if (mixed) {
-		k_pair<false><<<grid, bs, 0, s>>>(a, a.params, a.geom, st);
+	if (mixed) {
+		const bool full = !god && (a.flags & A_MONAGHAN) == A_MONAGHAN;
+		const uint32_t split = !a.persistent && (a.split == 4 || a.split == 8) ? a.split : 1u;
+		auto launch = [&](auto kernel) {
+			kernel<<<split > 1 ? grid1((uint64_t)a.n_total * split, bs) : grid, bs, 0, s>>>(a, a.params, a.geom, st);
+		};
+		if (split == 4) launch(god ? k_pair_split<true, false, 4> : full ? k_pair_split<false, true, 4> : k_pair_split<false, false, 4>);
+		else if (split == 8) launch(god ? k_pair_split<true, false, 8> : full ? k_pair_split<false, true, 8> : k_pair_split<false, false, 8>);
+		else if (god || !full) launch(god ? k_pair<true, false, 3> : k_pair<false, false, 3>);
+		// More warps pay once every SM has several rounds of blocks: 64 ring impacts (1.35M
+		// rows) 30.9 -> 30.0 ms for 20 steps, 256 small impacts (317k rows) 5.69 -> 5.83 ms
+		// for 10, the rings at dx = 1 mm (4,408 rows) 9.9 -> 11.3 ms for 100.
+		else launch(a.n_total >= PAIR_ROWS_MB4 ? k_pair<false, true, 4> : k_pair<false, true, 3>);
 	} else {
 		const unsigned g64 = grid1(a.n_total, P64_ROWS);
 		if (god) k_pair64<true><<<g64, P64_THREADS, 0, s>>>(a, a.params, a.geom, st);

@@ -1,0 +1,124 @@
+"""The updated-Lagrangian pair passes against the CPU oracle where their branches change:
+few and many neighbours (a row's list of pairs is worked off when it fills), positions too
+far from the origin for the FP32 candidate test, neighbour counts on lattices whose pairs
+lie exactly on the search radius, pipelines that leave actions out."""
+import numpy as np
+import pytest
+
+import oracle
+from mfree_iwf_gb300 import actions as A
+from mfree_iwf_gb300 import scenarios as S
+
+pytestmark = pytest.mark.gpu
+
+
+def moving_rings(hdx, shift=0.0):
+    sc = S.c1_rings(dx=4e-3, hdx=hdx, nbh_eps=1e-6)
+    a = sc.bodies[0].arrays
+    a["vx"] += 2.0 * np.sin(200.0 * a["y"])
+    a["vy"] += 2.0 * np.cos(150.0 * a["x"])
+    for f in ("Sxx", "Sxy", "Syy"):
+        a[f] += 1e4 * np.sin(90.0 * a["x"] + 70.0 * a["y"])
+    a["x"] += shift
+    return sc
+
+
+# 1e-9: the form's bound against the reference (summation order, last bits of atan2)
+@pytest.mark.parametrize("precision", ["fp64_strict", "fp64"])
+@pytest.mark.parametrize("hdx,shift", [(1.3, 0.0), (1.7, 0.0), (2.7, 0.0), (1.3, 2e6)])
+def test_pair_pass_against_oracle(lib, oracle_bin, precision, hdx, shift):
+    import mfree_iwf_gb300 as M
+    sc = moving_rings(hdx, shift)
+    want = oracle.run(sc, 5).dumps[-1]["bodies"][0]
+    sim = M.from_scenario(sc, precision=precision)
+    sim.step(5)
+    got = sim.get_state(0)
+    sim.close()
+    for f in ("x", "y", "vx", "vy", "rho", "Sxx", "Sxy", "Syy"):
+        e = np.linalg.norm(got[f] - want[f]) / np.linalg.norm(want[f])
+        assert e < 1e-9, (f, e)
+
+
+@pytest.mark.parametrize("hdx", [1.0, 1.3, 2.0])
+def test_capacity_is_the_exact_count(lib, hdx):
+    import mfree_iwf_gb300 as M
+    sc = moving_rings(hdx)
+    sc.nbh_eps = 0.0  # with h a multiple of dx / 2 some pairs lie on 2h exactly
+    sc.dt = 1e-300    # the four stages see the same positions, hence the same counts
+    sim = M.from_scenario(sc, precision="fp64_strict")
+    most = int(sim.neighbor_counts(0).max())
+    sim.close()
+    for cap, fails in ((most + 1, False), (most, True)):
+        sim = M.from_scenario(sc, precision="fp64_strict", max_nbh=cap)
+        if fails:
+            with pytest.raises(M.MfError) as e:
+                sim.step(1)
+            assert e.value.name == "MF_ERR_NBH_OVERFLOW"
+        else:
+            sim.step(1)
+        sim.close()
+
+
+DROP = {"none": [], "xsph": [A.CORRECTORS_XSPH], "viscosity": [A.CORRECTORS_MGHN_ARTIFICIAL_VISCOSITY],
+        "artificial stress": [A.CORRECTORS_MGHN_ARTIFICIAL_STRESS], "weights": [A.RIEMANN_UPDATE_INTEGRATION_WEIGHTS],
+        "momentum": [A.CONTMECH_MOMENTUM_UL], "stress": [A.DERIVE_STRESS_MONAGHAN, A.CONTMECH_MOMENTUM_UL],
+        "rates": [A.DERIVE_VELOCITY, A.MATERIAL_STRESS_RATE_JAUMANN, A.CONTMECH_CONTINUITY]}
+
+
+# FP64: as above.  Mixed: a pair sum of ~20 FP32 terms of ~10 roundings each is good to
+# ~1e-6 of its terms; five steps move the state by less than itself
+@pytest.mark.parametrize("precision,tol", [("fp64_strict", 1e-9), ("fp64", 1e-9), ("mixed", 1e-5)])
+@pytest.mark.parametrize("drop", list(DROP))
+def test_partial_pipelines_against_oracle(lib, oracle_bin, precision, tol, drop):
+    """Pipelines that leave actions out: the pair pass skips their terms."""
+    import mfree_iwf_gb300 as M
+    sc = moving_rings(1.3)
+    sc.actions = [a for a in sc.actions if a not in DROP[drop]]
+    want = oracle.run(sc, 5).dumps[-1]["bodies"][0]
+    sim = M.from_scenario(sc, precision=precision)
+    sim.step(5)
+    got = sim.get_state(0)
+    sim.close()
+    for f in ("x", "y", "vx", "vy", "rho", "Sxx", "Sxy", "Syy"):
+        e = np.linalg.norm(got[f] - want[f]) / np.linalg.norm(want[f])
+        assert e < tol, (f, e)
+
+
+@pytest.mark.parametrize("hdx", [1.3, 1.7, 2.7])
+def test_mixed_pair_pass_close_to_oracle(lib, oracle_bin, hdx):
+    """Few and many candidates per stencil column (a mask holds 32)."""
+    import mfree_iwf_gb300 as M
+    sc = moving_rings(hdx)
+    want = oracle.run(sc, 5).dumps[-1]["bodies"][0]
+    sim = M.from_scenario(sc, precision="mixed")
+    sim.step(5)
+    got = sim.get_state(0)
+    sim.close()
+    for f in ("x", "y", "vx", "vy", "rho", "Sxx", "Sxy", "Syy"):
+        e = np.linalg.norm(got[f] - want[f]) / np.linalg.norm(want[f])
+        assert e < 1e-5, (f, e)
+
+
+def test_large_batch_equals_instances_alone(lib):
+    """From 2^19 rows on the mixed pair pass runs at another register budget: the same
+    bits as an instance alone."""
+    import mfree_iwf_gb300 as M
+    ens = S.c4_ensemble(30)
+    assert ens.n_total >= 1 << 19
+    for b in ens.bodies:
+        b.arrays["vx"] += 0.5 * np.sin(200.0 * b.arrays["y"])
+    sim = M.from_scenario(ens, precision="mixed")
+    sim.step(3)
+    for k in (0, 29):
+        b = ens.bodies[k]
+        one = S.Scenario(method=ens.method, bodies=[b], actions=ens.actions, dt=b.params["dt"], nu=b.params["nu"],
+                         E=b.params["E"], rho0=b.params["rho0"], wdeltap=b.params["wdeltap"], corr_exp=ens.corr_exp,
+                         mghn_eps=ens.mghn_eps, alpha=ens.alpha, beta=ens.beta, eta=ens.eta, xsph_eps=ens.xsph_eps,
+                         nbh_eps=ens.nbh_eps)
+        alone = M.from_scenario(one, precision="mixed")
+        alone.step(3)
+        got, want = sim.get_state(k), alone.get_state(0)
+        alone.close()
+        for f in ("x", "y", "vx", "vy", "rho", "Sxx", "Sxy", "Syy"):
+            np.testing.assert_array_equal(got[f], want[f], err_msg=f)
+    sim.close()
