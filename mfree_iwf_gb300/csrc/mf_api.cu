@@ -19,6 +19,10 @@
 
 #include "../../include/mfree_gb300.h"
 #include "mf_kernels.h"
+// (the device helpers, for the monitor and transfer kernels below)
+#define MF_STRICT_FORM 0
+#define MF_NS mf_host
+#include "mf_common.cuh"
 
 using namespace mfk_host;
 
@@ -45,14 +49,18 @@ __global__ void k_monitor(uint32_t nb, const BodyParams* __restrict__ P, const d
 		uint32_t i = pr.off + k;
 		svx += vx[i];
 		svy += vy[i];
-		double r = rho ? rho[i] : (double)rho_f[i] + pr.rho0;
+		// (float -> double by integers; the square root once, of the largest square: a
+		// correctly rounded root is monotonic; no root of a zero force)
+		double r = rho ? rho[i] : mfk::f2d(rho_f[i]) + pr.rho0;
 		double p = eos ? pr.c0sq * (r - pr.rho0) : 0.;
-		double sxx = (Sxx ? Sxx[i] : (double)Sxx_f[i]) - p;
-		double syy = (Syy ? Syy[i] : (double)Syy_f[i]) - p;
-		double sxy = Sxy ? Sxy[i] : (double)Sxy_f[i];
-		vm = fmax(vm, sqrt(fmax(sxx * sxx - sxx * syy + syy * syy + 3. * sxy * sxy, 0.)));
-		fc += sqrt(fcx[i] * fcx[i] + fcy[i] * fcy[i]);
+		double sxx = (Sxx ? Sxx[i] : mfk::f2d(Sxx_f[i])) - p;
+		double syy = (Syy ? Syy[i] : mfk::f2d(Syy_f[i])) - p;
+		double sxy = Sxy ? Sxy[i] : mfk::f2d(Sxy_f[i]);
+		vm = fmax(vm, sxx * sxx - sxx * syy + syy * syy + 3. * sxy * sxy);
+		const double fx = fcx[i], fy = fcy[i];
+		if (fx != 0. || fy != 0.) fc += sqrt(fx * fx + fy * fy);
 	}
+	vm = sqrt(vm);
 	__shared__ double s0[256], s1[256], s2[256], s3[256];
 	s0[threadIdx.x] = svx; s1[threadIdx.x] = svy; s2[threadIdx.x] = vm; s3[threadIdx.x] = fc;
 	__syncthreads();
@@ -212,7 +220,7 @@ struct mf_ctx {
 	std::string err;
 	std::vector<HostBody> bodies;
 	bool ready = false;
-	uint32_t n_total = 0;
+	uint32_t n_total = 0, max_body = 0;  // rows of all bodies, of the largest
 	uint32_t flags = 0;
 	bool mixed = false, strict = false;
 	bool uw_mixed = false;  // weak UL, mixed form: FP32 ellipse and moments, FP32 / float-float pass sums
@@ -452,6 +460,8 @@ ULArgs ul_args(mf_ctx* c, uint32_t stage) {
 	ULArgs a{};
 	a.n_total = c->n_total;
 	a.n_bodies = (uint32_t)c->bodies.size();
+	a.max_body = c->max_body;
+	a.sm_count = (uint32_t)std::max(0, c->sm_count);
 	a.stage = stage;
 	a.flags = c->flags;
 	a.max_nbh = c->cfg.max_nbh;
@@ -624,6 +634,7 @@ mf_status finalize(mf_ctx* c) {
 		}
 
 	uint32_t n = c->n_total;
+	for (auto& b : c->bodies) c->max_body = std::max(c->max_body, b.n);
 	CK(c->body_of.alloc(n));
 	std::vector<uint32_t> bof(n);
 	for (size_t b = 0; b < c->bodies.size(); b++)
@@ -732,7 +743,9 @@ mf_status ul_step(mf_ctx* c) {
 		timing_count(c, slot_pair, c->n_total);
 		timing_end(c, slot_all, c->n_total);
 		if (e != cudaSuccess) return cuda_fail(c, e, "ul_stage");
-		c->launches += (a.strict_grid || s == 0) ? 8 + 4 : (a.skip_gather ? 1 : 2);
+		const bool small = c->strict ? mf_strict::ul_small_grid(a) : mf_fast::ul_small_grid(a);
+		const uint32_t grid = !(a.strict_grid || s == 0) ? 0 : !small ? 9 : a.n_bodies == 1 ? 1 : 2;
+		c->launches += grid + (a.skip_gather ? 1 : 2);
 	}
 	if (c->n_bc) {  // rk4.h:105: the conditions act on the particles after the combine
 		cudaError_t e = c->strict ? mf_strict::ul_bc(c->n_bc, c->bc_rows.p, c->bc_v.p, c->sd[0][2].p, c->sd[0][3].p, c->stream)

@@ -65,6 +65,8 @@ struct StateSoA {
 
 struct ULArgs {
 	uint32_t n_total, n_bodies, stage;    // stage 0..3
+	uint32_t max_body, sm_count;          // rows of the largest body (0: unknown); SMs
+	uint32_t fill_cells;                  // set by the grid build: the gather also fills the cell table
 	uint32_t flags;                       // action bits
 	uint32_t max_nbh;                     // neighbour capacity (0 = unchecked)
 	uint32_t strict_grid;                 // 1: rebuild the reference grid at this stage
@@ -282,6 +284,7 @@ struct ContactArgs {
 #define MF_DECLARE_LAUNCHERS(NS)                                                                              \
 	namespace NS {                                                                                           \
 	size_t ul_sort_tmp_bytes(uint32_t n, int bits);                                                          \
+	bool ul_small_grid(const mfk_host::ULArgs& a);                                                            \
 	size_t ul_rec_bytes(bool mixed);                                                                         \
 	cudaError_t ul_stage(const mfk_host::ULArgs& a, bool mixed, cudaStream_t s);                             \
 	cudaError_t ul_bc(uint32_t n_bc, const uint32_t* rows, const double* v, double* vx, double* vy, cudaStream_t s); \

@@ -152,6 +152,7 @@ extern "C" MF_API mf_status mf_ul_step_noalloc(const mf_device_body* body, const
 	ULArgs a{};
 	a.n_total = n;
 	a.n_bodies = 1;
+	a.max_body = n;
 	a.flags = flags;
 	a.max_nbh = 200;  // MAX_NBH, particle.h:31
 	a.strict_grid = 1;

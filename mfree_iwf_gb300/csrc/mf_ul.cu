@@ -9,8 +9,8 @@
 //   ul_geom      per-body cell geometry, cell offsets   (grid.h:105-115)
 //   ul_hash      global cell key per row                (grid.h:35-41)
 //   CUB radix sort of (key, row)                        (body.h:137)
-//   ul_cells     cell start table, empty cells filled from the right (grid.h:48-81)
-//   ul_gather    the rows' stage state in cell order, with the per-particle actions
+//   ul_gather    the cell start table, empty cells filled from the right (grid.h:48-81);
+//                the rows' stage state in cell order, with the per-particle actions
 //                EOS (material.h:37-64), artificial stress (correctors.h:37-81) and
 //                integration weights (riemann_integration.h:28-33) fused in
 //   ul_pair      one thread per row: walks the 3x3 cell stencil of the reference grid
@@ -179,6 +179,45 @@ __global__ void k_bbox(uint32_t n, const double* __restrict__ x, const double* _
 	}
 }
 
+// Cell geometry of one body (grid.h:105-115) from its bounding box, h_max and (mixed form)
+// largest squared speed; bad: not a valid grid (one cell, or too many, is set).
+__device__ Geom body_geometry(const BodyParams& pr, int mixed, double bminx, double bminy, double bmaxx, double bmaxy,
+                              double hmax, double v2max, bool& bad) {
+	Geom g{};
+	bminx -= 1e-6; bminy -= 1e-6;
+	bmaxx += 1e-6; bmaxy += 1e-6;
+	double dx = hmax * 2.;
+	double slack = 0.;
+	uint32_t span = 1;
+	double lx = bmaxx - bminx, ly = bmaxy - bminy;
+	if (mixed) {
+		// a particle moves at most ~ |v| dt per step; allow twice the fastest speed
+		slack = 2. * sqrt(v2max) * pr.dt;
+		dx = 2. * hmax + 2. * slack;
+		// half-size cells with a 5x5 stencil cover the same reach with ~40 % fewer
+		// candidates than 3x3 cells of the full reach; used while the body's cells
+		// stay below twice its particles
+		double hx = 0.5 * dx;
+		if (ceil(lx / hx) * ceil(ly / hx) <= 2.0 * pr.n) {
+			dx = hx;
+			span = 2;
+		}
+	}
+	double fnx = ceil(lx / dx), fny = ceil(ly / dx);
+	uint32_t nx = (uint32_t)fnx, ny = (uint32_t)fny;
+	uint32_t num_cell = nx * ny;
+	bad = false;
+	if (!(num_cell < pr.n) && !mixed) bad = true;
+	if (!(fnx * fny < 4.0e9) || nx == 0 || ny == 0) {
+		nx = ny = 1;
+		num_cell = 1;
+		bad = true;
+	}
+	g.bbmin_x = bminx; g.bbmin_y = bminy; g.dx = dx; g.slack = slack;
+	g.nx = nx; g.ny = ny; g.num_cell = num_cell; g.span = span;
+	return g;
+}
+
 // Cell geometry per body (grid.h:105-115) and the exclusive scan of cell counts.
 // One block; bodies are processed serially in chunks for the scan.
 __global__ void k_geom(uint32_t nb, const unsigned long long* bb, const BodyParams* P, int mixed, Geom* G,
@@ -196,46 +235,14 @@ __global__ void k_geom(uint32_t nb, const unsigned long long* bb, const BodyPara
 			g.dx = 1.;
 			g.span = 1;
 		} else if (b < nb) {
-			double bminx = ord_decode(bb[6 * b + 0]), bminy = ord_decode(bb[6 * b + 1]);
-			double bmaxx = ord_decode(bb[6 * b + 2]), bmaxy = ord_decode(bb[6 * b + 3]);
-			double hmax = ord_decode(bb[6 * b + 4]);
-			bminx -= 1e-6; bminy -= 1e-6;
-			bmaxx += 1e-6; bmaxy += 1e-6;
-			double dx = hmax * 2.;
-			double slack = 0.;
-			uint32_t span = 1;
-			double lx = bmaxx - bminx, ly = bmaxy - bminy;
-			if (mixed) {
-				// a particle moves at most ~ |v| dt per step; allow twice the fastest speed
-				slack = 2. * sqrt(ord_decode(bb[6 * b + 5])) * P[b].dt;
-				dx = 2. * hmax + 2. * slack;
-				// half-size cells with a 5x5 stencil cover the same reach with ~40 % fewer
-				// candidates than 3x3 cells of the full reach; used while the body's cells
-				// stay below twice its particles
-				double hx = 0.5 * dx;
-				if (ceil(lx / hx) * ceil(ly / hx) <= 2.0 * P[b].n) {
-					dx = hx;
-					span = 2;
-				}
-			}
-			double fnx = ceil(lx / dx), fny = ceil(ly / dx);
-			uint32_t nx = (uint32_t)fnx, ny = (uint32_t)fny;
-			uint32_t num_cell = nx * ny;
-			bool bad = false;
-			if (!(num_cell < P[b].n) && !mixed) {
+			bool bad;
+			g = body_geometry(P[b], mixed, ord_decode(bb[6 * b + 0]), ord_decode(bb[6 * b + 1]), ord_decode(bb[6 * b + 2]),
+			                  ord_decode(bb[6 * b + 3]), ord_decode(bb[6 * b + 4]), ord_decode(bb[6 * b + 5]), bad);
+			if (bad) {
 				fail_body(failed, st, ERR_GRID, P[b].off, b);
-				bad = true;
+				if (failed) g.num_cell = 0;  // masked from this stage on
 			}
-			if (!(fnx * fny < 4.0e9) || nx == 0 || ny == 0) {
-				fail_body(failed, st, ERR_GRID, P[b].off, b);
-				nx = ny = 1;
-				num_cell = 1;
-				bad = true;
-			}
-			if (bad && failed) num_cell = 0;  // masked from this stage on
-			g.bbmin_x = bminx; g.bbmin_y = bminy; g.dx = dx; g.slack = slack;
-			g.nx = nx; g.ny = ny; g.num_cell = num_cell; g.span = span;
-			cnt = num_cell;
+			cnt = g.num_cell;
 		}
 		s_cnt[threadIdx.x] = cnt;
 		__syncthreads();
@@ -296,22 +303,209 @@ __global__ void k_hash(uint32_t n, const double* __restrict__ x, const double* _
 	keys[i] = (tot == 0) ? 0u : key;
 }
 
-// Cell start table over all bodies' cells (grid.h:48-81): cell_start[c] is the
-// first sorted position with key >= c, so empty cells get the next start.
-__global__ void k_cells(uint32_t n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ total_cells,
-                        uint32_t* cell_start) {
-	uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-	uint32_t tot = *total_cells;
-	if (k > n) return;
+// Cell start table over all bodies' cells (grid.h:48-81): cell_start[c] is the first
+// sorted position with key >= c, so empty cells get the next start.  Position k (up to
+// and including n) fills in the cells that start there; run by the gather kernels.
+__device__ __forceinline__ void fill_cells(const ULArgs& a, uint32_t k) {
+	const uint32_t n = a.n_total, tot = *a.total_cells;
 	if (k == n) {
-		uint32_t last = (n == 0) ? 0u : keys[n - 1] + 1;
-		for (uint32_t c = last; c <= tot; c++) cell_start[c] = n;
+		const uint32_t last = a.keys_sorted[n - 1] + 1;
+		for (uint32_t c = last; c <= tot; c++) a.cell_start[c] = n;
 		return;
 	}
-	uint32_t key = min(keys[k], tot);
-	uint32_t prev = (k == 0) ? 0u : min(keys[k - 1], tot) + 1;
-	if (k == 0 || keys[k] != keys[k - 1])
-		for (uint32_t c = prev; c <= key; c++) cell_start[c] = k;
+	const uint32_t key = min(a.keys_sorted[k], tot);
+	const uint32_t prev = (k == 0) ? 0u : min(a.keys_sorted[k - 1], tot) + 1;
+	if (k == 0 || a.keys_sorted[k] != a.keys_sorted[k - 1])
+		for (uint32_t c = prev; c <= key; c++) a.cell_start[c] = k;
+}
+
+// ---- The grid of small bodies (at most GRID_BODY_MAX rows each): a block per body does
+// what the kernels above do in eight launches -- bounding box, geometry, keys, the sort
+// and the cell table -- in two (k_body_box, k_body_sort), and one body in one.  The
+// rows of a body stay in its own range of the cell order; a counting sort over its cells,
+// each cell's rows then put in ascending order, gives the radix sort's stable order.
+// 256 small impacts (512 bodies of some 600 rows): 90 us a step in 13 launches -> 30 us.
+// Larger bodies (ul_small_grid), and contexts that mask failed bodies (whose rows leave
+// the cell order), take the general kernels.
+constexpr uint32_t GRID_BODY_MAX = 4608;    // rows: two cells each and a 16-bit index fit 48 KB
+constexpr uint32_t GRID_MAX_BODIES = 4096;  // every block adds up the cells of the bodies before it
+
+// Block-wide reduction in shared memory (blockDim.x a multiple of 32, at most 1024)
+template <class T, class Op>
+__device__ __forceinline__ T block_reduce(T v, T* s, T identity, Op op) {
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+	__syncthreads();
+	if ((threadIdx.x & 31u) == 0) s[threadIdx.x >> 5] = v;
+	__syncthreads();
+	v = (threadIdx.x & 31u) < (blockDim.x >> 5) ? s[threadIdx.x & 31u] : identity;
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+	return v;
+}
+
+// Bounding box, h_max, largest squared speed and from them the geometry of body b
+// (cell_off left 0); every thread returns it
+__device__ __forceinline__ Geom body_box(const ULArgs& a, int mixed, uint32_t b) {
+	typedef unsigned long long u64;
+	__shared__ u64 s_red[32];
+	__shared__ Geom s_geom;
+	const BodyParams& pr = a.params[b];
+	const mfk_host::StateSoA& sv = a.stage == 0 ? a.base : a.st;
+	u64 mnx = ord_encode(1.7976931348623157e308), mny = mnx, mxx = ord_encode(-1.7976931348623157e308), mxy = mxx, mh = mxx;
+	u64 mv = ord_encode(0.);
+	for (uint32_t i = pr.off + threadIdx.x; i < pr.off + pr.n; i += blockDim.x) {
+		const u64 ex = ord_encode(sv.x[i]), ey = ord_encode(sv.y[i]);
+		mnx = min(mnx, ex);
+		mxx = max(mxx, ex);
+		mny = min(mny, ey);
+		mxy = max(mxy, ey);
+		mh = max(mh, ord_encode(a.h[i]));
+		if (mixed) {
+			const double vx = sv.vx[i], vy = sv.vy[i];
+			mv = max(mv, ord_encode(vx * vx + vy * vy));
+		}
+	}
+	auto lo = [](u64 p, u64 q) { return min(p, q); };
+	auto hi = [](u64 p, u64 q) { return max(p, q); };
+	mnx = block_reduce(mnx, s_red, ~0ull, lo);
+	mny = block_reduce(mny, s_red, ~0ull, lo);
+	mxx = block_reduce(mxx, s_red, 0ull, hi);
+	mxy = block_reduce(mxy, s_red, 0ull, hi);
+	mh = block_reduce(mh, s_red, 0ull, hi);
+	if (mixed) mv = block_reduce(mv, s_red, 0ull, hi);
+	if (threadIdx.x == 0) {
+		bool bad;
+		s_geom = body_geometry(pr, mixed, ord_decode(mnx), ord_decode(mny), ord_decode(mxx), ord_decode(mxy), ord_decode(mh),
+		                       ord_decode(mv), bad);
+		if (bad) raise(reinterpret_cast<DevStatus*>(a.status), ERR_GRID, pr.off);
+	}
+	__syncthreads();
+	return s_geom;
+}
+
+__global__ void __launch_bounds__(1024) k_body_box(ULArgs a, int mixed, uint32_t* cells) {
+	const uint32_t b = blockIdx.x;
+	const Geom g = body_box(a, mixed, b);
+	if (threadIdx.x == 0) {
+		a.geom[b] = g;
+		cells[b] = g.num_cell;
+	}
+}
+
+// The body's rows in cell order and its part of the cell table.  ONE: a single body, its
+// geometry computed here; else `cells` holds every body's cell count.
+template <bool ONE>
+__global__ void __launch_bounds__(1024) k_body_sort(ULArgs a, int mixed, const uint32_t* cells, uint32_t hist_cap,
+                                                    uint32_t cell_cap) {
+	extern __shared__ uint32_t s_dyn[];  // [hist_cap] cell counters, then 16-bit row indices
+	__shared__ unsigned long long s_red[32];
+	__shared__ uint32_t s_warp[32];
+	uint16_t* slot = reinterpret_cast<uint16_t*>(s_dyn + hist_cap);
+	const uint32_t b = blockIdx.x, T = blockDim.x, tid = threadIdx.x;
+	const mfk_host::StateSoA& sv = a.stage == 0 ? a.base : a.st;
+	const uint32_t off = a.params[b].off, n = a.params[b].n;
+	Geom g;
+	unsigned long long before = 0, total;
+	if (ONE) {
+		g = body_box(a, mixed, b);
+		total = g.num_cell;
+	} else {
+		g = a.geom[b];
+		total = 0;
+		for (uint32_t q = tid; q < a.n_bodies; q += T) {
+			const uint32_t c = cells[q];
+			total += c;
+			if (q < b) before += c;
+		}
+		auto add = [](unsigned long long p, unsigned long long q) { return p + q; };
+		total = block_reduce(total, s_red, 0ull, add);
+		before = block_reduce(before, s_red, 0ull, add);
+	}
+	const bool fits = total <= cell_cap;
+	if (!fits) before = 0;
+	g.cell_off = (uint32_t)before;
+	if (tid == 0) {
+		a.geom[b] = g;
+		if (b == 0) {
+			*a.total_cells = fits ? (uint32_t)total : 0u;
+			if (!fits) raise(reinterpret_cast<DevStatus*>(a.status), ERR_GRID, 0);
+		}
+	}
+	if (!fits) {  // downstream kernels see an empty grid
+		for (uint32_t i = tid; i < n; i += T) {
+			a.perm[off + i] = off + i;
+			a.keys_sorted[off + i] = 0;
+		}
+		return;
+	}
+	// the cells' counters: shared memory, or (scattered particles: more cells than the
+	// block's share) the body's part of the cell table itself
+	const uint32_t nc = g.num_cell;
+	volatile uint32_t* hist = nc <= hist_cap ? s_dyn : a.cell_start + g.cell_off;
+	for (uint32_t c = tid; c < nc; c += T) hist[c] = 0;
+	__syncthreads();
+	for (uint32_t i = tid; i < n; i += T) {
+		uint32_t ix = (uint32_t)((sv.x[off + i] - g.bbmin_x) / g.dx);
+		uint32_t iy = (uint32_t)((sv.y[off + i] - g.bbmin_y) / g.dx);
+		if (ix >= g.nx || iy >= g.ny) {
+			raise(reinterpret_cast<DevStatus*>(a.status), ERR_GRID, off + i);
+			ix = min(ix, g.nx - 1);
+			iy = min(iy, g.ny - 1);
+		}
+		const uint32_t key = ix * g.ny + iy;
+		a.keys[off + i] = key;
+		atomicAdd(const_cast<uint32_t*>(&hist[key]), 1u);
+	}
+	__syncthreads();
+	// exclusive scan: each thread a contiguous piece
+	const uint32_t per = (nc + T - 1) / T, c0 = min(tid * per, nc), c1 = min(c0 + per, nc);
+	uint32_t sum = 0;
+	for (uint32_t c = c0; c < c1; c++) sum += hist[c];
+	uint32_t run = sum;
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t up = __shfl_up_sync(0xffffffffu, run, o);
+		if ((tid & 31u) >= (uint32_t)o) run += up;
+	}
+	if ((tid & 31u) == 31u) s_warp[tid >> 5] = run;
+	__syncthreads();
+	uint32_t start = run - sum;
+	for (uint32_t w = 0; w < (tid >> 5); w++) start += s_warp[w];
+	for (uint32_t c = c0; c < c1; c++) {
+		const uint32_t k = hist[c];
+		hist[c] = start;
+		start += k;
+	}
+	__syncthreads();
+	for (uint32_t i = tid; i < n; i += T) slot[atomicAdd(const_cast<uint32_t*>(&hist[a.keys[off + i]]), 1u)] = (uint16_t)i;
+	__syncthreads();
+	// every cell's rows ascending (hist[c] is now the end of cell c)
+	for (uint32_t c = tid; c < nc; c += T) {
+		const uint32_t s0 = c ? hist[c - 1] : 0u, s1 = hist[c];
+		for (uint32_t p = s0 + 1; p < s1; p++) {
+			const uint16_t v = slot[p];
+			uint32_t q = p;
+			for (; q > s0 && slot[q - 1] > v; q--) slot[q] = slot[q - 1];
+			slot[q] = v;
+		}
+	}
+	__syncthreads();
+	for (uint32_t p = tid; p < n; p += T) {
+		const uint32_t i = slot[p];
+		a.perm[off + p] = off + i;
+		a.keys_sorted[off + p] = g.cell_off + a.keys[off + i];
+	}
+	// the cell table: the first row of every cell, from the ends just used (in place where
+	// they stand in the table: piece by piece from the top, the piece's lower end read first)
+	uint32_t prev = c0 < c1 && c0 > 0 ? hist[c0 - 1] : 0u;
+	__syncthreads();
+	for (uint32_t c = c0; c < c1; c++) {
+		const uint32_t end = hist[c];
+		a.cell_start[g.cell_off + c] = off + prev;
+		prev = end;
+	}
+	if (b == a.n_bodies - 1 && tid == 0) a.cell_start[(uint32_t)total] = a.n_total;
 }
 
 // ---------------------------------------------------------------- gather
@@ -442,6 +636,7 @@ __device__ __forceinline__ void per_particle64(uint32_t flags, const BodyParams&
 
 __global__ void k_gather64(ULArgs a, const BodyParams* __restrict__ P) {
 	uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+	if (a.fill_cells && k <= a.n_total) fill_cells(a, k);
 	if (k >= a.n_total) return;
 	uint32_t i = a.perm[k];
 	StageView<false> v = stage_view<false>(a);
@@ -506,6 +701,7 @@ __device__ __forceinline__ void put_rec32(const ULArgs& a, const BodyParams& pr,
 
 __global__ void k_gather32(ULArgs a, const BodyParams* __restrict__ P) {
 	uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+	if (a.fill_cells && k <= a.n_total) fill_cells(a, k);
 	if (k >= a.n_total) return;
 	uint32_t i = a.perm[k];
 	StageView<true> v = stage_view<true>(a);
@@ -1406,23 +1602,42 @@ __global__ void k_neighbors(ULArgs a, const Geom* __restrict__ G, uint32_t* coun
 	if (pass == 0) counts[i] = cnt;
 }
 
+}  // namespace
+bool ul_small_grid(const ULArgs& a);
+namespace {
+
 inline unsigned grid1(uint64_t n, unsigned bs) { return (unsigned)((n + bs - 1) / bs); }
 
-cudaError_t build_grid(const ULArgs& a, bool mixed, cudaStream_t s) {
+// The grid of the stage's positions; the caller's gather comes next.
+cudaError_t build_grid(ULArgs& a, bool mixed, cudaStream_t s) {
 	DevStatus* st = reinterpret_cast<DevStatus*>(a.status);
+	const uint32_t cell_cap = a.cell_cap ? a.cell_cap : a.n_total + 1;
+	if (ul_small_grid(a)) {
+		const uint32_t hist_cap = (mixed ? 2u : 1u) * a.max_body + 16u;
+		const size_t smem = hist_cap * sizeof(uint32_t) + a.max_body * sizeof(uint16_t);
+		const unsigned T = a.max_body > 1024u ? 1024u : 256u;
+		uint32_t* cells = reinterpret_cast<uint32_t*>(a.bbox);  // (the general kernels' bounding boxes)
+		if (a.n_bodies == 1) {
+			k_body_sort<true><<<1, T, smem, s>>>(a, mixed ? 1 : 0, cells, hist_cap, cell_cap);
+		} else {
+			k_body_box<<<a.n_bodies, T, 0, s>>>(a, mixed ? 1 : 0, cells);
+			k_body_sort<false><<<a.n_bodies, T, smem, s>>>(a, mixed ? 1 : 0, cells, hist_cap, cell_cap);
+		}
+		return cudaGetLastError();
+	}
 	k_bbox_init<<<grid1(a.n_bodies, 128), 128, 0, s>>>(a.n_bodies, a.bbox);
 	const mfk_host::StateSoA& sv = a.stage == 0 ? a.base : a.st;
 	k_bbox<<<grid1(a.n_total, 256), 256, 0, s>>>(a.n_total, sv.x, sv.y, a.h, sv.vx, sv.vy, a.body_of, mixed ? 1 : 0,
 	                                              a.bbox, a.failed);
 	k_geom<<<1, 1024, 0, s>>>(a.n_bodies, a.bbox, a.params, mixed ? 1 : 0, a.geom, a.total_cells,
-	                          a.cell_cap ? a.cell_cap : a.n_total + 1, st, a.failed);
+	                          cell_cap, st, a.failed);
 	k_hash<<<grid1(a.n_total, 256), 256, 0, s>>>(a.n_total, sv.x, sv.y, a.body_of, a.geom, a.total_cells, a.keys,
 	                                              a.perm_in, st, a.failed);
 	size_t tmp = a.sort_tmp_bytes;
 	cudaError_t e = cub::DeviceRadixSort::SortPairs(a.sort_tmp, tmp, a.keys, a.keys_sorted, a.perm_in, a.perm,
 	                                                (int)a.n_total, 0, a.sort_bits, s);
 	if (e != cudaSuccess) return e;
-	k_cells<<<grid1(a.n_total + 1, 256), 256, 0, s>>>(a.n_total, a.keys_sorted, a.total_cells, a.cell_start);
+	a.fill_cells = 1;  // (the gather that follows also fills the cell table)
 	return cudaGetLastError();
 }
 
@@ -1435,19 +1650,28 @@ size_t ul_sort_tmp_bytes(uint32_t n, int bits) {
 	return bytes;
 }
 
+// One block's FP64 divisions for the cell keys hold its SM's narrow pipe for 7.5 ns a row:
+// up to 1024 rows that is a fraction of the launches saved; a single body of 4,408 rows
+// takes 45 us this way and 26 with the general kernels, unless every SM has such a body.
+bool ul_small_grid(const ULArgs& a) {
+	const uint32_t limit = a.n_bodies >= a.sm_count && a.sm_count ? GRID_BODY_MAX : 1024u;
+	return a.max_body && a.max_body <= limit && a.n_bodies <= GRID_MAX_BODIES && !a.failed;
+}
+
 size_t ul_rec_bytes(bool mixed) { return mixed ? sizeof(Rec32) : sizeof(Rec64); }
 
-cudaError_t ul_stage(const ULArgs& a, bool mixed, cudaStream_t s) {
-	if (a.n_total == 0) return cudaSuccess;
+cudaError_t ul_stage(const ULArgs& args, bool mixed, cudaStream_t s) {
+	if (args.n_total == 0) return cudaSuccess;
+	ULArgs a = args;
 	DevStatus* st = reinterpret_cast<DevStatus*>(a.status);
 	if (a.strict_grid || a.stage == 0) {
 		cudaError_t e = build_grid(a, mixed, s);
 		if (e != cudaSuccess) return e;
 	}
 	if (mixed) {
-		if (!a.skip_gather) k_gather32<<<grid1(a.n_total, 256), 256, 0, s>>>(a, a.params);
+		if (!a.skip_gather) k_gather32<<<grid1((uint64_t)a.n_total + 1, 256), 256, 0, s>>>(a, a.params);
 	} else {
-		k_gather64<<<grid1(a.n_total, 256), 256, 0, s>>>(a, a.params);
+		k_gather64<<<grid1((uint64_t)a.n_total + 1, 256), 256, 0, s>>>(a, a.params);
 	}
 	unsigned bs = a.block ? a.block : 128;
 	unsigned grid = a.persistent ? a.grid : grid1(a.n_total, bs);
@@ -1496,13 +1720,14 @@ cudaError_t ul_bc(uint32_t n_bc, const uint32_t* rows, const double* v, double* 
 	return cudaGetLastError();
 }
 
-cudaError_t ul_neighbors(const ULArgs& a, uint32_t* counts, uint32_t* idx, const uint64_t* offs, int pass,
+cudaError_t ul_neighbors(const ULArgs& args, uint32_t* counts, uint32_t* idx, const uint64_t* offs, int pass,
                          cudaStream_t s) {
-	if (a.n_total == 0) return cudaSuccess;
+	if (args.n_total == 0) return cudaSuccess;
+	ULArgs a = args;
 	if (pass == 0) {
 		cudaError_t e = build_grid(a, false, s);
 		if (e != cudaSuccess) return e;
-		k_gather64<<<grid1(a.n_total, 256), 256, 0, s>>>(a, a.params);
+		k_gather64<<<grid1((uint64_t)a.n_total + 1, 256), 256, 0, s>>>(a, a.params);
 	}
 	k_neighbors<<<grid1(a.n_total, 128), 128, 0, s>>>(a, a.geom, counts, idx, offs, pass);
 	return cudaGetLastError();

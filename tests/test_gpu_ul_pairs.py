@@ -122,3 +122,49 @@ def test_large_batch_equals_instances_alone(lib):
         for f in ("x", "y", "vx", "vy", "rho", "Sxx", "Sxy", "Syy"):
             np.testing.assert_array_equal(got[f], want[f], err_msg=f)
     sim.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64_strict", "fp64", "mixed"])
+@pytest.mark.parametrize("dx,instances", [(1e-3, 1), (4e-3, 1), (None, 5), (1e-3, 161)])
+def test_small_body_grid_equals_general(lib, precision, dx, instances):
+    """The grid of small bodies (a block each) against the general kernels, which a context
+    that masks failed bodies always takes: the same cells and order, hence the same bits."""
+    import mfree_iwf_gb300 as M
+    sc = S.c1_rings(dx=dx) if instances == 1 else S.c4_ensemble(instances, dx_range=(3e-3, 4e-3))
+    if instances > 152:  # (a block per SM: bodies up to 4608 rows take this grid too)
+        sc.bodies[7] = S.c4_ensemble(1, dx_range=(dx, dx)).bodies[0]
+    for b in sc.bodies:
+        b.arrays["vx"] += 1.5 * np.sin(200.0 * b.arrays["y"])
+        b.arrays["x"][: 3] -= 0.05  # (and a few particles apart from the rest: empty cells)
+    out = []
+    for general in (0, 1):
+        sim = M.from_scenario(sc, precision=precision)
+        sim.set_option("mask_failed", general)
+        try:
+            sim.step(4)
+        except M.MfError as e:  # a particle without neighbours counts itself: none expected
+            pytest.fail(str(e))
+        out.append([sim.get_state(k) for k in range(len(sc.bodies))])
+        sim.close()
+    for a, b in zip(*out):
+        for f in ("x", "y", "vx", "vy", "rho", "Sxx", "Sxy", "Syy"):
+            np.testing.assert_array_equal(a[f], b[f], err_msg=f)
+
+
+def test_small_body_grid_with_scattered_particles(lib):
+    """A body whose cells outnumber its particles (the mixed form allows it up to three a
+    particle and context): the counters stand in the cell table itself."""
+    import mfree_iwf_gb300 as M
+    out = []
+    for general in (0, 1):
+        sc = S.c4_ensemble(3, dx_range=(2e-3, 4e-3))
+        a = sc.bodies[1].arrays
+        a["x"][0] -= 1.2  # a particle far off stretches the box to more than two cells a particle
+        sim = M.from_scenario(sc, precision="mixed")
+        sim.set_option("mask_failed", general)
+        sim.step(3)
+        out.append([sim.get_state(k) for k in range(3)])
+        sim.close()
+    for a, b in zip(*out):
+        for f in ("x", "y", "vx", "vy", "rho", "Sxx"):
+            np.testing.assert_array_equal(a[f], b[f], err_msg=f)
