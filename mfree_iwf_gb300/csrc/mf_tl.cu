@@ -766,20 +766,25 @@ __global__ void __launch_bounds__(256, 5) k_tlB32(TLArgs a) {
 // 10 / (7 pi) of the 2-D cubic spline (kernel.cpp:24)
 constexpr float K_SPLINE_2D = 0.45472840883398667f;
 
-// Corrected gradient of pair (i, j): the cubic spline's gradient at X_i - X_j (zero
-// at r >= 2h and for r <= 1e-12, kernel.cpp:20-55) times the row's invB / C.
-__device__ __forceinline__ float2 rl_grad32(float4 Xi, float4 Xj, float4 Gi, float h1, float fac) {
-	float xij = ffd(Xi.x, Xi.y, Xj.x, Xj.y), yij = ffd(Xi.z, Xi.w, Xj.z, Xj.w);
-	float r2 = xij * xij + yij * yij;
-	float rinv = rsqrtf(fmaxf(r2, 1e-30f));
-	float q = r2 * rinv * h1;
-	float der = 0.f;
-	if (q < 2.f && r2 > 1e-24f) {
-		float t = 2.f - q;
-		der = (q >= 1.f ? -0.75f * t * t : -3.0f * q * (1.f - 0.75f * q)) * h1 * rinv * fac;
-	}
-	float gx = xij * der, gy = yij * der;
-	return make_float2(gx * Gi.x + gy * Gi.y, gx * Gi.z + gy * Gi.w);
+// grad W of pair (i, j) over 3 fac (fac = K_SPLINE_2D / h^2, applied to the row's sums) at
+// X_i - X_j: the cubic spline's (zero at r >= 2h and for r <= 1e-12, kernel.cpp:20-55) as
+// dW/dq ~ u^2 - t^2 / 4 with t = max(2 - q, 0), u = max(1 - q, 0), one expression for both
+// pieces; times `scale`.  The correction invB / C is linear and the same for all pairs of
+// a row, so it too is applied to the row's sums.  (With two pieces and the correction in
+// every pair the passes took 43.3 and 67.2 us at 440k rows, now 37.4 and 68.1 under the
+// profiler; a step of the ring impact at dx = 0.05 mm, 1.76M rows, 1717 us, now 1650:
+// pass A was bound by instructions; pass B, with fewer of them, by the latency of its
+// gathers, which this leaves.)
+__device__ __forceinline__ float2 rl_grad32(float4 Xi, float4 Xj, float h1, float scale) {
+	const float xij = ffd(Xi.x, Xi.y, Xj.x, Xj.y), yij = ffd(Xi.z, Xi.w, Xj.z, Xj.w);
+	const float r2 = xij * xij + yij * yij;
+	float rinv;  // (no rescaling of subnormals: they are cut off below)
+	asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rinv) : "f"(r2));
+	const float sr = r2 > 1e-24f ? rinv * h1 : 0.f;  // 1 / (r h)
+	const float q = r2 * sr;
+	const float t = fmaxf(2.f - q, 0.f), u = fmaxf(1.f - q, 0.f);
+	const float g = (u * u - 0.25f * t * t) * (sr * scale);
+	return make_float2(xij * g, yij * g);
 }
 
 // Pass A's gathers of one pair: reference position, quad weight, displacement and
@@ -797,15 +802,13 @@ __device__ __forceinline__ PairA tlA_load(const TLArgs& a, uint32_t j) {
 	return p;
 }
 
+// Sums of the displacement (velocity) differences times the uncorrected gradient
 struct AccA {
 	float Hxx = 0.f, Hxy = 0.f, Hyx = 0.f, Hyy = 0.f;
 	float Fxx = 0.f, Fxy = 0.f, Fyx = 0.f, Fyy = 0.f;
 };
-__device__ __forceinline__ void tlA_add(uint32_t flags, const PairA& p, float4 Xi, float4 Gi, float h1, float fac,
-                                        float4 ui, float4 vi, AccA& s) {
-	float2 w = rl_grad32(Xi, p.X, Gi, h1, fac);
-	w.x *= p.qw;  // times the neighbour's quad weight
-	w.y *= p.qw;
+__device__ __forceinline__ void tlA_add(uint32_t flags, const PairA& p, float4 Xi, float h1, float4 ui, float4 vi, AccA& s) {
+	const float2 w = rl_grad32(Xi, p.X, h1, p.qw);  // times the neighbour's quad weight
 	if (flags & A_DISP) {
 		float dux = ffd(p.u.x, p.u.y, ui.x, ui.y), duy = ffd(p.u.z, p.u.w, ui.z, ui.w);
 		s.Hxx += dux * w.x;
@@ -832,8 +835,8 @@ __global__ void __launch_bounds__(256, MB) k_tlA32r(TLArgs a) {
 	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= a.n_total) return;
 	const uint32_t flags = a.flags;
-	const float4 Xi = ((const float4*)a.XF)[i], Gi = ((const float4*)a.G)[i];
-	const float h1 = 1.f / ((const float*)a.h32)[i], fac = K_SPLINE_2D * h1 * h1;
+	const float4 Xi = ((const float4*)a.XF)[i];
+	const float h1 = 1.f / ((const float*)a.h32)[i];
 	const float4 ui = ((const float4*)a.recA)[i];
 	const float4 vi = rb_field(a.recB, a.n_total, RB_V)[i];
 	AccA s;
@@ -842,30 +845,36 @@ __global__ void __launch_bounds__(256, MB) k_tlA32r(TLArgs a) {
 		const uint32_t run = a.runs[q];
 		const uint32_t j0 = run & (TL_RUN_MAX_ROWS - 1u), j1 = j0 + (run >> TL_RUN_SHIFT) + 1u;
 		if (U == 1) {
-			for (uint32_t j = j0; j < j1; j++) tlA_add(flags, tlA_load(a, j), Xi, Gi, h1, fac, ui, vi, s);
+			for (uint32_t j = j0; j < j1; j++) tlA_add(flags, tlA_load(a, j), Xi, h1, ui, vi, s);
 		} else {
 			for (uint32_t j = j0; j < j1; j += 2) {
 				const bool two = j + 1 < j1;
 				const PairA p0 = tlA_load(a, j), p1 = tlA_load(a, two ? j + 1 : j);
-				tlA_add(flags, p0, Xi, Gi, h1, fac, ui, vi, s);
-				if (two) tlA_add(flags, p1, Xi, Gi, h1, fac, ui, vi, s);
+				tlA_add(flags, p0, Xi, h1, ui, vi, s);
+				if (two) tlA_add(flags, p1, Xi, h1, ui, vi, s);
 			}
 		}
 	}
-	tlA_finish(a, i, s.Hxx, s.Hxy, s.Hyx, s.Hyy, s.Fxx, s.Fxy, s.Fyx, s.Fyy);
+	// the corrected gradient of a pair is (G.x gx + G.y gy, G.z gx + G.w gy), G = 3 fac invB / C
+	float4 G = ((const float4*)a.G)[i];
+	const float f3 = 3.f * K_SPLINE_2D * h1 * h1;
+	G.x *= f3; G.y *= f3; G.z *= f3; G.w *= f3;
+	tlA_finish(a, i, s.Hxx * G.x + s.Hxy * G.y, s.Hxx * G.z + s.Hxy * G.w, s.Hyx * G.x + s.Hyy * G.y,
+	           s.Hyx * G.z + s.Hyy * G.w, s.Fxx * G.x + s.Fxy * G.y, s.Fxx * G.z + s.Fxy * G.w,
+	           s.Fyx * G.x + s.Fyy * G.y, s.Fyx * G.z + s.Fyy * G.w);
 }
 
 // Pass B's gathers of one pair: row j's record and reference position.
 struct PairB {
 	float4 P, x, v, hmrc, X;
 };
-__device__ __forceinline__ PairB tlB_load(const TLArgs& a, uint32_t j) {
+__device__ __forceinline__ PairB tlB_load(const TLArgs& a, uint32_t flags, uint32_t j) {
 	const uint32_t n = a.n_total;
 	PairB p;
 	p.hmrc = __ldg(rb_field(a.recB, n, RB_H) + j);
 	p.X = __ldg((const float4*)a.XF + j);
-	p.P = (a.flags & A_STRESS_TL) ? __ldg(rb_field(a.recB, n, RB_P) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-	if (a.flags & A_ART_VISC) {
+	p.P = (flags & A_STRESS_TL) ? __ldg(rb_field(a.recB, n, RB_P) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+	if (flags & A_ART_VISC) {
 		p.x = __ldg(rb_field(a.recB, n, RB_X) + j);
 		p.v = __ldg(rb_field(a.recB, n, RB_V) + j);
 	} else {
@@ -874,31 +883,38 @@ __device__ __forceinline__ PairB tlB_load(const TLArgs& a, uint32_t j) {
 	return p;
 }
 
+// Pass B's sums: of m_j (P_i + P_j - rho0^2 Pi_ij I) grad w_ij, with the row's own P_i by
+// the sum of the gradients.  The stress forces and the viscosity share them, rho0^2 being
+// the common scale of the momentum equation's stress term (1 / rho0^2 at the end).
 struct AccB {
-	float Pxx_x = 0.f, Pyx_y = 0.f, Pxy_x = 0.f, Pyy_y = 0.f, av_x = 0.f, av_y = 0.f;
+	float ax = 0.f, ay = 0.f, wx = 0.f, wy = 0.f;
 };
-__device__ __forceinline__ void tlB_add(uint32_t flags, const PairB& p, const RecB& ri, float4 Xi, float4 Gi, float h1,
-                                        float fac, float sc, float alpha, float beta, float eta2, AccB& s) {
-	float2 w = rl_grad32(Xi, p.X, Gi, h1, fac);
-	w.x *= p.hmrc.y;  // times the neighbour's mass
-	w.y *= p.hmrc.y;
-	if (flags & A_STRESS_TL) {
-		float fx = sc * w.x, fy = sc * w.y;
-		s.Pxx_x += (ri.P.x + p.P.x) * fx;
-		s.Pyx_y += (ri.P.z + p.P.z) * fy;
-		s.Pxy_x += (ri.P.y + p.P.y) * fx;
-		s.Pyy_y += (ri.P.w + p.P.w) * fy;
-	}
+// Per-row constants: 1/h; 3 fac invB / C; eta^2 / 4, beta rho0^2 / 2, alpha rho0^2 / 2
+struct RowB {
+	float h1, eta2q, half_beta, half_alpha;
+	float4 G;
+};
+__device__ __forceinline__ void tlB_add(uint32_t flags, const PairB& p, const RecB& ri, float4 Xi, const RowB& k, AccB& s) {
+	const float2 g = rl_grad32(Xi, p.X, k.h1, p.hmrc.y);  // times the neighbour's mass
+	const float wx = g.x * k.G.x + g.y * k.G.y, wy = g.x * k.G.z + g.y * k.G.w;
+	float pi2 = 0.f;  // rho0^2 Pi_ij
 	if (flags & A_ART_VISC) {
-		float xij = ffd(ri.x.x, ri.x.y, p.x.x, p.x.y), yij = ffd(ri.x.z, ri.x.w, p.x.z, p.x.w);
-		float vijx = ffd(ri.v.x, ri.v.y, p.v.x, p.v.y), vijy = ffd(ri.v.z, ri.v.w, p.v.z, p.v.w);
-		float vijposij = approach(vijx, vijy, xij, yij);
-		if (vijposij < 0.f) {
-			float piij = art_visc_pi(ri.hmrc, p.hmrc, xij, yij, vijposij, alpha, beta, eta2);
-			s.av_x += -piij * w.x;
-			s.av_y += -piij * w.y;
+		const float xij = ffd(ri.x.x, ri.x.y, p.x.x, p.x.y), yij = ffd(ri.x.z, ri.x.w, p.x.z, p.x.w);
+		const float dvx = ffd(p.v.x, p.v.y, ri.v.x, ri.v.y), dvy = ffd(p.v.z, p.v.w, ri.v.z, ri.v.w);
+		const float dot = dvx * xij + dvy * yij;  // -v_ij . x_ij
+		if (dot > 0.f) {                          // approaching
+			// with n = 2 h_ij dot, D = r^2 + eta^2 h_ij^2, rs = rho_i + rho_j and
+			// A = 1 / (D rs): Pi = n A (alpha c_ij + beta / 2 n A rs)
+			const float hs = ri.hmrc.x + p.hmrc.x, rs = ri.hmrc.z + p.hmrc.z;
+			const float D = xij * xij + yij * yij + k.eta2q * hs * hs;
+			const float nA = __fdividef(hs * dot, D * rs);
+			pi2 = nA * (k.half_alpha * (ri.hmrc.w + p.hmrc.w) + k.half_beta * rs * nA);
 		}
 	}
+	s.ax += (p.P.x - pi2) * wx + p.P.z * wy;
+	s.ay += p.P.y * wx + (p.P.w - pi2) * wy;
+	s.wx += wx;
+	s.wy += wy;
 }
 
 // MB: blocks of 256 per SM the register budget is cut for (3: 72 registers; 4: 64,
@@ -907,15 +923,20 @@ template <int U, int MB>
 __global__ void __launch_bounds__(256, MB) k_tlB32r(TLArgs a) {
 	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= a.n_total) return;
-	const uint32_t flags = a.flags;
+	// (the stress sums only reach the momentum equation)
+	const uint32_t flags = (a.flags & A_MOMENTUM_TL) ? a.flags : a.flags & ~A_STRESS_TL;
 	const BodyParams& pr = a.params[a.body_of[i]];
-	const float rho0 = pr.frho0;
-	const float r21 = 1.f / (rho0 * rho0);
-	const float sc = r21 * rho0;
+	const float rho0 = pr.frho0, rho02 = rho0 * rho0;
 	const RecB ri = rb_load(a.recB, a.n_total, i);
-	const float4 Xi = ((const float4*)a.XF)[i], Gi = ((const float4*)a.G)[i];
-	const float h1 = 1.f / ri.hmrc.x, fac = K_SPLINE_2D * h1 * h1;
-	const float alpha = pr.falpha, beta = pr.fbeta, eta2 = pr.feta2;
+	const float4 Xi = ((const float4*)a.XF)[i];
+	RowB rk;
+	rk.h1 = 1.f / ri.hmrc.x;
+	rk.eta2q = 0.25f * pr.feta2;
+	rk.half_alpha = 0.5f * pr.falpha * rho02;
+	rk.half_beta = 0.5f * pr.fbeta * rho02;
+	rk.G = ((const float4*)a.G)[i];
+	const float f3 = 3.f * K_SPLINE_2D * rk.h1 * rk.h1;
+	rk.G.x *= f3; rk.G.y *= f3; rk.G.z *= f3; rk.G.w *= f3;
 	AccB s;
 	uint32_t q = a.r_sl[i >> 5] + (i & 31u), nr = a.r_cnt[i];
 	for (uint32_t r = 0; r < nr; r++, q += 32) {
@@ -923,17 +944,24 @@ __global__ void __launch_bounds__(256, MB) k_tlB32r(TLArgs a) {
 		const uint32_t j0 = run & (TL_RUN_MAX_ROWS - 1u), j1 = j0 + (run >> TL_RUN_SHIFT) + 1u;
 		if (U == 1) {
 			for (uint32_t j = j0; j < j1; j++)
-				tlB_add(flags, tlB_load(a, j), ri, Xi, Gi, h1, fac, sc, alpha, beta, eta2, s);
+				tlB_add(flags, tlB_load(a, flags, j), ri, Xi, rk, s);
 		} else {
 			for (uint32_t j = j0; j < j1; j += 2) {
 				const bool two = j + 1 < j1;
-				const PairB p0 = tlB_load(a, j), p1 = tlB_load(a, two ? j + 1 : j);
-				tlB_add(flags, p0, ri, Xi, Gi, h1, fac, sc, alpha, beta, eta2, s);
-				if (two) tlB_add(flags, p1, ri, Xi, Gi, h1, fac, sc, alpha, beta, eta2, s);
+				const PairB p0 = tlB_load(a, flags, j), p1 = tlB_load(a, flags, two ? j + 1 : j);
+				tlB_add(flags, p0, ri, Xi, rk, s);
+				if (two) tlB_add(flags, p1, ri, Xi, rk, s);
 			}
 		}
 	}
-	tlB_finish(a, i, pr, rho0, s.Pxx_x, s.Pyx_y, s.Pxy_x, s.Pyy_y, s.av_x, s.av_y);
+	// the sums over rho0^2 are handed on as the viscosity's share (tlB_finish adds the
+	// contact force)
+	if (flags & A_STRESS_TL) {
+		s.ax += ri.P.x * s.wx + ri.P.z * s.wy;
+		s.ay += ri.P.y * s.wx + ri.P.w * s.wy;
+	}
+	const float r21 = 1.f / rho02;
+	tlB_finish(a, i, pr, rho0, 0.f, 0.f, 0.f, 0.f, s.ax * r21, s.ay * r21);
 }
 
 // ---- mixed form over halo tiles.  The same per-row arithmetic, in the same order, as
