@@ -445,47 +445,58 @@ __global__ void __launch_bounds__(THREADS, 1)
 }  // namespace tc
 
 // Fused inference: the whole forward pass of every member in one persistent kernel,
-// the hidden activations never leaving the SM.  A CTA takes tiles of 256 rows of one
-// member (two halves of 128 rows, one TMEM accumulator of up to 256 FP32 columns each)
-// and runs them through all layers:
+// the hidden activations never leaving the SM.  A pair of CTAs (a cluster, on two SMs)
+// takes tiles of 512 rows of one member, two halves of 256 rows, 128 of a half's in each
+// CTA (one TMEM accumulator of up to 256 FP32 columns per half and CTA), and runs them
+// through all layers:
 //   - the epilogue warps write the tile's input rows (FP32 -> BF16, zero padded to the
 //     first layer's K) into shared memory in the 128-byte-swizzled K-major layout that
 //     a TMA load would produce, so the tensor core reads them as an operand: per 64-wide
-//     K chunk the 256 rows in order (half 0's 128, then half 1's);
-//   - the producer (warp 0) streams each layer's BF16 weights, 64-wide K chunks of all
-//     N rows, through a ring of shared-memory stages with TMA;
-//   - the MMA issuer (warp 1) multiplies, per K chunk, both halves (A = the half's rows,
-//     B = the weights: M = 128, N = the layer's width) and commits each half's
-//     accumulator after its last chunk.  An M = 128 product takes about as long for any
-//     N up to 256, so the narrow output layer runs transposed: A = its weights (the
-//     outputs padded to 128 or 256 rows by the tensor map's zero fill), B = all 256 rows
-//     of the tile (N = 256), half the products of two M = 128 halves;
-//   - the epilogue warps (8: four TMEM lane quarters x two halves) read their half's
-//     accumulator (two TMEM loads in flight: the next 32 columns load while these are
-//     converted), add the bias, apply ReLU, round to BF16 and write the next layer's
-//     operand over the current one (whose products are complete by then); after the
-//     output layer a warp holds 32 consecutive outputs (TMEM lanes) of its half's rows
-//     (columns), adds the bias and stores each row's 32 outputs with one coalesced store.
-// Only the inputs (in FP32), the weights (from L2: every CTA on a member reads the same
+//     K chunk the CTA's 256 rows in order (half 0's 128, then half 1's);
+//   - the producers (warp 0 of each CTA) stream each layer's BF16 weights, 64-wide K
+//     chunks, through a ring of shared-memory stages with TMA, half of the chunk's N rows
+//     to each CTA, both reporting to the first CTA's barrier;
+//   - the MMA issuer (warp 1 of the first CTA) multiplies with cta_group::2: A = a half's
+//     256 rows, B = the chunk's N weight rows, each CTA holding half of both.  A layer's
+//     chunks stay in the ring for both halves: half 0's epilogue runs under half 1's
+//     products, and half 0's next products under half 1's epilogue;
+//   - the epilogue warps (16 in each CTA: four TMEM lane quarters x two halves x two
+//     column sets) read their half's accumulator, add the bias, apply ReLU, round to BF16
+//     and write the next layer's operand over the current one (whose products are complete
+//     by then); the output layer's rows go through shared memory, 16 outputs at a time, for
+//     coalesced stores, the next tile's input having been handed on before the last of them.
+// Why pairs: the products of a 256 x 256 layer of 256 rows take an SM about 4,500 clocks
+// and the epilogue as long, so one has to run under the other.  A CTA by itself has 96 KB
+// left for weights beside its activations, less than the 128 KB of one such layer, and
+// its halves could be no more than a chunk or two apart; half the weights in each CTA
+// make room for a layer and a chunk, and are read from L2 half as often.  262,140 rows,
+// 5 members, 6-256-256-256-66: 626 us with single CTAs and both halves in step; 575 with
+// the issuer's ring divisions out and 16 epilogue warps; 510 with pairs and an elected
+// issuing lane; 422 with 16-column TMEM loads ahead of the conversions and two bias
+// copies, 403 with the half loops spelled out (the products alone: 196 us).  What is left is each half's own chain: products,
+// epilogue, handing over.
+// Only the inputs (in FP32), the weights (from L2: every pair on a member reads the same
 // ones) and the outputs move through memory.  The products are the per-layer path's --
 // BF16 operands, FP32 accumulation in K order, the bias added in FP32 -- with K padded
 // to 64 by zeros.  Every wait is bounded; on a timeout the kernel sets the error word,
 // waits (bounded) for its own copies and products in flight, frees the TMEM and returns.
 namespace fz {
 
-constexpr int TILE = 256, HALF = 128;
-constexpr int CHUNK = HALF * 128;  // one 64-wide K chunk of a half: 128 rows x 128 bytes
-constexpr int EPI = 8;
+constexpr int HALF = 128;            // rows of a half in one CTA
+constexpr int TILE = 4 * HALF;       // two halves, two CTAs
+constexpr int CHUNK = HALF * 128;    // one 64-wide K chunk of a half's rows: 128 rows x 128 bytes
+constexpr int EPI = 16;              // epilogue warps: two per half and TMEM lane quarter
 constexpr int THREADS = 64 + 32 * EPI;
+constexpr int HALF_WARPS = EPI / 2;
+constexpr int STAGES = 5;            // weight chunks in shared memory: a layer's (K <= 256) and one more
 constexpr uint32_t TMEM_COLS = 512;  // two accumulators of up to 256 columns
 
 struct Maps {
-	CUtensorMap w[MF_MLP_MAX_LAYERS];  // per layer: [members][N][K] BF16, boxes of 64 K x N rows
+	CUtensorMap w[MF_MLP_MAX_LAYERS];  // per layer: [members][N][K] BF16, boxes of 64 K x N / 2 rows
 };
 struct Args {
-	int L, in, out, rows, stages, kc_max, n_max;
+	int L, in, out, rows, kc_max, n_max;
 	int N[MF_MLP_MAX_LAYERS], KC[MF_MLP_MAX_LAYERS];  // MMA width (padded to 16); K / 64 (K padded to 64)
-	int mb_last;                                       // 128-row blocks of the transposed output layer (1 or 2)
 	int b_off[MF_MLP_MAX_LAYERS];
 	const float* bias;
 	long long b_per;
@@ -499,12 +510,14 @@ struct Args {
 
 // the mbarriers (2 per weight stage, 2 x 2 per half, 1 to drain) and the TMEM address,
 // rounded up to 16 bytes
-__host__ __device__ constexpr size_t bar_bytes(int stages) { return (8 * (2 * stages + 5) + 4 + 15) / 16 * 16; }
-// shared memory: 1 KB for the 1 KB alignment of the swizzled operands, the operand
-// chunks of the tile, the weight stages, the barriers and one layer's bias
-__host__ __device__ constexpr size_t smem_bytes(int kc_max, int n_max, int stages) {
-	return 1024 + (size_t)2 * kc_max * CHUNK + (size_t)stages * n_max * 128 + bar_bytes(stages) + (size_t)n_max * 4;
+constexpr size_t BAR_BYTES = (8 * (2 * STAGES + 5) + 4 + 15) / 16 * 16;
+// shared memory: the operand chunks of the tile, the weight stages, the barriers and each
+// half's two copies of a layer's bias (the current one's and the next one's).  (The swizzled operands need 1 KB alignment,
+// which the start of dynamic shared memory has; the kernel checks it.)
+__host__ __device__ constexpr size_t smem_bytes(int kc_max, int n_max) {
+	return (size_t)2 * kc_max * CHUNK + (size_t)STAGES * n_max * 64 + BAR_BYTES + (size_t)4 * n_max * 4;
 }
+static_assert(smem_bytes(4, 256) <= 227 * 1024, "the widest layers fit");
 
 // the 16-byte unit holding columns col .. col + 7 (col a multiple of 8) of row r of half
 // h: K chunk col / 64 (the chunk's 256 rows: half 0, then half 1), unit (col % 64) / 8
@@ -524,63 +537,129 @@ __device__ __forceinline__ uint32_t pack2_relu(float a, float b) {
 	asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;\n" : "=r"(d) : "f"(b), "f"(a));
 	return d;
 }
-// 32 columns of the warp's 32 TMEM lanes without waiting (tmem_wait before use)
-__device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, uint32_t* r) {
-	asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-	             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+__device__ __forceinline__ void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+// 16 columns of the warp's 32 TMEM lanes without waiting (tmem_wait before use)
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t* r) {
+	asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+	             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
 	             : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
-// named barrier 1 over the 256 epilogue threads; epi_all also returns the AND of p over them
-__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 256;\n" ::: "memory"); }
-__device__ __forceinline__ bool epi_all(bool p) {
+
+// ---- the pair of CTAs.  Rank 0 issues the products and holds their barriers.
+__device__ __forceinline__ uint32_t cluster_rank() {
 	uint32_t r;
-	asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %1, 0;\nbar.red.and.pred q, 1, 256, q;\nselp.u32 %0, 1, 0, q;\n}\n"
+	asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+	return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+	asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
+// the address of rank 0's copy of a shared-memory object
+__device__ __forceinline__ uint32_t in_rank0(const void* p) {
+	uint32_t a;
+	asm volatile("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(a) : "r"(tc::saddr(p)));
+	return a;
+}
+// An arrival at a barrier of either CTA, of the default (CTA) scope: what it vouches for --
+// this CTA's operand, behind the writers' proxy fences, and its accumulators, behind
+// tcgen05.fence -- is only touched again by this SM's own tensor core.  (A release at
+// cluster scope waits for all earlier stores of the thread: 602 us instead of 529, see
+// k_mlp_fused.)
+__device__ __forceinline__ void arrive_cluster(uint32_t bar) {
+	asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+// one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+	uint32_t r;
+	asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(r)::"memory");
+	return r != 0;
+}
+// tc::mbar_wait of a whole warp, which agrees on the outcome
+__device__ __forceinline__ bool wait_warp(uint64_t* b, uint32_t ph) { return __all_sync(0xffffffffu, tc::mbar_wait(b, ph)); }
+// a box to this CTA's shared memory, its bytes reported to `bar` of either CTA
+__device__ __forceinline__ void tma_load_pair(void* dst, const CUtensorMap* tm, int x, int y, int z, uint32_t bar) {
+	asm volatile(
+	    "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(
+	        tc::saddr(dst)),
+	    "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(z), "r"(bar)
+	    : "memory");
+}
+__device__ __forceinline__ void mma_pair(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
+	asm volatile(
+	    "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+	    "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+	    : "memory");
+}
+// the products issued so far -> one arrival at this barrier of both CTAs
+__device__ __forceinline__ void commit_pair(uint64_t* bar) {
+	asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(
+	                 tc::saddr(bar)),
+	             "h"((uint16_t)3)
+	             : "memory");
+}
+
+// barrier over the epilogue threads of half h (named barrier 1 + h); the AND of p over them
+__device__ __forceinline__ bool half_all(int h, bool p) {
+	uint32_t r;
+	asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %1, 0;\nbar.red.and.pred q, %2, %3, q;\nselp.u32 %0, 1, 0, q;\n}\n"
 	             : "=r"(r)
-	             : "r"((uint32_t)p)
+	             : "r"((uint32_t)p), "r"(1 + h), "n"(32 * HALF_WARPS)
 	             : "memory");
 	return r != 0;
 }
 
-// 32 accumulator columns col0 .. col0 + 31 of row r (in v) -> bias (sb4: the layer's bias
-// in shared memory), ReLU, BF16 -> their four 16-byte units of the next operand; columns
-// at or past N (the layer's width) become zeros up to the next layer's K
-__device__ __forceinline__ void hidden_units(uint8_t* act, int h, int r, int col0, int N, const uint32_t* v,
-                                             const float4* sb4) {
+// (a + b, rounded as two FP32 additions)
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+	float2 d;
+	asm("{\n.reg .b64 x, y;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nadd.rn.f32x2 x, x, y;\nmov.b64 {%0, %1}, x;\n}\n"
+	    : "=f"(d.x), "=f"(d.y)
+	    : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+	return d;
+}
+// 16 accumulator columns col0 .. col0 + 15 of row r (in v) -> bias (sb: the layer's in
+// shared memory), ReLU, BF16 -> their two 16-byte units of the next operand; columns at or
+// past N (the layer's width, a multiple of 16) become zeros up to the next layer's K
+__device__ __forceinline__ void hidden_units(uint8_t* act, int h, int r, int col0, int N, const uint32_t* v, const float* sb) {
+	uint32_t w[8] = {};
+	if (col0 < N) {
+		const float4* b4 = reinterpret_cast<const float4*>(sb + col0);
 #pragma unroll
-	for (int u = 0; u < 4; u++) {
-		const int col = col0 + 8 * u;
-		uint4 w = make_uint4(0, 0, 0, 0);
-		if (col < N) {
-			const float4 b0 = sb4[col >> 2], b1 = sb4[(col >> 2) + 1];
-			float f[8];
-#pragma unroll
-			for (int e = 0; e < 8; e++) f[e] = __uint_as_float(v[8 * u + e]);
-			w = make_uint4(pack2_relu(f[0] + b0.x, f[1] + b0.y), pack2_relu(f[2] + b0.z, f[3] + b0.w),
-			               pack2_relu(f[4] + b1.x, f[5] + b1.y), pack2_relu(f[6] + b1.z, f[7] + b1.w));
+		for (int u = 0; u < 4; u++) {
+			const float4 b = b4[u];
+			const float2 f = add2(make_float2(__uint_as_float(v[4 * u]), __uint_as_float(v[4 * u + 1])), make_float2(b.x, b.y));
+			const float2 g = add2(make_float2(__uint_as_float(v[4 * u + 2]), __uint_as_float(v[4 * u + 3])), make_float2(b.z, b.w));
+			w[2 * u] = pack2_relu(f.x, f.y);
+			w[2 * u + 1] = pack2_relu(g.x, g.y);
 		}
-		*unit_at(act, h, r, col) = w;
 	}
+	*unit_at(act, h, r, col0) = make_uint4(w[0], w[1], w[2], w[3]);
+	*unit_at(act, h, r, col0 + 8) = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     k_mlp_fused(const __grid_constant__ Maps maps, const Args a, uint32_t* err) {
 	using namespace tc;
-	extern __shared__ uint8_t smem_raw[];
-	const uint32_t raw = saddr(smem_raw);
-	uint8_t* act = smem_raw + (((raw + 1023u) & ~1023u) - raw);
-	const size_t wst = (size_t)a.n_max * 128;
-	const int S = a.stages, L = a.L;
+	extern __shared__ __align__(1024) uint8_t smem_raw[];
+	if (saddr(smem_raw) & 1023u) {  // (the driver's layout has always been aligned)
+		atomicOr(err, 1u);
+		return;
+	}
+	uint8_t* act = smem_raw;
+	const size_t wst = (size_t)a.n_max * 64;  // half of a chunk's rows
+	constexpr int S = STAGES;
+	const int L = a.L;
 	uint8_t* sW = act + (size_t)2 * a.kc_max * CHUNK;
-	uint64_t* w_full = reinterpret_cast<uint64_t*>(sW + (size_t)S * wst);
+	uint64_t* w_full = reinterpret_cast<uint64_t*>(sW + (size_t)S * wst);  // rank 0's: both CTAs' boxes have landed
 	uint64_t* w_empty = w_full + S;
 	uint64_t* acc_full = w_empty + S;    // per half: the layer's products are complete
-	uint64_t* act_ready = acc_full + 2;  // per half: the operand of the next layer is written
+	uint64_t* act_ready = acc_full + 2;  // rank 0's, per half: both CTAs have written the next layer's operand
 	uint64_t* fin = act_ready + 2;
 	uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(fin + 1);
-	float* sbias = reinterpret_cast<float*>(sW + (size_t)S * wst + bar_bytes(S));  // the current layer's bias
+	float* sbias = reinterpret_cast<float*>(sW + (size_t)S * wst + BAR_BYTES);  // per half and step parity: a layer's bias
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const uint32_t rank = cluster_rank();
 	const int tpm = (a.rows + TILE - 1) / TILE, total = tpm * a.members;
+	const int first = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 
 	if (threadIdx.x == 0) {
 		for (int s = 0; s < S; s++) {
@@ -589,208 +668,241 @@ __global__ void __launch_bounds__(THREADS, 1)
 		}
 		for (int h = 0; h < 2; h++) {
 			mbar_init(acc_full + h, 1);
-			mbar_init(act_ready + h, 32 * EPI / 2);  // every thread of the half's four warps
+			mbar_init(act_ready + h, 2 * HALF_WARPS);  // the half's warps of both CTAs
 		}
 		mbar_init(fin, 1);
 		asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 	}
 	if (warp == 1) {
-		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(saddr(tmem_slot)),
+		asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(saddr(tmem_slot)),
 		             "r"(TMEM_COLS)
 		             : "memory");
-		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
 	}
 	fence_before();
 	__syncthreads();
+	cluster_sync();
 	fence_after();
-	const uint32_t tmem = *tmem_slot;
-	bool ok = true;
+	const uint32_t tmem = *tmem_slot;  // (all columns: the same address in both CTAs)
+	bool ok = true, good = true;
 
 	if (warp == 0) {
 		if (lane == 0) {  // weight producer
-			uint32_t it = 0;
-			for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+			// (ring positions are counted: the divisions of an index cost the issuer below more
+			// than the products of a chunk)
+			int st = 0, loads = 0;
+			uint32_t ph = 1;  // parity of the phase that frees the stage (the first round waits for none)
+			for (int t = first; t < total && ok; t += pairs) {
 				const int z = t % a.members;
 				for (int l = 0; l < L && ok; l++) {
-					// the output layer's box is 128 * mb_last rows, zero filled past its width
-					const uint32_t bytes = (uint32_t)(l + 1 < L ? a.N[l] : 128 * a.mb_last) * 128u;
-					for (int kc = 0; kc < a.KC[l]; kc++, it++) {
-						const int s = (int)(it % S);
-						const uint32_t use = it / S;
-						if (use > 0 && !(ok = mbar_wait(w_empty + s, (use - 1) & 1u))) break;
-						mbar_expect_tx(w_full + s, bytes);
-						tma_load_3d(sW + (size_t)s * wst, &maps.w[l], kc * 64, 0, z, w_full + s);
+					const int rows = a.N[l] >> 1;
+					for (int kc = 0; kc < a.KC[l]; kc++) {
+						if (loads == S && !(ok = mbar_wait(w_empty + st, ph))) break;
+						if (rank == 0) mbar_expect_tx(w_full + st, 2u * (uint32_t)rows * 128u);
+						tma_load_pair(sW + (size_t)st * wst, &maps.w[l], kc * 64, (int)rank * rows, z, in_rank0(w_full + st));
+						loads = min(loads + 1, S);
+						if (++st == S) {
+							st = 0;
+							ph ^= 1u;
+						}
 					}
 				}
 			}
-			// the loads still in flight land before the CTA leaves (consumed ones: at once)
-			for (uint32_t k = it > (uint32_t)S ? it - S : 0; k < it; k++) mbar_wait(w_full + k % S, (k / S) & 1u);
+			// the loads still in flight land, and are used, before the CTA leaves: the last
+			// `loads` stages, the newest just before st
+			for (int k = 0; k < loads; k++) {
+				if (--st < 0) {
+					st = S - 1;
+					ph ^= 1u;
+				}
+				if (rank == 0) mbar_wait(w_full + st, ph ^ 1u);
+				mbar_wait(w_empty + st, ph ^ 1u);
+			}
 		}
 	} else if (warp == 1) {
-		if (lane == 0) {  // MMA issuer
-			uint32_t it = 0, step = 0;
+		if (rank == 0) {  // MMA issuer: the whole warp walks along, one elected lane issues
+			// (issued from a branch of lane 0, a product took 150 clocks to issue whatever its N:
+			// its operands are warp-uniform registers, which a divergent branch has to gather)
+			uint32_t step = 0, ph = 0;
+			int st = 0;  // ring stage of the layer's next chunk (ph: its phase)
 			bool issued = false;
-			for (int t = blockIdx.x; t < total && ok; t += gridDim.x)
+			const uint64_t act_d = sw128_desc(saddr(act)), w_d = sw128_desc(saddr(sW));
+			const uint32_t w16 = (uint32_t)(wst >> 4);  // (descriptors count 16 bytes)
+			for (int t = first; t < total && ok; t += pairs)
 				for (int l = 0; l < L && ok; l++, step++) {
-					if (!(ok = mbar_wait(act_ready, step & 1u)) || !(ok = mbar_wait(act_ready + 1, step & 1u))) break;
-					fence_after();
-					const bool last = l + 1 == L;
-					const uint32_t idesc = last ? idesc_bf16(HALF, TILE) : idesc_bf16(HALF, a.N[l]);
-					for (int kc = 0; kc < a.KC[l]; kc++, it++) {
-						const int s = (int)(it % S);
-						if (!(ok = mbar_wait(w_full + s, (it / S) & 1u))) break;
-						fence_after();
-						const uint32_t wb = saddr(sW + (size_t)s * wst), ab = saddr(act + (size_t)2 * kc * CHUNK);
-						if (!last) {
-							for (int h = 0; h < 2; h++) {  // D[row][n] of half h: A = its rows, B = the weights
-								const uint32_t a0 = ab + (uint32_t)(h * CHUNK);
+					const int KC = a.KC[l], layer_st = st;
+					const uint32_t idesc = idesc_bf16(2 * HALF, a.N[l]);
+					for (int h = 0; h < 2 && ok; h++) {
+						if (!(ok = wait_warp(act_ready + h, step & 1u))) break;
+						st = layer_st;
+						uint64_t ad = act_d + (uint32_t)(h * (CHUNK >> 4));
+						for (int kc = 0; kc < KC; kc++, ad += 2 * (CHUNK >> 4)) {
+							if (h == 0 && !(ok = wait_warp(w_full + st, st < layer_st ? ph ^ 1u : ph))) break;
+							fence_after();
+							issued = true;
+							const uint64_t wd = w_d + (uint32_t)st * w16;
+							if (elect_one()) {
 #pragma unroll
 								for (int k = 0; k < 4; k++)  // K = 16 per instruction: 32 bytes along the swizzled row
-									mma_bf16(tmem + (uint32_t)(h * 256), sw128_desc(a0 + 32u * k), sw128_desc(wb + 32u * k), idesc,
-									         (kc | k) != 0);
-								if (kc == a.KC[l] - 1) mma_commit(acc_full + h);
+									mma_pair(tmem + (uint32_t)(h * 256), ad + 2 * k, wd + 2 * k, idesc, (kc | k) != 0);
+								if (h == 1) commit_pair(w_empty + st);  // the stage is free once these products are done
+								if (kc == KC - 1) commit_pair(acc_full + h);
 							}
-						} else {
-							for (int mb = 0; mb < a.mb_last; mb++) {  // D[out][row]: A = 128 weight rows, B = the tile's 256 rows
-								const uint32_t w0 = wb + (uint32_t)(mb * CHUNK);
-#pragma unroll
-								for (int k = 0; k < 4; k++)
-									mma_bf16(tmem + (uint32_t)(mb * 256), sw128_desc(w0 + 32u * k), sw128_desc(ab + 32u * k), idesc,
-									         (kc | k) != 0);
-							}
-							if (kc == a.KC[l] - 1) {
-								mma_commit(acc_full);
-								mma_commit(acc_full + 1);
-							}
+							__syncwarp();
+							if (++st == STAGES) st = 0;
 						}
-						mma_commit(w_empty + s);  // the stage is free once these products are done
-						issued = true;
 					}
+					if (st <= layer_st) ph ^= 1u;  // (a layer has at most STAGES - 1 chunks)
 				}
-			if (issued) {  // nothing of this CTA's left in the tensor pipe before the TMEM is freed
-				mma_commit(fin);
-				mbar_wait(fin, 0);
+			if (issued) {  // nothing of the pair's left in the tensor pipes before the TMEM is freed
+				if (elect_one())
+					asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(saddr(fin))
+					             : "memory");
+				__syncwarp();
+				wait_warp(fin, 0);
 			}
 		}
-	} else {  // epilogue: half h, TMEM lane quarter q, row r of the half
-		const int h = (warp - 2) >> 2, q = warp & 3, r = 32 * q + lane, et = threadIdx.x - 64;
-		const uint32_t tq = tmem + ((uint32_t)(32 * q) << 16);  // this warp's lane quarter
-		const float4* sb4 = reinterpret_cast<const float4*>(sbias);
-		// tile tt: member tt % members (CTAs running side by side read different members'
-		// weights), rows (tt / members) * 256 + ...; the first 8 input columns of this
+	} else {  // epilogue: half h, TMEM lane quarter q, row r of the CTA's 128, column set `part`
+		const int h = (warp - 2) / HALF_WARPS, part = (warp - 2) / 4 % 2, q = warp & 3, r = 32 * q + lane;
+		const int et = (threadIdx.x - 64) % (32 * HALF_WARPS);  // thread of the half
+		const uint32_t acc = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(h * 256);  // this warp's lane quarter
+		const uint32_t ready = in_rank0(act_ready + h);
+		// tile tt: member tt % members (pairs running side by side read different members'
+		// weights), rows (tt / members) * TILE + ...; the first 8 input columns of this
 		// thread's row are fetched ahead into registers
 		float xp[8];
+		auto x_row = [&](int tt, bool& live) {
+			const int grow = (tt / a.members) * TILE + (2 * h + (int)rank) * HALF + r;
+			live = grow < a.rows;
+			return a.x + (tt % a.members) * a.sx + (long long)(live ? grow : 0) * a.in;
+		};
 		auto x_fetch = [&](int tt) {
-			const int grow = (tt / a.members) * TILE + h * HALF + r;
-			const bool live = grow < a.rows;
-			const float* xr = a.x + (tt % a.members) * a.sx + (long long)(live ? grow : 0) * a.in;
+			bool live;
+			const float* xr = x_row(tt, live);
 #pragma unroll
-			for (int j = 0; j < 8; j++) xp[j] = live && j < a.in ? xr[j] : 0.f;
+			for (int j = 0; j < 8; j++) xp[j] = part == 0 && live && j < a.in ? xr[j] : 0.f;
 		};
 		auto x_write = [&](int tt) {  // the input row, BF16, zero padded to the first layer's K
-			*unit_at(act, h, r, 0) = make_uint4(pack2(xp[0], xp[1]), pack2(xp[2], xp[3]), pack2(xp[4], xp[5]), pack2(xp[6], xp[7]));
-			const int grow = (tt / a.members) * TILE + h * HALF + r;
-			const bool live = grow < a.rows;
-			const float* xr = a.x + (tt % a.members) * a.sx + (long long)(live ? grow : 0) * a.in;
-			for (int col = 8; col < a.KC[0] * 64; col += 8) {
+			if (part == 0)
+				*unit_at(act, h, r, 0) = make_uint4(pack2(xp[0], xp[1]), pack2(xp[2], xp[3]), pack2(xp[4], xp[5]), pack2(xp[6], xp[7]));
+			bool live;
+			const float* xr = x_row(tt, live);
+			for (int col = part == 0 ? 16 : 8; col < a.KC[0] * 64; col += 16) {
 				float f[8];
 #pragma unroll
 				for (int j = 0; j < 8; j++) f[j] = live && col + j < a.in ? xr[col + j] : 0.f;
 				*unit_at(act, h, r, col) = make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
 			}
 			proxy_fence();  // generic-proxy writes, read next by the tensor core
-			mbar_arrive(act_ready + h);
+			__syncwarp();
+			if (lane == 0) arrive_cluster(ready);
 		};
-		// the bias of layer l of tile tt's member into shared memory (all 256 threads)
-		auto fill = [&](int tt, int l) {
-			const float* src = a.bias + (tt % a.members) * a.b_per + a.b_off[l];
-			for (int i = et; i < a.N[l]; i += 32 * EPI) sbias[i] = src[i];
-		};
-		int t = blockIdx.x;
+		int t = first;
 		if (t < total) {
 			x_fetch(t);
-			fill(t, 0);
+			x_write(t);
 		}
-		epi_sync();
-		if (t < total) x_write(t);
 		uint32_t step = 0;
-		for (; t < total && ok; t += gridDim.x) {
-			const int z = t % a.members, row0 = (t / a.members) * TILE + h * HALF, tn = t + gridDim.x;
+		for (; t < total && ok; t += pairs) {
+			const int z = t % a.members, tn = t + pairs;
+			const int row0 = (t / a.members) * TILE + (2 * h + (int)rank) * HALF + 32 * q;  // of this warp
 			for (int l = 0; l < L; l++, step++) {
 				const bool last = l + 1 == L;
+				const float* bias = a.bias + z * a.b_per + a.b_off[l];
+				const int N = a.N[l];
+				const float bv = et < N ? __ldg(bias + et) : 0.f;
 				if (last && tn < total) x_fetch(tn);  // its latency hides under the products
-				const bool mine = mbar_wait(acc_full + h, step & 1u);
-				if (mine) {
-					fence_after();
-					const int N = a.N[l];
-					uint32_t va[32], vb[32];
-					if (!last) {
-						// this half's accumulator, 32 columns at a time, the next 32 loading
-						// while these are converted
-						const uint32_t acc = tq + (uint32_t)(h * 256);
-						const int Kn = 64 * a.KC[l + 1];
-						if (N > 0) tmem_ld32_async(acc, va);
+				// the bias to shared memory while the products run; the half's threads agree here on
+				// whether the last wait ended well (none waits alone at this barrier)
+				float* sb = sbias + (2 * h + (int)(step & 1u)) * a.n_max;
+				if (et < N) sb[et] = bv;
+				__syncwarp();
+				if (!(ok = half_all(h, good))) break;
+				good = mbar_wait(acc_full + h, step & 1u);
+				__syncwarp();
+				fence_after();
+				uint32_t va[16], vb[16];
+				if (!last) {
+					// 16 columns at a time, the half's two warps of a lane quarter in turn, the next
+					// ones loading while these are converted
+					const int Kn = 64 * a.KC[l + 1];
+					if (16 * part < N) tmem_ld16_async(acc + (uint32_t)(16 * part), va);
+					for (int c0 = 16 * part; c0 < Kn; c0 += 64) {
 						tmem_wait();
-						for (int c0 = 0; c0 < Kn; c0 += 64) {
-							if (c0 + 32 < N) tmem_ld32_async(acc + (uint32_t)(c0 + 32), vb);
-							hidden_units(act, h, r, c0, N, va, sb4);
-							tmem_wait();
-							if (c0 + 64 < N) tmem_ld32_async(acc + (uint32_t)(c0 + 64), va);
-							hidden_units(act, h, r, c0 + 32, N, vb, sb4);
-							tmem_wait();
-						}
-						fence_before();
-						proxy_fence();
-						mbar_arrive(act_ready + h);
-					} else {
-						// D[output f][tile row]: this warp holds outputs 128 mb + 32 q + lane of
-						// its half's 128 rows (columns 128 h ..); one coalesced store per row
-						float* yz = a.y + z * a.sy;
-						for (int mb = 0; mb < a.mb_last; mb++) {
-							if (128 * mb + 32 * q >= a.out) continue;  // no output of this warp here
-							const int f = 128 * mb + 32 * q + lane;
-							const float bf = f < N ? sbias[f] : 0.f;
-							const bool fo = f < a.out;
-							const uint32_t acc = tq + (uint32_t)(mb * 256 + h * HALF);
-							tmem_ld32_async(acc, va);
-							tmem_wait();
-							for (int p = 0; p < 4; p += 2) {
-								tmem_ld32_async(acc + (uint32_t)(32 * (p + 1)), vb);
-#pragma unroll
-								for (int j = 0; j < 32; j++) {
-									const int gr = row0 + 32 * p + j;
-									if (fo && gr < a.rows) yz[(long long)gr * a.ldy + f] = __uint_as_float(va[j]) + bf;
-								}
-								tmem_wait();
-								if (p + 2 < 4) tmem_ld32_async(acc + (uint32_t)(32 * (p + 2)), va);
-#pragma unroll
-								for (int j = 0; j < 32; j++) {
-									const int gr = row0 + 32 * (p + 1) + j;
-									if (fo && gr < a.rows) yz[(long long)gr * a.ldy + f] = __uint_as_float(vb[j]) + bf;
-								}
-								tmem_wait();
-							}
-						}
+						if (c0 + 32 < N) tmem_ld16_async(acc + (uint32_t)(c0 + 32), vb);
+						hidden_units(act, h, r, c0, N, va, sb);
+						tmem_wait();
+						if (c0 + 64 < N) tmem_ld16_async(acc + (uint32_t)(c0 + 64), va);
+						hidden_units(act, h, r, c0 + 32, N, vb, sb);
+					}
+					fence_before();
+					proxy_fence();
+					__syncwarp();
+					if (lane == 0) arrive_cluster(ready);
+				} else {
+					// 16 outputs at a time through this warp's 2 KB of the last K chunk (free by
+					// now): a thread writes its row's, 16-byte units XORed against bank conflicts,
+					// and half a warp reads a row.  The next tile's input, handed on when the last
+					// accumulators have been read, lies below that chunk, or waits until the half is
+					// through with it
+					float* stage = reinterpret_cast<float*>(act + (size_t)(2 * (a.kc_max - 1) + h) * CHUNK + (2 * q + part) * 2048);
+					const bool early = a.kc_max > a.KC[0];
+					bool handed = false;
+					auto hand_on = [&] {
 						fence_before();
 						if (tn < total) x_write(tn);
+						handed = true;
+					};
+					float* yz = a.y + z * a.sy;
+					const int c = lane & 15;
+					auto put = [&](int c0, const uint32_t* v) {
+#pragma unroll
+						for (int u = 0; u < 4; u++)
+							*reinterpret_cast<uint4*>(stage + 16 * lane + 4 * (u ^ (lane >> 1 & 3))) =
+							    make_uint4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+						const int f = c0 + c;
+						const float b = f < N ? sb[f] : 0.f;
+						__syncwarp();
+						float* yp = yz + (long long)(row0 + (lane >> 4)) * a.ldy + f;
+#pragma unroll
+						for (int i = 0; i < 16; i++, yp += 2 * a.ldy) {
+							const int rr = 2 * i + (lane >> 4);
+							const float o = stage[16 * rr + 4 * ((c >> 2) ^ (i & 3)) + (c & 3)] + b;
+							if (f < a.out && row0 + rr < a.rows) *yp = o;
+						}
+						__syncwarp();
+					};
+					if (16 * part < a.out) tmem_ld16_async(acc + (uint32_t)(16 * part), va);
+					for (int c0 = 16 * part; c0 < a.out; c0 += 64) {
+						const int c1 = c0 + 32, c2 = c0 + 64;
+						tmem_wait();
+						if (c1 < a.out) tmem_ld16_async(acc + (uint32_t)c1, vb);
+						if (c2 >= a.out) {
+							tmem_wait();
+							if (early) hand_on();
+						}
+						put(c0, va);
+						if (c1 < a.out) {
+							tmem_wait();
+							if (c2 < a.out) tmem_ld16_async(acc + (uint32_t)c2, va);
+							put(c1, vb);
+						}
 					}
+					if (!early) half_all(h, true);
+					if (!handed) hand_on();
 				}
-				// every epilogue thread is done with this step's bias, and all agree on
-				// going on (a wait that gave up ends the loop for all 256 together)
-				ok = epi_all(mine);
-				if (!ok) break;
-				if (!last) fill(t, l + 1);
-				else if (tn < total) fill(tn, 0);
-				epi_sync();
 			}
 		}
 	}
+	ok = ok && good;
 	if (!ok) atomicOr(err, 1u);
 	fence_before();
 	__syncthreads();
+	cluster_sync();  // (neither CTA frees its TMEM or leaves while the other may still use its memory)
 	fence_after();
+	__syncwarp();
 	if (warp == 1)
-		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+		asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
 }
 
 // weights of one layer for the fused kernel: [members][N][Kp] BF16, K padded to Kp
@@ -1229,7 +1341,8 @@ struct mf_mlp {
 	long long wf_per = 0;
 	bool wf_dirty = true;  // Wb changed since Wf was packed
 	fz::Maps maps{};
-	int fz_kc = 1, fz_n = 16, fz_stages = 0;
+	int fz_kc = 1, fz_n = 16;
+	bool fz_fits = false;
 	Buf<uint32_t> dev_err; // set by a bounded wait of the tcgen05 GEMM that gave up
 	~mf_mlp() {
 		if (graph) cudaGraphExecDestroy(graph);
@@ -1321,28 +1434,23 @@ cudaError_t gemm(mf_mlp* m, const GemmArgs& g) {
 long long sH(const mf_mlp* m, int l) { return (long long)m->rows * m->pd[l]; }
 
 // The fused inference kernel takes models whose padded widths are all at most 256 (one
-// accumulator per half tile, at most four K chunks) and whose operands leave room for at
-// least two weight stages in shared memory.
+// accumulator per half tile, at most four K chunks).
 void fused_plan(mf_mlp* m) {
 	m->fz_kc = 1;
 	m->fz_n = 16;
 	bool fits = true;
 	for (int l = 0; l < m->L; l++) {
 		m->fz_kc = std::max(m->fz_kc, (m->pd[l] + 63) / 64);
-		// the output layer's weight box: 128 or 256 rows (it runs transposed, M = 128 per block)
-		m->fz_n = std::max(m->fz_n, l + 1 < m->L ? m->pd[l + 1] : (m->pd[l + 1] + 127) / 128 * 128);
+		m->fz_n = std::max(m->fz_n, m->pd[l + 1]);
 		fits = fits && m->pd[l] <= 256 && m->pd[l + 1] <= 256;
 	}
-	m->fz_stages = 0;
-	if (fits)
-		for (int st = 4; st >= 2 && !m->fz_stages; st--)
-			if (fz::smem_bytes(m->fz_kc, m->fz_n, st) <= TC_SMEM_MAX) m->fz_stages = st;
+	m->fz_fits = fits;
 }
 
-bool fused_eligible(const mf_mlp* m) { return m->tc && m->fused && m->fz_stages >= 2; }
+bool fused_eligible(const mf_mlp* m) { return m->tc && m->fused && m->fz_fits; }
 
 // (re)packs the BF16 weights for the fused kernel and encodes one tensor map per layer:
-// [members][N][Kp] with member stride wf_per, boxes of 64 K x N rows x 1 member
+// [members][N][Kp] with member stride wf_per, boxes of 64 K x N / 2 rows x 1 member
 mf_status fused_prepare(mf_mlp* m) {
 	if (!m->wf_dirty) return MF_OK;
 	if (!m->Wf.p) {
@@ -1364,8 +1472,7 @@ mf_status fused_prepare(mf_mlp* m) {
 		MCK(cudaGetLastError());
 		const cuuint64_t dW[3] = {(cuuint64_t)Kp, (cuuint64_t)N, (cuuint64_t)m->members};
 		const cuuint64_t sW[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)m->wf_per * 2};
-		const cuuint32_t box_rows = l + 1 < m->L ? (cuuint32_t)N : (cuuint32_t)((N + 127) / 128 * 128);  // zero filled past N
-		const cuuint32_t bW[3] = {64, box_rows, 1}, e1[3] = {1, 1, 1};
+		const cuuint32_t bW[3] = {64, (cuuint32_t)(N / 2), 1}, e1[3] = {1, 1, 1};  // (N: a multiple of 16)
 		if (enc(&m->maps.w[l], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, m->Wf.p + m->wf_off[l], dW, sW, bW, e1,
 		        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
 		        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
@@ -1385,10 +1492,8 @@ cudaError_t fused_forward(mf_mlp* m, const float* x, long long sx, int rows, flo
 	a.in = m->dims[0];
 	a.out = m->dims[m->L];
 	a.rows = rows;
-	a.stages = m->fz_stages;
 	a.kc_max = m->fz_kc;
 	a.n_max = m->fz_n;
-	a.mb_last = (m->pd[m->L] + 127) / 128;
 	for (int l = 0; l < m->L; l++) {
 		a.N[l] = m->pd[l + 1];
 		a.KC[l] = (m->pd[l] + 63) / 64;
@@ -1403,8 +1508,8 @@ cudaError_t fused_forward(mf_mlp* m, const float* x, long long sx, int rows, flo
 	a.ldy = ldy;
 	a.members = m->members;
 	const long long tiles = (long long)(rows + fz::TILE - 1) / fz::TILE * m->members;
-	const int G = (int)std::min<long long>(tiles, m->sm_count);
-	fz::k_mlp_fused<<<G, fz::THREADS, fz::smem_bytes(a.kc_max, a.n_max, a.stages), m->stream>>>(m->maps, a,
+	const int G = 2 * (int)std::min<long long>(tiles, std::max(1, m->sm_count / 2));  // pairs of CTAs
+	fz::k_mlp_fused<<<G, fz::THREADS, fz::smem_bytes(a.kc_max, a.n_max), m->stream>>>(m->maps, a,
 	                                                                                           m->dev_err.p);
 	m->launches++;
 	return cudaGetLastError();
