@@ -388,7 +388,7 @@ typedef struct mf_mlp_config {
 	int32_t members;                      /* ensemble size, 1..64 */
 	int32_t n_layers;                     /* weight layers, 1..MF_MLP_MAX_LAYERS */
 	int32_t dims[MF_MLP_MAX_LAYERS + 1];  /* widths, input first, each 1..MF_MLP_MAX_WIDTH */
-	int32_t max_batch;                    /* rows per pass: the training minibatch and the inference chunk */
+	int32_t max_batch;                    /* rows per pass: the training minibatch and the per-layer inference chunk */
 	int32_t device;
 	uint64_t seed;                        /* weight initialisation and minibatch sampling */
 } mf_mlp_config;
@@ -411,7 +411,8 @@ MF_API mf_status mf_mlp_set_data(mf_mlp* model, const float* x, const float* y, 
  * rows with replacement; learning rate cosine-annealed from lr0 to lr1 over the call.
  * loss_history (may be NULL) receives [steps][members] minibatch losses. */
 MF_API mf_status mf_mlp_train(mf_mlp* model, int32_t steps, float lr0, float lr1, float* loss_history);
-/* Every member's outputs y [members][n][dims[L]] for x [n][dims[0]]. */
+/* Every member's outputs y [members][n][dims[L]] for x [n][dims[0]].  Between host arrays
+ * the fused kernel works in chunks of up to 64 MB of staging, kept with the model. */
 MF_API mf_status mf_mlp_predict(mf_mlp* model, const float* x, int32_t n, float* y);
 MF_API mf_status mf_mlp_launch_count(const mf_mlp* model, uint64_t* launches);
 MF_API mf_status mf_mlp_get_stream(const mf_mlp* model, void** stream);

@@ -473,8 +473,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 // 5 members, 6-256-256-256-66: 626 us with single CTAs and both halves in step; 575 with
 // the issuer's ring divisions out and 16 epilogue warps; 510 with pairs and an elected
 // issuing lane; 422 with 16-column TMEM loads ahead of the conversions and two bias
-// copies, 403 with the half loops spelled out (the products alone: 196 us).  What is left is each half's own chain: products,
-// epilogue, handing over.
+// copies, 403 with the half loops spelled out (the products alone: 196 us).  What is
+// left is each half's own chain: products, epilogue, handing over.
 // Only the inputs (in FP32), the weights (from L2: every pair on a member reads the same
 // ones) and the outputs move through memory.  The products are the per-layer path's --
 // BF16 operands, FP32 accumulation in K order, the bias added in FP32 -- with K padded
@@ -1323,6 +1323,8 @@ struct mf_mlp {
 	Buf<bf16> dzb[2];          // BF16 [members][rows][widest]: a layer's output gradient and the one before it
 	Buf<float> loss;           // [members]
 	Buf<float> Xin, Yin;       // batches from the host: [members][rows][in], [members][rows][out]
+	Buf<float> Xst, Yst;       // fused inference from or to the host: staged rows, st_rows of them
+	int st_rows = 0;
 	Buf<float> Xd, Yd;         // training set [n][in], [n][out]
 	Buf<float> hist;
 	Buf<TrainCtl> ctl;
@@ -1883,6 +1885,30 @@ MF_API mf_status mf_mlp_train(mf_mlp* m, int32_t steps, float lr0, float lr1, fl
 	return tc_status(m);
 }
 
+// Rows of a chunk of fused inference between host arrays: as many as STAGE_BYTES of staging
+// hold (kept with the model, grown as calls ask for it), never fewer than max_batch, whose
+// buffers are there anyway and serve where the memory for more is not.  (A launch of 512
+// rows for 5 members fills 10 of 152 SMs, and each chunk's copies wait for it: 10,000 rows
+// in 20 chunks of 512 took 836 us, in one 137.)
+constexpr size_t STAGE_BYTES = 64u << 20;
+int stage_chunk(mf_mlp* m, int n) {
+	const size_t row = (size_t)(m->dims[0] + m->members * m->dims[m->L]) * 4;
+	const int want = (int)std::min<size_t>((size_t)n, STAGE_BYTES / row);
+	if (want <= m->rows) return m->rows;
+	if (want > m->st_rows) {
+		m->st_rows = 0;
+		if (m->Xst.alloc((size_t)want * m->dims[0]) != cudaSuccess ||
+		    m->Yst.alloc((size_t)want * m->members * m->dims[m->L]) != cudaSuccess) {
+			cudaGetLastError();
+			m->Xst.free();
+			m->Yst.free();
+			return m->rows;
+		}
+		m->st_rows = want;
+	}
+	return want;
+}
+
 MF_API mf_status mf_mlp_predict(mf_mlp* m, const float* x, int32_t n, float* y) {
 	if (!m || n < 0 || (n > 0 && (!x || !y))) return MF_ERR_ARG;
 	MCK(cudaSetDevice(m->device));
@@ -1894,22 +1920,25 @@ MF_API mf_status mf_mlp_predict(mf_mlp* m, const float* x, int32_t n, float* y) 
 		const bool xd = device_pointer(x), yd = device_pointer(y);
 		if (xd && yd) {  // one launch over every row, straight from x into y
 			MCK(fused_forward(m, x, 0, n, y, (long long)n * out, out));
-		} else
-			for (int r0 = 0; r0 < n; r0 += m->rows) {
-				const int b = std::min(m->rows, n - r0);
+		} else {
+			const int chunk = stage_chunk(m, n);
+			float *xst = chunk > m->rows ? m->Xst.p : m->Xin.p, *yst = chunk > m->rows ? m->Yst.p : m->Yin.p;
+			for (int r0 = 0; r0 < n; r0 += chunk) {
+				const int b = std::min(chunk, n - r0);
 				const float* xs = x + (size_t)r0 * in;
 				if (!xd) {
-					MCK(cudaMemcpyAsync(m->Xin.p, xs, (size_t)b * in * 4, cudaMemcpyDefault, s));
-					xs = m->Xin.p;
+					MCK(cudaMemcpyAsync(xst, xs, (size_t)b * in * 4, cudaMemcpyDefault, s));
+					xs = xst;
 				}
 				if (yd) {
 					MCK(fused_forward(m, xs, 0, b, y + (size_t)r0 * out, (long long)n * out, out));
 				} else {
-					MCK(fused_forward(m, xs, 0, b, m->Yin.p, (long long)m->rows * out, out));
-					MCK(cudaMemcpy2DAsync(y + (size_t)r0 * out, (size_t)n * out * 4, m->Yin.p, (size_t)m->rows * out * 4,
-					                      (size_t)b * out * 4, m->members, cudaMemcpyDefault, s));
+					MCK(fused_forward(m, xs, 0, b, yst, (long long)b * out, out));
+					MCK(cudaMemcpy2DAsync(y + (size_t)r0 * out, (size_t)n * out * 4, yst, (size_t)b * out * 4, (size_t)b * out * 4,
+					                      m->members, cudaMemcpyDefault, s));
 				}
 			}
+		}
 		MCK(cudaStreamSynchronize(s));
 		return tc_status(m);
 	}

@@ -395,7 +395,7 @@ class Mlp:
     def predict(self, x: np.ndarray) -> np.ndarray:
         """x [n, in] -> [members, n, out]."""
         x = np.ascontiguousarray(x, np.float32)
-        y = np.zeros((self.members, len(x), self.dims[-1]), np.float32)
+        y = np.empty((self.members, len(x), self.dims[-1]), np.float32)  # (every entry is written)
         self._check(self._lib.mf_mlp_predict(self._h, _fp(x), len(x), _fp(y)), "mf_mlp_predict")
         return y
 

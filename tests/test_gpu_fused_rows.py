@@ -55,3 +55,24 @@ def test_several_tiles_to_a_pair(lib, dims):
         want, _ = R.forward(params[z], dims, x[some], emulate=True)
         assert np.linalg.norm(y[z][some] - want) < 3e-3 * np.linalg.norm(want), z
         assert np.isfinite(y[z]).all() and (np.abs(y[z]).max(axis=1) > 0).all()
+
+
+@pytest.mark.parametrize("rows", [8, 17, 8170, 8171, 16343])
+def test_host_arrays_in_staged_chunks(lib, rows):
+    """Host arrays of fewer rows than max_batch, more, and of one, exactly one and several
+    staged chunks (64 MB: 8,171 rows of 5 inputs and 8 x 256 outputs) give the device
+    arrays' outputs bit for bit (rows are independent of the chunks); a smaller call after
+    a larger one reuses its staging."""
+    import torch
+    from mfree_iwf_gb300.surrogate import Mlp
+    mlp = Mlp([5, 32, 256], members=8, max_batch=16, seed=2)
+    x = np.random.default_rng(rows).uniform(-1, 1, size=(rows, 5)).astype(np.float32)
+    xd = torch.from_numpy(x).cuda()
+    yd = torch.empty((8, rows, 256), device="cuda", dtype=torch.float32)
+    fp = lambda t: ctypes.cast(t.data_ptr(), ctypes.POINTER(ctypes.c_float))
+    mlp._check(mlp._lib.mf_mlp_predict(mlp._h, fp(xd), rows, fp(yd)), "mf_mlp_predict")
+    want = yd.cpu().numpy()
+    np.testing.assert_array_equal(mlp.predict(x), want)
+    for n in (rows, rows // 2 + 1):
+        np.testing.assert_array_equal(mlp.predict(x[:n]), want[:, :n])
+    mlp.close()
