@@ -535,7 +535,20 @@ __global__ void k_weak_pack(WeakArgs a) {
 	pk[2 * j + 1] = make_float4(vx.hi, vx.lo, vy.hi, vy.lo);
 }
 
-__global__ void __launch_bounds__(256, 8) k_gp_pass32(WeakArgs a) {
+// a 32-byte record in one load (32-byte aligned)
+__device__ __forceinline__ void load8(const float4* p, float4& a, float4& b) {
+	asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+	    : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+	    : "l"(p));
+}
+
+// Bound by the L1 data pipe and the latency of the gathers behind the list entries (4.8 TB/s
+// of the lists and states; 16-bit neighbours, a sixth of the lists' bytes less, gained
+// nothing), so u and v of a neighbour come in one 32-byte load.  6 blocks: 40 registers
+// (8 blocks spill, 279 us).  3.2M Gauss points, per stage: 261 us with two 16-byte loads,
+// 247 now; also measured: two arrays 288, velocities as FP32 in an array of their own 249,
+// entries prefetched 2 to 4 ahead 340 to 524.
+__global__ void __launch_bounds__(256, 6) k_gp_pass32(WeakArgs a) {
 	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= a.n_g) return;
 	const float2* gw = (const float2*)a.g_w;  // gradient times the particle's quad weight
@@ -548,8 +561,9 @@ __global__ void __launch_bounds__(256, 8) k_gp_pass32(WeakArgs a) {
 	for (uint32_t k = 0; k < c; k++, q += 32) {
 		uint32_t j = a.g_snbr[q];
 		float2 w = gw[q];
+		float4 u, v;
+		load8(pk + 2 * j, u, v);
 		if (flags & A_DISP_W) {
-			float4 u = __ldg(pk + 2 * j);
 			float ux = (u.x - uxi.hi) + (u.y - uxi.lo), uy = (u.z - uyi.hi) + (u.w - uyi.lo);
 			Hxx += ux * w.x;
 			Hxy += ux * w.y;
@@ -557,7 +571,6 @@ __global__ void __launch_bounds__(256, 8) k_gp_pass32(WeakArgs a) {
 			Hyy += uy * w.y;
 		}
 		if (flags & A_VEL_W) {
-			float4 v = __ldg(pk + 2 * j + 1);
 			float vx = v.x + v.y, vy = v.z + v.w;
 			Fxx += vx * w.x;
 			Fxy += vx * w.y;
