@@ -1216,8 +1216,14 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 }
 
 // The Gray-Monaghan pair terms at the offset (xij, yij) = x_i - x_j, r2 its square.
-__device__ __forceinline__ void pair32_fast(uint32_t flags, const Row32& k, const Rec32& ri, const Rec32& rj, float xij,
-                                            float yij, float r2, Acc32& s) {
+struct Terms32 {
+	float ax = 0.f, ay = 0.f;                // of av
+	float dvx, dvy, qx = 0.f, qy = 0.f;      // of vx_x .. vy_y: dv times q
+	float f = 0.f;                           // of xs: dv times f
+};
+__device__ __forceinline__ Terms32 pair32_terms(uint32_t flags, const Row32& k, const Rec32& ri, const Rec32& rj, float xij,
+                                                float yij, float r2) {
+	Terms32 o;
 	// W = fac (t^3 / 4 - u^3), |grad W| = 3 fac (t^2 / 4 - u^2) / h with t = 2 - q,
 	// u = max(1 - q, 0) (t clamped at 0 beyond 2h); 3 fac is applied to the row's sums
 	const float sr = r2 > 1e-24f ? rsqrt_approx(r2) * k.h1 : 0.f;  // 1 / (r h); kernel.cpp's r > 1e-12
@@ -1228,6 +1234,8 @@ __device__ __forceinline__ void pair32_fast(uint32_t flags, const Row32& k, cons
 	const float g = (u2 - t2q) * sr;
 	const float gx = xij * g, gy = yij * g;
 	const float dvx = ff_diff(rj.vx, ri.vx), dvy = ff_diff(rj.vy, ri.vy);
+	o.dvx = dvx;
+	o.dvy = dvy;
 	const float inv_rs = rcp_approx(ri.rho + rj.rho);
 	float piij = 0.f;
 	if (flags & A_ART_VISC) {
@@ -1252,24 +1260,36 @@ __device__ __forceinline__ void pair32_fast(uint32_t flags, const Row32& k, cons
 			tyy += fab * (ri.Ryy + rj.Ryy);
 		}
 		const float mx = rj.m * gx, my = rj.m * gy;
-		s.av_x += (txx - piij) * mx + txy * my;
-		s.av_y += txy * mx + (tyy - piij) * my;
+		o.ax = __fmaf_rn(txx - piij, mx, __fmul_rn(txy, my));
+		o.ay = __fmaf_rn(txy, mx, __fmul_rn(tyy - piij, my));
 	} else if (flags & A_ART_VISC) {
 		const float mp = rj.m * piij;
-		s.av_x -= mp * gx;
-		s.av_y -= mp * gy;
+		o.ax = -mp * gx;
+		o.ay = -mp * gy;
 	}
 	if (flags & A_DERIVE_VEL) {
-		const float qx = rj.qw * gx, qy = rj.qw * gy;
-		s.vx_x += dvx * qx;
-		s.vx_y += dvx * qy;
-		s.vy_x += dvy * qx;
-		s.vy_y += dvy * qy;
+		o.qx = rj.qw * gx;
+		o.qy = rj.qw * gy;
+	}
+	if (flags & A_XSPH) o.f = w * inv_rs;
+	return o;
+}
+// ... and their sums, every rounding spelled out: the walks of a row by one thread and by
+// eight lanes (row_by_lanes) agree to the bit.
+__device__ __forceinline__ void pair32_fast(uint32_t flags, const Row32& k, const Rec32& ri, const Rec32& rj, float xij,
+                                            float yij, float r2, Acc32& s) {
+	const Terms32 o = pair32_terms(flags, k, ri, rj, xij, yij, r2);
+	s.av_x = __fadd_rn(s.av_x, o.ax);
+	s.av_y = __fadd_rn(s.av_y, o.ay);
+	if (flags & A_DERIVE_VEL) {
+		s.vx_x = __fmaf_rn(o.dvx, o.qx, s.vx_x);
+		s.vx_y = __fmaf_rn(o.dvx, o.qy, s.vx_y);
+		s.vy_x = __fmaf_rn(o.dvy, o.qx, s.vy_x);
+		s.vy_y = __fmaf_rn(o.dvy, o.qy, s.vy_y);
 	}
 	if (flags & A_XSPH) {
-		const float f = w * inv_rs;
-		s.xs_x += f * dvx;
-		s.xs_y += f * dvy;
+		s.xs_x = __fmaf_rn(o.f, o.dvx, s.xs_x);
+		s.xs_y = __fmaf_rn(o.f, o.dvy, s.xs_y);
 	}
 }
 
@@ -1360,12 +1380,25 @@ __device__ __forceinline__ void pair32_godunov(uint32_t flags, const BodyParams&
 // and lane 0 finishes the row.  L > 1 puts more rows' work in flight when the rows are
 // few (the launch would otherwise cover a handful of SMs); it changes the order of the
 // pair sums, not their terms.
-template <bool GOD, bool FULL, int L = 1>
+// ORDERED (L = 8, no Godunov actions): the lanes split the tests and the pair terms, and
+// each sums one of the eight sums over the row's pairs in their order: a thread's result,
+// to the bit.
+constexpr uint32_t ORD_CAP = 64;  // neighbours listed before they are evaluated
+struct OrdRow {
+	float term[8][8];
+	uint32_t list[ORD_CAP];
+	float pad[8];  // (the four rows of a warp 8 banks apart)
+};
+template <bool GOD, bool FULL, int L = 1, bool ORDERED = false>
 __device__ __forceinline__ void pair32_row(const ULArgs& a, const BodyParams* __restrict__ P,
                                            const Geom* __restrict__ G, DevStatus* st, uint32_t k,
-                                           uint32_t lane = 0) {
+                                           uint32_t lane = 0, OrdRow* sh = nullptr) {
 	uint32_t b = a.rec_body[k];
-	if (is_failed(a.failed, b)) return;  // a failed body stays as it was (all L lanes of the row)
+	// a failed body stays as it was (all L lanes of the row, on the first one's reading: another
+	// row may be failing the body just now)
+	bool failed = is_failed(a.failed, b);
+	if (L > 1) failed = __shfl_sync(((1u << L) - 1u) << (threadIdx.x & 31u & ~(unsigned)(L - 1)), failed, 0, L);
+	if (failed) return;
 	const float4* rec = reinterpret_cast<const float4*>(a.rec);
 	const size_t n = a.n_total;
 	const Rec32 ri = load_rec(rec, n, k, __ldg(rec + k));
@@ -1401,7 +1434,86 @@ __device__ __forceinline__ void pair32_row(const ULArgs& a, const BodyParams* __
 		yij = __fadd_rn(__fsub_rn(ri.y.hi, head.z), __fsub_rn(ri.y.lo, head.w));
 		return __fmaf_rn(yij, yij, __fmul_rn(xij, xij));
 	};
-	for (int ni = lo_i; ni < hi_i; ni++) {
+	if (ORDERED) {
+		const uint32_t shift = threadIdx.x & 24u, gmask = 0xffu << shift;
+		// this lane's sum, and which factors of a pair it adds: {ax, ay, dvx, dvy, qx, qy, f, 1}
+		const uint32_t fa = 0x66332210u >> (4 * lane) & 15u, fb = 0x32545477u >> (4 * lane) & 15u;
+		float acc = 0.f;
+		uint32_t cnt = 0;
+		auto evaluate = [&] {
+			__syncwarp(gmask);
+			for (uint32_t p0 = 0; p0 < cnt; p0 += 8) {
+				if (p0 + lane < cnt) {
+					const uint32_t kj = sh->list[p0 + lane];
+					const float4 head = __ldg(rec + kj);
+					float xij, yij;
+					const float r2 = offs(head, xij, yij);
+					const Terms32 o = pair32_terms(flags, rk, ri, load_rec(rec, n, kj, head), xij, yij, r2);
+					float4* t = reinterpret_cast<float4*>(sh->term[lane]);
+					t[0] = make_float4(o.ax, o.ay, o.dvx, o.dvy);
+					t[1] = make_float4(o.qx, o.qy, o.f, 1.f);
+				}
+				__syncwarp(gmask);
+				const uint32_t m = min(cnt - p0, 8u);
+#pragma unroll
+				for (uint32_t u = 0; u < 8; u++)
+					if (u < m) acc = __fmaf_rn(sh->term[u][fa], sh->term[u][fb], acc);
+				__syncwarp(gmask);
+			}
+			cnt = 0;
+		};
+		for (int n0 = lo_i; n0 < hi_i; n0 += 8) {
+			// a lane per stencil column, then the columns' candidates as one range
+			uint32_t j0 = 0, len = 0;
+			if (n0 + (int)lane < hi_i) {
+				const uint32_t cell = g.cell_off + (uint32_t)(n0 + (int)lane) * g.ny;
+				j0 = a.cell_start[min(cell + (uint32_t)lo_j, tot)];
+				len = a.cell_start[min(cell + (uint32_t)hi_j, tot)] - j0;
+			}
+			uint32_t end = len;
+#pragma unroll
+			for (int o = 1; o < 8; o <<= 1) {
+				const uint32_t v = __shfl_up_sync(gmask, end, o, 8);
+				if ((int)lane >= o) end += v;
+			}
+			const uint32_t base = j0 - (end - len), total = __shfl_sync(gmask, end, 7, 8);
+			uint32_t ends[7];
+#pragma unroll
+			for (int q = 0; q < 7; q++) ends[q] = __shfl_sync(gmask, end, q, 8);
+			for (uint32_t c0 = 0; c0 < total; c0 += 32) {
+				if (cnt + 32u > ORD_CAP) evaluate();
+				uint32_t kj[4];
+				bool in[4];
+#pragma unroll
+				for (int r = 0; r < 4; r++) {
+					const uint32_t cand = c0 + 8 * r + lane;
+					uint32_t col = 0;
+#pragma unroll
+					for (int q = 0; q < 7; q++) col += cand >= ends[q];
+					kj[r] = __shfl_sync(gmask, base, col, 8) + cand;
+					in[r] = cand < total && kj[r] != k;
+				}
+				float4 head[4];
+#pragma unroll
+				for (int r = 0; r < 4; r++)
+					if (in[r]) head[r] = __ldg(rec + kj[r]);
+#pragma unroll
+				for (int r = 0; r < 4; r++) {
+					float xij, yij;
+					in[r] = in[r] && !(offs(head[r], xij, yij) > reach2);
+					const uint32_t hit = __ballot_sync(gmask, in[r]) >> shift & 255u;
+					if (in[r]) sh->list[cnt + __popc(hit & ((1u << lane) - 1u))] = kj[r];
+					cnt += __popc(hit);
+				}
+			}
+		}
+		evaluate();
+		float* sums[8] = {&s.av_x, &s.av_y, &s.vx_x, &s.vx_y, &s.vy_x, &s.vy_y, &s.xs_x, &s.xs_y};
+#pragma unroll
+		for (int q = 0; q < 8; q++) *sums[q] = __shfl_sync(gmask, acc, q, 8);
+		if (lane != 0) return;
+	}
+	for (int ni = lo_i; !ORDERED && ni < hi_i; ni++) {
 		uint32_t c0 = min(g.cell_off + (uint32_t)ni * g.ny + (uint32_t)lo_j, tot);
 		uint32_t c1 = min(g.cell_off + (uint32_t)ni * g.ny + (uint32_t)hi_j, tot);
 		uint32_t j0 = a.cell_start[c0], j1 = a.cell_start[c1];
@@ -1436,7 +1548,7 @@ __device__ __forceinline__ void pair32_row(const ULArgs& a, const BodyParams* __
 			}
 		}
 	}
-	if (L > 1) {
+	if (L > 1 && !ORDERED) {
 		const unsigned gmask = ((1u << L) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(L - 1));
 		constexpr int NS = GOD ? 15 : 8;
 		float* acc[15] = {&s.vx_x, &s.vx_y, &s.vy_x, &s.vy_y, &s.av_x, &s.av_y, &s.xs_x, &s.xs_y,
@@ -1534,6 +1646,21 @@ __global__ void __launch_bounds__(256, 3) k_pair_split(ULArgs a, const BodyParam
 	const uint32_t k = t / L;
 	if (k >= a.n_total) return;  // a row's L lanes leave together (L divides the warp)
 	pair32_row<GOD, FULL, L>(a, P, G, st, k, t % L);
+}
+
+// The same walk by eight lanes a row, for few rows: a row's tests and pairs are a chain of
+// gathers, 18 us a stage with a thread a row whether there are 4,400 rows or 17,600.  As
+// long as the blocks fit the SMs at once (4 of 16 rows by their registers, 9,728 rows on 152
+// SMs) the lanes make it shorter: 4,408 rows 17.9 -> 12.0 us, 9,176 rows 18.0 -> 14.1; 9,860
+// rows would take 20.6.
+constexpr unsigned ORD_THREADS = 128;
+template <bool FULL>
+__global__ void __launch_bounds__(ORD_THREADS, 4) k_pair_ordered(ULArgs a, const BodyParams* __restrict__ P,
+                                                                 const Geom* __restrict__ G, DevStatus* st) {
+	__shared__ __align__(16) OrdRow rows[ORD_THREADS / 8];
+	const uint32_t t = blockIdx.x * ORD_THREADS + threadIdx.x, k = t / 8;
+	if (k >= a.n_total) return;  // a row's 8 lanes leave together
+	pair32_row<false, FULL, 8, true>(a, P, G, st, k, t % 8, rows + threadIdx.x / 8);
 }
 
 constexpr uint32_t PAIR_ROWS_MB4 = 1u << 19;
@@ -1687,7 +1814,10 @@ cudaError_t ul_stage(const ULArgs& args, bool mixed, cudaStream_t s) {
 		auto launch = [&](auto kernel) {
 			kernel<<<split > 1 ? grid1((uint64_t)a.n_total * split, bs) : grid, bs, 0, s>>>(a, a.params, a.geom, st);
 		};
-		if (split == 4) launch(god ? k_pair_split<true, false, 4> : full ? k_pair_split<false, true, 4> : k_pair_split<false, false, 4>);
+		if (split == 1 && !god && !a.persistent && a.n_total <= a.sm_count * (4u * ORD_THREADS / 8u))
+			(full ? k_pair_ordered<true> : k_pair_ordered<false>)<<<grid1(8ull * a.n_total, ORD_THREADS), ORD_THREADS, 0, s>>>(
+			    a, a.params, a.geom, st);
+		else if (split == 4) launch(god ? k_pair_split<true, false, 4> : full ? k_pair_split<false, true, 4> : k_pair_split<false, false, 4>);
 		else if (split == 8) launch(god ? k_pair_split<true, false, 8> : full ? k_pair_split<false, true, 8> : k_pair_split<false, false, 8>);
 		else if (god || !full) launch(god ? k_pair<true, false, 3> : k_pair<false, false, 3>);
 		// More warps pay once every SM has several rounds of blocks: 64 ring impacts (1.35M

@@ -168,3 +168,23 @@ def test_small_body_grid_with_scattered_particles(lib):
     for a, b in zip(*out):
         for f in ("x", "y", "vx", "vy", "rho", "Sxx"):
             np.testing.assert_array_equal(a[f], b[f], err_msg=f)
+
+
+@pytest.mark.parametrize("hdx", [1.0, 1.3, 2.0, 2.7, 3.5])
+@pytest.mark.parametrize("drop", ["none", "xsph", "rates"])
+def test_row_by_lanes_equals_row_by_thread(lib, hdx, drop):
+    """Few rows: eight lanes a row, whose list of neighbours fills and is worked off; a batch
+    of the same body with many rows walks a row with one thread: the same bits."""
+    import mfree_iwf_gb300 as M
+    sc = moving_rings(hdx)
+    sc.actions = [a for a in sc.actions if a not in DROP[drop]]
+    out = []
+    for copies in (1, 60):
+        sc.bodies = sc.bodies[:1] * copies
+        sim = M.from_scenario(sc, precision="mixed")
+        assert (sc.bodies[0].n * copies > 152 * 64) == (copies > 1)
+        sim.step(5)
+        out.append(sim.get_state(copies - 1))
+        sim.close()
+    for f in ("x", "y", "vx", "vy", "rho", "Sxx", "Sxy", "Syy"):
+        np.testing.assert_array_equal(out[0][f], out[1][f], err_msg=f)
