@@ -203,7 +203,7 @@ constexpr uint32_t TL_RUN_MAX_LEN = 32;
 // One weak-form stage: particles (state x, y, vx, vy) and Gauss points (state rho,
 // Sxx, Sxy, Syy in the rho/Sxx/Sxy/Syy or *_f slots of the StateSoA).
 struct WeakArgs {
-	uint32_t n_p, n_g, n_bodies, stage, flags, block;
+	uint32_t n_p, n_g, n_bodies, stage, flags, block, sm_count;
 	const BodyParams* params;
 	const uint32_t *body_of, *gp_body;
 	const double *X, *Y, *m, *qw_p, *gp_qw, *fcx, *fcy;

@@ -544,11 +544,15 @@ __device__ __forceinline__ void load8(const float4* p, float4& a, float4& b) {
 
 // Bound by the L1 data pipe and the latency of the gathers behind the list entries (4.8 TB/s
 // of the lists and states; 16-bit neighbours, a sixth of the lists' bytes less, gained
-// nothing), so u and v of a neighbour come in one 32-byte load.  6 blocks: 40 registers
-// (8 blocks spill, 279 us).  3.2M Gauss points, per stage: 261 us with two 16-byte loads,
-// 247 now; also measured: two arrays 288, velocities as FP32 in an array of their own 249,
-// entries prefetched 2 to 4 ahead 340 to 524.
-__global__ void __launch_bounds__(256, 6) k_gp_pass32(WeakArgs a) {
+// nothing), so u and v of a neighbour come in one 32-byte load, at 40 registers and so 6
+// blocks of 256 an SM (MB).  3.2M Gauss points, per stage: 261 us with two 16-byte loads and
+// 8 blocks, 247 now; also measured: one load at 8 blocks 279 (spills), two arrays 288,
+// velocities as FP32 in an array of their own 249, entries prefetched 2 to 4 ahead 340 to
+// 524.  Where 8 blocks an SM need a wave less, of one or two, they stay (gp_eight): plates
+// of 290k / 513k Gauss points 1885 / 2442 us for 5 steps with them, 1974 / 2469 with 6; at
+// 392k (two waves either way) 2290 and 2082, at 1.5M 5488 and 5388.
+template <int MB>
+__global__ void __launch_bounds__(256, MB) k_gp_pass32(WeakArgs a) {
 	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= a.n_g) return;
 	const float2* gw = (const float2*)a.g_w;  // gradient times the particle's quad weight
@@ -562,8 +566,9 @@ __global__ void __launch_bounds__(256, 6) k_gp_pass32(WeakArgs a) {
 		uint32_t j = a.g_snbr[q];
 		float2 w = gw[q];
 		float4 u, v;
-		load8(pk + 2 * j, u, v);
+		if (MB < 8) load8(pk + 2 * j, u, v);
 		if (flags & A_DISP_W) {
+			if (MB == 8) u = __ldg(pk + 2 * j);
 			float ux = (u.x - uxi.hi) + (u.y - uxi.lo), uy = (u.z - uyi.hi) + (u.w - uyi.lo);
 			Hxx += ux * w.x;
 			Hxy += ux * w.y;
@@ -571,6 +576,7 @@ __global__ void __launch_bounds__(256, 6) k_gp_pass32(WeakArgs a) {
 			Hyy += uy * w.y;
 		}
 		if (flags & A_VEL_W) {
+			if (MB == 8) v = __ldg(pk + 2 * j + 1);
 			float vx = v.x + v.y, vy = v.z + v.w;
 			Fxx += vx * w.x;
 			Fxy += vx * w.y;
@@ -737,6 +743,15 @@ cudaError_t weak_sell(uint32_t n, const uint32_t* off, const uint32_t* nbr, cons
 	return cudaGetLastError();
 }
 
+// 8 blocks of 256 threads an SM in the mixed Gauss-point pass (see there)
+static bool gp_eight(const WeakArgs& a, unsigned bs) {
+	auto waves = [&](unsigned per_sm) {
+		const unsigned slots = per_sm * 256u / bs * a.sm_count, blocks = grid1(a.n_g, bs);
+		return (blocks + slots - 1) / slots;
+	};
+	return waves(8) < waves(6) && waves(8) <= 2;
+}
+
 cudaError_t weak_stage(const WeakArgs& a, bool mixed, int part, cudaStream_t s) {
 	// 0: BCs on the stage state, 1: pack (mixed), 2: Gauss-point pass, 3: particle pass,
 	// 4: BCs on the particles after the step, 5: smoothing, 6: clocks
@@ -752,7 +767,8 @@ cudaError_t weak_stage(const WeakArgs& a, bool mixed, int part, cudaStream_t s) 
 #endif
 		break;
 	case 2:
-		if (mixed) k_gp_pass32<<<grid1(a.n_g, bs), bs, 0, s>>>(a);
+		if (mixed && gp_eight(a, bs)) k_gp_pass32<8><<<grid1(a.n_g, bs), bs, 0, s>>>(a);
+		else if (mixed) k_gp_pass32<6><<<grid1(a.n_g, bs), bs, 0, s>>>(a);
 		else k_gp_pass64<<<grid1(a.n_g, bs), bs, 0, s>>>(a);
 		break;
 	case 3:
