@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/mfree_gb300.h"
+#include "mf_launch.cuh"
 
 namespace {
 
@@ -73,7 +74,11 @@ __device__ __forceinline__ void ldsm_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2
 	             : "r"(a));
 }
 
+// The training step is a chain of small launches (a dozen of 2 to 8 us), each launched by
+// launch_after: 50 steps of 5 members 4.15 -> 3.93 ms.  (Started already when the previous
+// kernel's blocks had passed their own wait, 4.54 ms: they take its blocks' places.)
 __global__ void __launch_bounds__(256) k_gemm_nt(GemmArgs g) {
+	after_previous();
 	__shared__ __align__(128) bf16 As[2][NT_BM][NT_LD];
 	__shared__ __align__(128) bf16 Bs[2][NT_BN][NT_LD];
 	const int z = blockIdx.z;
@@ -289,6 +294,7 @@ __host__ __device__ constexpr uint32_t tmem_cols(int N) { return N <= 128 ? 256u
 __global__ void __launch_bounds__(THREADS, 1)
     k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, GemmArgs g,
               int rows_per_member, uint32_t* err) {
+	after_previous();
 	extern __shared__ uint8_t smem_raw[];
 	// gridDim.z > 1: each block takes n_slice of the N columns (rows of W past N are zero)
 	const int n0 = blockIdx.z * g.n_slice, N = gridDim.z > 1 ? g.n_slice : g.N;
@@ -1088,6 +1094,7 @@ struct Bwd {
 	int w_tiles, b_tiles;
 };
 __global__ void __launch_bounds__(THREADS) k_backward(Bwd g) {
+	after_previous();
 	extern __shared__ __align__(16) bf16 smem[];
 	const int z = blockIdx.y, nx = (g.in_p + T - 1) / T;
 	const bf16 *dz = g.dz + z * g.sDz, *H = g.H + z * g.sHin;
@@ -1148,6 +1155,7 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
 // a warp per row
 __global__ void __launch_bounds__(128) k_gather(const TrainCtl* ctl, int rows, int in, int in_p, int out, long long sH0,
                                                 long long sY, const float* X, const float* Y, bf16* H0, float* Yb) {
+	after_previous();
 	const int r = blockIdx.x * 4 + threadIdx.x / 32, z = blockIdx.y, lane = threadIdx.x % 32;
 	if (r >= rows) return;
 	const uint64_t key = ctl->seed ^ ((uint64_t)(ctl->step + 1) << 20) ^ ((uint64_t)z << 52) ^ (uint64_t)r;
@@ -1172,6 +1180,7 @@ __global__ void k_input(int members, int batch, int in, int in_p, const float* x
 // mean squared error of member z over batch x out; dZ = 2 (y_pred - y) / (batch * out)
 __global__ void k_mse(int batch, int out, int out_p, const float* yp, long long syp, const float* y, long long sy,
                       float* dz, bf16* dzb, long long sdz, float* loss) {
+	after_previous();
 	const int z = blockIdx.y;
 	float s = 0.f;
 	const float inv = 1.f / (float)(batch * out);
@@ -1207,6 +1216,7 @@ struct AdamSet {
 	bf16* wb;  // optional
 };
 __global__ void __launch_bounds__(256) k_adam(const TrainCtl* ctl, AdamSet weights, AdamSet biases, unsigned w_blocks) {
+	after_previous();
 	__shared__ float s_lr, s_c1, s_c2;
 	const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
 	const bool wts = blockIdx.x < w_blocks;
@@ -1252,6 +1262,7 @@ __global__ void __launch_bounds__(256) k_adam(const TrainCtl* ctl, AdamSet weigh
 
 // the step's losses into the history, and the counters ready for the next step
 __global__ void k_step_end(TrainCtl* ctl, float* loss, int members) {
+	after_previous();
 	const uint32_t row = ctl->step - ctl->t0;
 	for (int z = threadIdx.x; z < members; z += blockDim.x) {
 		if (ctl->hist && row < ctl->total) ctl->hist[(size_t)row * members + z] = loss[z];
@@ -1420,8 +1431,8 @@ cudaError_t gemm_tc(mf_mlp* m, GemmArgs g) {
 	        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
 		return cudaErrorInvalidValue;
 	const int G = std::max(1, std::min(row_tiles, m->sm_count / m->members));
-	tc::k_gemm_tc<<<dim3(G, m->members, slices), tc::THREADS, tc::smem_bytes(g.n_slice, g.K), m->stream>>>(
-	    tA, tW, g, m->rows, m->dev_err.p);
+	launch_after(tc::k_gemm_tc, dim3(G, m->members, slices), tc::THREADS, tc::smem_bytes(g.n_slice, g.K), m->stream,
+	                   tA, tW, g, m->rows, m->dev_err.p);
 	m->launches++;
 	return cudaGetLastError();
 }
@@ -1430,7 +1441,7 @@ cudaError_t gemm_tc(mf_mlp* m, GemmArgs g) {
 cudaError_t gemm(mf_mlp* m, const GemmArgs& g) {
 	if (tc_eligible(m, g)) return gemm_tc(m, g);
 	dim3 gnt((g.N + NT_BN - 1) / NT_BN, (g.M + NT_BM - 1) / NT_BM, m->members);
-	k_gemm_nt<<<gnt, 256, 0, m->stream>>>(g);
+	launch_after(k_gemm_nt, gnt, 256, 0, m->stream, g);
 	m->launches++;
 	return cudaGetLastError();
 }
@@ -1563,9 +1574,8 @@ cudaError_t backward_layers(mf_mlp* m, const float* y, int batch) {
 	const int L = m->L;
 	const long long sdz = (long long)m->rows * m->widest;  // member stride of dz, dzb
 	auto tiles = [](int n) { return (n + tr::T - 1) / tr::T; };
-	k_mse<<<dim3(32, m->members), 256, 0, s>>>(batch, m->dims[L], m->pd[L], m->Yp.p, sH(m, L), y,
-	                                           (long long)m->rows * m->dims[L], m->dz[L & 1].p, m->dzb[L & 1].p, sdz,
-	                                           m->loss.p);
+	launch_after(k_mse, dim3(32, m->members), 256, 0, s, batch, m->dims[L], m->pd[L], m->Yp.p, sH(m, L), y,
+	                   (long long)m->rows * m->dims[L], m->dz[L & 1].p, m->dzb[L & 1].p, sdz, m->loss.p);
 	m->launches++;
 	for (int l = L - 1; l >= 0; l--) {
 		tr::Bwd g{};
@@ -1579,7 +1589,7 @@ cudaError_t backward_layers(mf_mlp* m, const float* y, int batch) {
 		g.w_tiles = tiles(g.out_p) * tiles(g.in_p);
 		g.b_tiles = tiles(g.out_p);
 		const int x_tiles = l > 0 ? tiles(batch) * tiles(g.in_p) : 0;
-		tr::k_backward<<<dim3(g.w_tiles + g.b_tiles + x_tiles, m->members), tr::THREADS, tr::SMEM, s>>>(g);
+		launch_after(tr::k_backward, dim3(g.w_tiles + g.b_tiles + x_tiles, m->members), tr::THREADS, tr::SMEM, s, g);
 		m->launches++;
 	}
 	return cudaGetLastError();
@@ -1589,7 +1599,7 @@ cudaError_t adam_update(mf_mlp* m) {
 	const AdamSet w{m->w_per * m->members, m->W.p, m->gW.p, m->mW.p, m->vW.p, m->Wb.p};
 	const AdamSet b{m->b_per * m->members, m->Bias.p, m->gB.p, m->mB.p, m->vB.p, nullptr};
 	const unsigned wb = nblk(w.n, 1024);
-	k_adam<<<wb + nblk(b.n, 1024), 256, 0, m->stream>>>(m->ctl.p, w, b, wb);
+	launch_after(k_adam, wb + nblk(b.n, 1024), 256, 0, m->stream, m->ctl.p, w, b, wb);
 	m->launches++;
 	return cudaGetLastError();
 }
@@ -1598,15 +1608,14 @@ cudaError_t adam_update(mf_mlp* m) {
 cudaError_t train_step_launches(mf_mlp* m) {
 	cudaStream_t s = m->stream;
 	const int out = m->dims[m->L];
-	k_gather<<<dim3((m->rows + 3) / 4, m->members), 128, 0, s>>>(m->ctl.p, m->rows, m->dims[0], m->pd[0], out, sH(m, 0),
-	                                                             (long long)m->rows * out, m->Xd.p, m->Yd.p, m->H[0].p,
-	                                                             m->Yin.p);
+	launch_after(k_gather, dim3((m->rows + 3) / 4, m->members), 128, 0, s, m->ctl.p, m->rows, m->dims[0], m->pd[0],
+	                   out, sH(m, 0), (long long)m->rows * out, m->Xd.p, m->Yd.p, m->H[0].p, m->Yin.p);
 	m->launches++;
 	cudaError_t e;
 	if ((e = forward_layers(m, m->rows)) != cudaSuccess) return e;
 	if ((e = backward_layers(m, m->Yin.p, m->rows)) != cudaSuccess) return e;
 	if ((e = adam_update(m)) != cudaSuccess) return e;
-	k_step_end<<<1, 64, 0, s>>>(m->ctl.p, m->loss.p, m->members);
+	launch_after(k_step_end, 1, 64, 0, s, m->ctl.p, m->loss.p, m->members);
 	m->launches++;
 	return cudaGetLastError();
 }
