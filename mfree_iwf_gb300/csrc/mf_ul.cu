@@ -27,6 +27,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include "mf_common.cuh"
+#include "mf_launch.cuh"
 #include "mf_kernels.h"
 
 using namespace mfk;
@@ -114,6 +115,7 @@ __device__ __forceinline__ bool is_failed(const uint32_t* failed, uint32_t body)
 
 // --------------------------------------------------------------- grid build
 __global__ void k_bbox_init(uint32_t nb, unsigned long long* bb) {
+	after_previous();
 	uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
 	if (b >= nb) return;
 	bb[6 * b + 0] = ord_encode(1.7976931348623157e308);   // min x
@@ -132,6 +134,7 @@ __global__ void k_bbox(uint32_t n, const double* __restrict__ x, const double* _
                        const double* __restrict__ h, const double* __restrict__ vx, const double* __restrict__ vy,
                        const uint32_t* __restrict__ body_of, int mixed, unsigned long long* bb,
                        const uint32_t* failed) {
+	after_previous();
 	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	bool valid = i < n;
 	uint32_t b = valid ? body_of[i] : 0xffffffffu;
@@ -222,6 +225,7 @@ __device__ Geom body_geometry(const BodyParams& pr, int mixed, double bminx, dou
 // One block; bodies are processed serially in chunks for the scan.
 __global__ void k_geom(uint32_t nb, const unsigned long long* bb, const BodyParams* P, int mixed, Geom* G,
                        uint32_t* total_cells, uint32_t cell_cap, DevStatus* st, uint32_t* failed) {
+	after_previous();
 	__shared__ uint32_t s_cnt[1024];
 	__shared__ uint32_t s_base;
 	if (threadIdx.x == 0) s_base = 0;
@@ -278,6 +282,7 @@ __global__ void k_hash(uint32_t n, const double* __restrict__ x, const double* _
                        const uint32_t* __restrict__ body_of, const Geom* __restrict__ G,
                        const uint32_t* __restrict__ total_cells, uint32_t* keys, uint32_t* vals, DevStatus* st,
                        uint32_t* failed) {
+	after_previous();
 	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	const uint32_t b = body_of[i], tot = *total_cells;
@@ -385,6 +390,7 @@ __device__ __forceinline__ Geom body_box(const ULArgs& a, int mixed, uint32_t b)
 }
 
 __global__ void __launch_bounds__(1024) k_body_box(ULArgs a, int mixed, uint32_t* cells) {
+	after_previous();
 	const uint32_t b = blockIdx.x;
 	const Geom g = body_box(a, mixed, b);
 	if (threadIdx.x == 0) {
@@ -398,6 +404,7 @@ __global__ void __launch_bounds__(1024) k_body_box(ULArgs a, int mixed, uint32_t
 template <bool ONE>
 __global__ void __launch_bounds__(1024) k_body_sort(ULArgs a, int mixed, const uint32_t* cells, uint32_t hist_cap,
                                                     uint32_t cell_cap) {
+	after_previous();
 	extern __shared__ uint32_t s_dyn[];  // [hist_cap] cell counters, then 16-bit row indices
 	__shared__ unsigned long long s_red[32];
 	__shared__ uint32_t s_warp[32];
@@ -635,6 +642,7 @@ __device__ __forceinline__ void per_particle64(uint32_t flags, const BodyParams&
 #endif
 
 __global__ void k_gather64(ULArgs a, const BodyParams* __restrict__ P) {
+	after_previous();
 	uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
 	if (a.fill_cells && k <= a.n_total) fill_cells(a, k);
 	if (k >= a.n_total) return;
@@ -700,6 +708,7 @@ __device__ __forceinline__ void put_rec32(const ULArgs& a, const BodyParams& pr,
 }
 
 __global__ void k_gather32(ULArgs a, const BodyParams* __restrict__ P) {
+	after_previous();
 	uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
 	if (a.fill_cells && k <= a.n_total) fill_cells(a, k);
 	if (k >= a.n_total) return;
@@ -971,6 +980,7 @@ __device__ __forceinline__ void row_sums64(double (&v)[N], uint32_t lane) {
 template <bool GOD>
 __global__ void __launch_bounds__(P64_THREADS) k_pair64(ULArgs a, const BodyParams* __restrict__ P,
                                                         const Geom* __restrict__ G, DevStatus* st) {
+	after_previous();
 	__shared__ uint32_t s_list[P64_ROWS][P64_CAP + 1];  // (+ 1: rows start in different banks)
 	constexpr unsigned FULL = 0xffffffffu;
 	const uint32_t lane = threadIdx.x % P64_L;
@@ -1642,6 +1652,7 @@ __device__ __forceinline__ void pair32_row(const ULArgs& a, const BodyParams* __
 template <bool GOD, bool FULL, int L>
 __global__ void __launch_bounds__(256, 3) k_pair_split(ULArgs a, const BodyParams* __restrict__ P,
                                                        const Geom* __restrict__ G, DevStatus* st) {
+	after_previous();
 	const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
 	const uint32_t k = t / L;
 	if (k >= a.n_total) return;  // a row's L lanes leave together (L divides the warp)
@@ -1657,6 +1668,7 @@ constexpr unsigned ORD_THREADS = 128;
 template <bool FULL>
 __global__ void __launch_bounds__(ORD_THREADS, 4) k_pair_ordered(ULArgs a, const BodyParams* __restrict__ P,
                                                                  const Geom* __restrict__ G, DevStatus* st) {
+	after_previous();
 	__shared__ __align__(16) OrdRow rows[ORD_THREADS / 8];
 	const uint32_t t = blockIdx.x * ORD_THREADS + threadIdx.x, k = t / 8;
 	if (k >= a.n_total) return;  // a row's 8 lanes leave together
@@ -1674,6 +1686,7 @@ constexpr uint32_t PAIR_ROWS_MB4 = 1u << 19;
 template <bool GOD, bool FULL, int MB>
 __global__ void __launch_bounds__(256, MB) k_pair(ULArgs a, const BodyParams* __restrict__ P, const Geom* __restrict__ G,
                                                  DevStatus* st) {
+	after_previous();
 	if (!a.persistent) {
 		uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
 		if (k >= a.n_total) return;
@@ -1745,21 +1758,18 @@ cudaError_t build_grid(ULArgs& a, bool mixed, cudaStream_t s) {
 		const unsigned T = a.max_body > 1024u ? 1024u : 256u;
 		uint32_t* cells = reinterpret_cast<uint32_t*>(a.bbox);  // (the general kernels' bounding boxes)
 		if (a.n_bodies == 1) {
-			k_body_sort<true><<<1, T, smem, s>>>(a, mixed ? 1 : 0, cells, hist_cap, cell_cap);
+			launch_after(k_body_sort<true>, 1, T, smem, s, a, mixed ? 1 : 0, cells, hist_cap, cell_cap);
 		} else {
-			k_body_box<<<a.n_bodies, T, 0, s>>>(a, mixed ? 1 : 0, cells);
-			k_body_sort<false><<<a.n_bodies, T, smem, s>>>(a, mixed ? 1 : 0, cells, hist_cap, cell_cap);
+			launch_after(k_body_box, a.n_bodies, T, 0, s, a, mixed ? 1 : 0, cells);
+			launch_after(k_body_sort<false>, a.n_bodies, T, smem, s, a, mixed ? 1 : 0, cells, hist_cap, cell_cap);
 		}
 		return cudaGetLastError();
 	}
-	k_bbox_init<<<grid1(a.n_bodies, 128), 128, 0, s>>>(a.n_bodies, a.bbox);
+	launch_after(k_bbox_init, grid1(a.n_bodies, 128), 128, 0, s, a.n_bodies, a.bbox);
 	const mfk_host::StateSoA& sv = a.stage == 0 ? a.base : a.st;
-	k_bbox<<<grid1(a.n_total, 256), 256, 0, s>>>(a.n_total, sv.x, sv.y, a.h, sv.vx, sv.vy, a.body_of, mixed ? 1 : 0,
-	                                              a.bbox, a.failed);
-	k_geom<<<1, 1024, 0, s>>>(a.n_bodies, a.bbox, a.params, mixed ? 1 : 0, a.geom, a.total_cells,
-	                          cell_cap, st, a.failed);
-	k_hash<<<grid1(a.n_total, 256), 256, 0, s>>>(a.n_total, sv.x, sv.y, a.body_of, a.geom, a.total_cells, a.keys,
-	                                              a.perm_in, st, a.failed);
+	launch_after(k_bbox, grid1(a.n_total, 256), 256, 0, s, a.n_total, sv.x, sv.y, a.h, sv.vx, sv.vy, a.body_of, mixed ? 1 : 0, a.bbox, a.failed);
+	launch_after(k_geom, 1, 1024, 0, s, a.n_bodies, a.bbox, a.params, mixed ? 1 : 0, a.geom, a.total_cells, cell_cap, st, a.failed);
+	launch_after(k_hash, grid1(a.n_total, 256), 256, 0, s, a.n_total, sv.x, sv.y, a.body_of, a.geom, a.total_cells, a.keys, a.perm_in, st, a.failed);
 	size_t tmp = a.sort_tmp_bytes;
 	cudaError_t e = cub::DeviceRadixSort::SortPairs(a.sort_tmp, tmp, a.keys, a.keys_sorted, a.perm_in, a.perm,
 	                                                (int)a.n_total, 0, a.sort_bits, s);
@@ -1796,9 +1806,9 @@ cudaError_t ul_stage(const ULArgs& args, bool mixed, cudaStream_t s) {
 		if (e != cudaSuccess) return e;
 	}
 	if (mixed) {
-		if (!a.skip_gather) k_gather32<<<grid1((uint64_t)a.n_total + 1, 256), 256, 0, s>>>(a, a.params);
+		if (!a.skip_gather) launch_after(k_gather32, grid1((uint64_t)a.n_total + 1, 256), 256, 0, s, a, a.params);
 	} else {
-		k_gather64<<<grid1((uint64_t)a.n_total + 1, 256), 256, 0, s>>>(a, a.params);
+		launch_after(k_gather64, grid1((uint64_t)a.n_total + 1, 256), 256, 0, s, a, a.params);
 	}
 	unsigned bs = a.block ? a.block : 128;
 	unsigned grid = a.persistent ? a.grid : grid1(a.n_total, bs);
@@ -1812,11 +1822,10 @@ cudaError_t ul_stage(const ULArgs& args, bool mixed, cudaStream_t s) {
 		const bool full = !god && (a.flags & A_MONAGHAN) == A_MONAGHAN;
 		const uint32_t split = !a.persistent && (a.split == 4 || a.split == 8) ? a.split : 1u;
 		auto launch = [&](auto kernel) {
-			kernel<<<split > 1 ? grid1((uint64_t)a.n_total * split, bs) : grid, bs, 0, s>>>(a, a.params, a.geom, st);
+			launch_after(kernel, split > 1 ? grid1((uint64_t)a.n_total * split, bs) : grid, bs, 0, s, a, a.params, a.geom, st);
 		};
 		if (split == 1 && !god && !a.persistent && a.n_total <= a.sm_count * (4u * ORD_THREADS / 8u))
-			(full ? k_pair_ordered<true> : k_pair_ordered<false>)<<<grid1(8ull * a.n_total, ORD_THREADS), ORD_THREADS, 0, s>>>(
-			    a, a.params, a.geom, st);
+			launch_after(full ? k_pair_ordered<true> : k_pair_ordered<false>, grid1(8ull * a.n_total, ORD_THREADS), ORD_THREADS, 0, s, a, a.params, a.geom, st);
 		else if (split == 4) launch(god ? k_pair_split<true, false, 4> : full ? k_pair_split<false, true, 4> : k_pair_split<false, false, 4>);
 		else if (split == 8) launch(god ? k_pair_split<true, false, 8> : full ? k_pair_split<false, true, 8> : k_pair_split<false, false, 8>);
 		else if (god || !full) launch(god ? k_pair<true, false, 3> : k_pair<false, false, 3>);
@@ -1826,8 +1835,8 @@ cudaError_t ul_stage(const ULArgs& args, bool mixed, cudaStream_t s) {
 		else launch(a.n_total >= PAIR_ROWS_MB4 ? k_pair<false, true, 4> : k_pair<false, true, 3>);
 	} else {
 		const unsigned g64 = grid1(a.n_total, P64_ROWS);
-		if (god) k_pair64<true><<<g64, P64_THREADS, 0, s>>>(a, a.params, a.geom, st);
-		else k_pair64<false><<<g64, P64_THREADS, 0, s>>>(a, a.params, a.geom, st);
+		if (god) launch_after(k_pair64<true>, g64, P64_THREADS, 0, s, a, a.params, a.geom, st);
+		else launch_after(k_pair64<false>, g64, P64_THREADS, 0, s, a, a.params, a.geom, st);
 	}
 	if (a.ev_pair1) cudaEventRecord(a.ev_pair1, s);
 	return cudaGetLastError();
@@ -1857,7 +1866,7 @@ cudaError_t ul_neighbors(const ULArgs& args, uint32_t* counts, uint32_t* idx, co
 	if (pass == 0) {
 		cudaError_t e = build_grid(a, false, s);
 		if (e != cudaSuccess) return e;
-		k_gather64<<<grid1((uint64_t)a.n_total + 1, 256), 256, 0, s>>>(a, a.params);
+		launch_after(k_gather64, grid1((uint64_t)a.n_total + 1, 256), 256, 0, s, a, a.params);
 	}
 	k_neighbors<<<grid1(a.n_total, 128), 128, 0, s>>>(a, a.geom, counts, idx, offs, pass);
 	return cudaGetLastError();
