@@ -1748,6 +1748,15 @@ namespace {
 
 inline unsigned grid1(uint64_t n, unsigned bs) { return (unsigned)((n + bs - 1) / bs); }
 
+// Threads a block of the kernels with a thread a row: fewer where 256 would leave SMs without
+// a block, since an SM's rows share its narrow FP64 pipe
+// (4,408 rows, strict gather: 15.0 us on 18 SMs, 9.5 on 138).
+unsigned row_block(const ULArgs& a) {
+	unsigned bs = 256;
+	while (bs > 32 && grid1(a.n_total, bs) < a.sm_count) bs >>= 1;
+	return bs;
+}
+
 // The grid of the stage's positions; the caller's gather comes next.
 cudaError_t build_grid(ULArgs& a, bool mixed, cudaStream_t s) {
 	DevStatus* st = reinterpret_cast<DevStatus*>(a.status);
@@ -1769,7 +1778,8 @@ cudaError_t build_grid(ULArgs& a, bool mixed, cudaStream_t s) {
 	const mfk_host::StateSoA& sv = a.stage == 0 ? a.base : a.st;
 	launch_after(k_bbox, grid1(a.n_total, 256), 256, 0, s, a.n_total, sv.x, sv.y, a.h, sv.vx, sv.vy, a.body_of, mixed ? 1 : 0, a.bbox, a.failed);
 	launch_after(k_geom, 1, 1024, 0, s, a.n_bodies, a.bbox, a.params, mixed ? 1 : 0, a.geom, a.total_cells, cell_cap, st, a.failed);
-	launch_after(k_hash, grid1(a.n_total, 256), 256, 0, s, a.n_total, sv.x, sv.y, a.body_of, a.geom, a.total_cells, a.keys, a.perm_in, st, a.failed);
+	launch_after(k_hash, grid1(a.n_total, row_block(a)), row_block(a), 0, s, a.n_total, sv.x, sv.y, a.body_of, a.geom, a.total_cells,
+	             a.keys, a.perm_in, st, a.failed);
 	size_t tmp = a.sort_tmp_bytes;
 	cudaError_t e = cub::DeviceRadixSort::SortPairs(a.sort_tmp, tmp, a.keys, a.keys_sorted, a.perm_in, a.perm,
 	                                                (int)a.n_total, 0, a.sort_bits, s);
@@ -1805,10 +1815,11 @@ cudaError_t ul_stage(const ULArgs& args, bool mixed, cudaStream_t s) {
 		cudaError_t e = build_grid(a, mixed, s);
 		if (e != cudaSuccess) return e;
 	}
+	const unsigned rb = row_block(a);
 	if (mixed) {
-		if (!a.skip_gather) launch_after(k_gather32, grid1((uint64_t)a.n_total + 1, 256), 256, 0, s, a, a.params);
+		if (!a.skip_gather) launch_after(k_gather32, grid1((uint64_t)a.n_total + 1, rb), rb, 0, s, a, a.params);
 	} else {
-		launch_after(k_gather64, grid1((uint64_t)a.n_total + 1, 256), 256, 0, s, a, a.params);
+		launch_after(k_gather64, grid1((uint64_t)a.n_total + 1, rb), rb, 0, s, a, a.params);
 	}
 	unsigned bs = a.block ? a.block : 128;
 	unsigned grid = a.persistent ? a.grid : grid1(a.n_total, bs);
