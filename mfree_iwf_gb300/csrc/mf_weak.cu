@@ -421,7 +421,6 @@ __global__ void __launch_bounds__(256) k_p_pass64(WeakArgs a) {
 			fy += __shfl_xor_sync(0xffffffffu, fy, o);
 		}
 	}
-	if (!live) return;
 	const mfk_host::StateSoA& s = a.st;
 	double d = 0.;  // the rate of component `lane`
 	if (lane < 2) {
@@ -429,6 +428,9 @@ __global__ void __launch_bounds__(256) k_p_pass64(WeakArgs a) {
 	} else if (flags & A_MOMENTUM_W) {
 		d = ((lane == 2 ? a.fcx : a.fcy)[j] - (lane == 2 ? fx : fy)) * rcp64(a.m[j]);
 	}
+	// (lanes 2 and 3 now replace the stage velocity that lanes 0 and 1 have read)
+	__syncwarp();
+	if (!live) return;
 	const bool ok = p_rk64_one(a, lane == 0 ? a.base.x : lane == 1 ? a.base.y : lane == 2 ? a.base.vx : a.base.vy,
 	                           lane == 0 ? a.acc.x : lane == 1 ? a.acc.y : lane == 2 ? a.acc.vx : a.acc.vy,
 	                           lane == 0 ? a.st.x : lane == 1 ? a.st.y : lane == 2 ? a.st.vx : a.st.vy, j,
