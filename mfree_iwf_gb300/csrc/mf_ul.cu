@@ -1152,6 +1152,8 @@ __global__ void __launch_bounds__(P64_THREADS) k_pair64(ULArgs a, const BodyPara
 		}
 	}
 	if (flags & A_ADVECTION) { d[0] += ri.vx; d[1] += ri.vy; }
+	// (lanes 1 to 3 now replace the stage stress that every lane has read)
+	__syncwarp();
 	if (!live) return;
 	if (lane == 0) {
 		if (a.max_nbh && cnt >= a.max_nbh) fail_body(a.failed, st, ERR_NBH_OVERFLOW, i, b);
