@@ -1922,7 +1922,8 @@ static int stage_chunk(mf_mlp* m, int n) {
 
 // The pages of a result that is about to be copied into, made present by a write to each: a
 // copy into new host memory otherwise takes a fault of the device a page (30,000 rows x 5
-// members x 66, 40 MB: 32.4 ms, 1.8 this way).
+// members x 66, 40 MB: 32.4 ms, 1.8 this way).  Not for a result over the input: a write
+// could come before the copy that reads the input (those pages are present anyway).
 static void touch_pages(float* p, size_t bytes) {
 	const size_t page = (size_t)sysconf(_SC_PAGESIZE);
 	volatile char* c = reinterpret_cast<volatile char*>(p);
@@ -1943,6 +1944,8 @@ MF_API mf_status mf_mlp_predict(mf_mlp* m, const float* x, int32_t n, float* y) 
 			MCK(fused_forward(m, x, 0, n, y, (long long)n * out, out));
 		} else {
 			const int chunk = stage_chunk(m, n);
+			const uintptr_t xa = (uintptr_t)x, ya = (uintptr_t)y;
+			const bool apart = xa + (size_t)n * in * 4 <= ya || ya + (size_t)m->members * n * out * 4 <= xa;
 			float *xst = chunk > m->rows ? m->Xst.p : m->Xin.p, *yst = chunk > m->rows ? m->Yst.p : m->Yin.p;
 			for (int r0 = 0; r0 < n; r0 += chunk) {
 				const int b = std::min(chunk, n - r0);
@@ -1955,7 +1958,7 @@ MF_API mf_status mf_mlp_predict(mf_mlp* m, const float* x, int32_t n, float* y) 
 					MCK(fused_forward(m, xs, 0, b, y + (size_t)r0 * out, (long long)n * out, out));
 				} else {
 					MCK(fused_forward(m, xs, 0, b, yst, (long long)b * out, out));
-					for (int z = 0; z < m->members; z++)  // (while the kernel runs)
+					for (int z = 0; apart && z < m->members; z++)  // (while the kernel runs)
 						touch_pages(y + ((size_t)z * n + r0) * out, (size_t)b * out * 4);
 					MCK(cudaMemcpy2DAsync(y + (size_t)r0 * out, (size_t)n * out * 4, yst, (size_t)b * out * 4, (size_t)b * out * 4,
 					                      m->members, cudaMemcpyDefault, s));
