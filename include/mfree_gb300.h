@@ -273,7 +273,8 @@ MF_API mf_status mf_set_timing(mf_ctx* ctx, int32_t enable);
 /* kind: 0 = UL pair, 1 = TL pass A, 2 = TL pass B, 3 = contact, 4 = grid build, 5 = weak (Gauss) pass.
  * Returns the summed event time in ms, the launch count and rows processed. */
 MF_API mf_status mf_kernel_stats(mf_ctx* ctx, int32_t kind, double* total_ms, uint64_t* launches, uint64_t* rows);
-/* Number of kernel launches issued by this context since creation. */
+/* Number of launches of this library's kernels issued by this context since creation (the
+ * radix sort of the updated-Lagrangian grid, CUB's, not among them). */
 MF_API mf_status mf_launch_count(mf_ctx* ctx, uint64_t* launches);
 /* Autotuner: times the candidate launch shapes of the hot kernels (rows per block,
  * plain or persistent pair kernel, rows per work chunk) for trial_steps steps each on

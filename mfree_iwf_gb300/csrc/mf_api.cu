@@ -743,9 +743,7 @@ mf_status ul_step(mf_ctx* c) {
 		timing_count(c, slot_pair, c->n_total);
 		timing_end(c, slot_all, c->n_total);
 		if (e != cudaSuccess) return cuda_fail(c, e, "ul_stage");
-		const bool small = c->strict ? mf_strict::ul_small_grid(a) : mf_fast::ul_small_grid(a);
-		const uint32_t grid = !(a.strict_grid || s == 0) ? 0 : !small ? 9 : a.n_bodies == 1 ? 1 : 2;
-		c->launches += grid + (a.skip_gather ? 1 : 2);
+		c->launches += c->strict ? mf_strict::ul_stage_launches(a) : mf_fast::ul_stage_launches(a);
 	}
 	if (c->n_bc) {  // rk4.h:105: the conditions act on the particles after the combine
 		cudaError_t e = c->strict ? mf_strict::ul_bc(c->n_bc, c->bc_rows.p, c->bc_v.p, c->sd[0][2].p, c->sd[0][3].p, c->stream)
@@ -2146,7 +2144,7 @@ mf_status uw_step(mf_ctx* c) {
 		timing_begin(c, 2, slot);
 		if ((e = launch(a, 1)) != cudaSuccess) return cuda_fail(c, e, "weak UL particle pass");
 		timing_end(c, slot, c->n_total);
-		c->launches += 4;
+		c->launches += c->uw_order ? 2 : 4;  // (two neighbourhoods before the passes, or the one launch counted above)
 	}
 	if (c->n_bc) {  // rk4.h:196
 		e = c->strict ? mf_strict::ul_bc(c->n_bc, c->bc_rows.p, c->bc_v.p, c->sd[0][2].p, c->sd[0][3].p, c->stream)
@@ -2267,7 +2265,7 @@ mf_status contact_run(mf_ctx* c, cudaStream_t s) {
 	cudaError_t e = c->strict ? mf_strict::contact_step(a, s) : mf_fast::contact_step(a, s);
 	timing_end(c, slot, c->n_slave);
 	if (e != cudaSuccess) return cuda_fail(c, e, "contact");
-	c->launches += 3;
+	c->launches += 2;
 	return MF_OK;
 }
 

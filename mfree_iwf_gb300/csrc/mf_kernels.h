@@ -284,7 +284,7 @@ struct ContactArgs {
 #define MF_DECLARE_LAUNCHERS(NS)                                                                              \
 	namespace NS {                                                                                           \
 	size_t ul_sort_tmp_bytes(uint32_t n, int bits);                                                          \
-	bool ul_small_grid(const mfk_host::ULArgs& a);                                                            \
+	uint32_t ul_stage_launches(const mfk_host::ULArgs& a);                                                    \
 	size_t ul_rec_bytes(bool mixed);                                                                         \
 	cudaError_t ul_stage(const mfk_host::ULArgs& a, bool mixed, cudaStream_t s);                             \
 	cudaError_t ul_bc(uint32_t n_bc, const uint32_t* rows, const double* v, double* vx, double* vy, cudaStream_t s); \

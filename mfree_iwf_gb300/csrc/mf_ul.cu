@@ -1744,10 +1744,6 @@ __global__ void k_neighbors(ULArgs a, const Geom* __restrict__ G, uint32_t* coun
 	if (pass == 0) counts[i] = cnt;
 }
 
-}  // namespace
-bool ul_small_grid(const ULArgs& a);
-namespace {
-
 inline unsigned grid1(uint64_t n, unsigned bs) { return (unsigned)((n + bs - 1) / bs); }
 
 // Threads a block of the kernels with a thread a row: fewer where 256 would leave SMs without
@@ -1757,6 +1753,14 @@ unsigned row_block(const ULArgs& a) {
 	unsigned bs = 256;
 	while (bs > 32 && grid1(a.n_total, bs) < a.sm_count) bs >>= 1;
 	return bs;
+}
+
+// One block's FP64 divisions for the cell keys hold its SM's narrow pipe for 7.5 ns a row:
+// up to 1024 rows that is a fraction of the launches saved; a single body of 4,408 rows
+// takes 45 us this way and 26 with the general kernels, unless every SM has such a body.
+bool ul_small_grid(const ULArgs& a) {
+	const uint32_t limit = a.n_bodies >= a.sm_count && a.sm_count ? GRID_BODY_MAX : 1024u;
+	return a.max_body && a.max_body <= limit && a.n_bodies <= GRID_MAX_BODIES && !a.failed;
 }
 
 // The grid of the stage's positions; the caller's gather comes next.
@@ -1799,12 +1803,12 @@ size_t ul_sort_tmp_bytes(uint32_t n, int bits) {
 	return bytes;
 }
 
-// One block's FP64 divisions for the cell keys hold its SM's narrow pipe for 7.5 ns a row:
-// up to 1024 rows that is a fraction of the launches saved; a single body of 4,408 rows
-// takes 45 us this way and 26 with the general kernels, unless every SM has such a body.
-bool ul_small_grid(const ULArgs& a) {
-	const uint32_t limit = a.n_bodies >= a.sm_count && a.sm_count ? GRID_BODY_MAX : 1024u;
-	return a.max_body && a.max_body <= limit && a.n_bodies <= GRID_MAX_BODIES && !a.failed;
+// Kernels of this file that ul_stage launches: the grid's (CUB's sort not counted), the
+// gather, the pair pass.
+uint32_t ul_stage_launches(const ULArgs& a) {
+	if (a.n_total == 0) return 0;
+	const bool grid = a.strict_grid || a.stage == 0;
+	return (!grid ? 0u : !ul_small_grid(a) ? 4u : a.n_bodies == 1 ? 1u : 2u) + (a.skip_gather ? 1u : 2u);
 }
 
 size_t ul_rec_bytes(bool mixed) { return mixed ? sizeof(Rec32) : sizeof(Rec64); }
