@@ -595,9 +595,20 @@ __device__ __forceinline__ void per_particle32(uint32_t flags, const BodyParams&
 	if (flags & A_ART_STRESS) {
 		// principal stresses from the stress circle; cos 2 theta and sin 2 theta (halved) as
 		// its components over its radius, in place of atan2f, cosf and sinf of the angle
-		const float dev = sxx - syy, twice = 2.f * sxy, mean = 0.5f * (sxx + syy);
+		float dev = sxx - syy, twice = 2.f * sxy;
+		const float mean = 0.5f * (sxx + syy);
+		// (an exponent whose square could leave the range: scaled by a power of two)
+		const uint32_t e = max(__float_as_uint(fabsf(dev)), __float_as_uint(fabsf(twice))) >> 23;
+		const uint32_t k = min(max(e, 1u), 253u);
+		const bool scaled = e - 80u > 94u;
+		if (scaled) {
+			dev *= __uint_as_float((254u - k) << 23);
+			twice *= __uint_as_float((254u - k) << 23);
+		}
 		const float R2 = dev * dev + twice * twice;
-		const float R1 = R2 > 1e-30f ? rsqrtf(R2) : 0.f, radius = 0.5f * R2 * R1;
+		const float R1 = R2 > 1e-30f ? rsqrtf(R2) : 0.f;
+		float radius = 0.5f * R2 * R1;
+		if (scaled) radius *= __uint_as_float(k << 23);
 		const float c2 = R2 > 1e-30f ? 0.5f * dev * R1 : 0.5f, s2 = 0.5f * twice * R1;
 		const float eps = -pr.fmghn_eps / (rho * rho);
 		const float ra = eps * fmaxf(mean + radius, 0.f), rb = eps * fmaxf(mean - radius, 0.f);
@@ -628,9 +639,20 @@ __device__ __forceinline__ void per_particle64(uint32_t flags, const BodyParams&
 	r.c = sqrt(pr.K * rho1);
 	r.Rxx = r.Rxy = r.Ryy = 0.;
 	if (flags & A_ART_STRESS) {
-		const double dev = r.sxx - r.syy, twice = 2. * Sxy, mean = 0.5 * (r.sxx + r.syy);
+		double dev = r.sxx - r.syy, twice = 2. * Sxy;
+		const double mean = 0.5 * (r.sxx + r.syy);
+		// (an exponent whose square could leave the range: scaled by a power of two)
+		const uint32_t e = (uint32_t)max(__double2hiint(fabs(dev)), __double2hiint(fabs(twice))) >> 20;
+		const uint32_t k = min(max(e, 1u), 2045u);
+		const bool scaled = e - 600u > 800u;
+		if (scaled) {
+			dev *= __hiloint2double((int)((2046u - k) << 20), 0);
+			twice *= __hiloint2double((int)((2046u - k) << 20), 0);
+		}
 		const double R2 = fma(dev, dev, twice * twice);
-		const double R1 = R2 > 0. ? rsqrt64(R2) : 0., radius = 0.5 * R2 * R1;
+		const double R1 = R2 > 0. ? rsqrt64(R2) : 0.;
+		double radius = 0.5 * R2 * R1;
+		if (scaled) radius *= __hiloint2double((int)(k << 20), 0);
 		const double c2 = R2 > 0. ? 0.5 * dev * R1 : 0.5, s2 = 0.5 * twice * R1;  // halves of cos, sin 2 theta
 		const double eps = -pr.mghn_eps * r.rho21;
 		const double ra = eps * clamp0(mean + radius), rb = eps * clamp0(mean - radius);
