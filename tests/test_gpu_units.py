@@ -1,6 +1,6 @@
-"""The updated-Lagrangian step in mass units apart by a power of two: densities, masses, moduli
-and stresses scale exactly, positions and velocities do not change.  Stresses whose squares
-overflow or underflow the format are part of the range."""
+"""Steps in mass units apart by a power of two: densities, masses, moduli and stresses scale
+exactly, positions and velocities do not change.  Stresses whose squares overflow or underflow
+the format, and densities whose cubes do, are part of the range."""
 import numpy as np
 import pytest
 
@@ -9,9 +9,9 @@ from mfree_iwf_gb300 import scenarios as S
 pytestmark = pytest.mark.gpu
 
 
-def moved(precision, k, stress, speed):
+def moved(precision, k, stress, speed, method=S.METHOD_UL):
     import mfree_iwf_gb300 as M
-    sc = S.c1_rings(dx=4e-3)
+    sc = S.c1_rings(dx=4e-3, method=method)
     a, u = sc.bodies[0].arrays, 2.0 ** k
     a["vx"] = speed * np.sin(200.0 * a["y"])
     a["vy"] = speed * np.cos(150.0 * a["x"])
@@ -39,3 +39,11 @@ def test_mass_units(lib, precision, k, stress, speed, tol):
     want, got = moved(precision, 0, stress, speed), moved(precision, k, stress, speed)
     for f in want:
         assert np.linalg.norm(got[f] - want[f]) <= tol * np.linalg.norm(want[f]), f
+
+
+# the run-walk passes of the mixed form, with viscosity
+@pytest.mark.parametrize("k", [50, -60])
+def test_mass_units_total_lagrangian(lib, k):
+    want, got = (moved("mixed", q, 1e4, 2.0, S.METHOD_TL) for q in (0, k))
+    for f in want:
+        np.testing.assert_array_equal(got[f], want[f], err_msg=f)
