@@ -1059,6 +1059,7 @@ __global__ void __launch_bounds__(P64_THREADS) k_pair64(ULArgs a, const BodyPara
 		}
 	};
 	uint32_t cnt = 0, listed = 0;
+	bool alone = true;
 	const int cols = __reduce_max_sync(FULL, hi_i - lo_i);
 	for (int c = 0; c < cols; c++) {
 		uint32_t j0 = 0, j1 = 0;
@@ -1102,10 +1103,19 @@ __global__ void __launch_bounds__(P64_THREADS) k_pair64(ULArgs a, const BodyPara
 			if (__any_sync(FULL, full)) {  // a full row works its list off now (the others go on listing)
 				__syncwarp();
 				pairs(full ? listed : 0u);
-				if (full) listed = 0u;
+				if (full) {
+					listed = 0u;
+					alone = false;
+				}
 				__syncwarp();
 			}
 		}
+	}
+	// a row without neighbours takes itself: zero terms, unless its stress is not finite or its
+	// h zero, which then shows in the sums as it does through any neighbour
+	if (!GOD && live && alone && listed == 0u) {
+		if (lane == 0) list[0] = k;
+		listed = 1u;
 	}
 	__syncwarp();
 	pairs(listed);
@@ -1595,6 +1605,10 @@ __device__ __forceinline__ void pair32_row(const ULArgs& a, const BodyParams* __
 	}
 	float d[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 	const float rhoi = ri.rho;
+	if (!GOD && rk.stress) {  // (a stress that is not finite shows in a row without neighbours too)
+		s.av_x = __fmaf_rn(ri.sxx, 0.f, __fmaf_rn(ri.sxy, 0.f, s.av_x));
+		s.av_y = __fmaf_rn(ri.syy, 0.f, s.av_y);
+	}
 	if (!GOD) {  // the factors that pair32_fast left out
 		const float gsc = 3.f * rk.fac, xsc = 2.f * pr.fxsph_eps * ri.m * rk.fac;
 		s.av_x *= gsc; s.av_y *= gsc;
