@@ -174,6 +174,8 @@ MF_DEV double rsqrt64(double d) {
 	const double e = fma(-d * y, y, 1.);
 	return fma(y * e, fma(0.375, e, 0.5), y);
 }
+// v > 0 by its bits (no FP64 compare; subnormals below 2^-1042 count as zero, NaN is not above it)
+MF_DEV bool above0(double v) { return (uint32_t)__double2hiint(v) - 1u < 0x7ff00000u; }
 // max(v, 0) by the sign bit (no FP64 compare); NaN stays NaN or becomes 0 by its sign
 MF_DEV double clamp0(double v) { return __double2hiint(v) < 0 ? 0. : v; }
 

@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(256) k_tlB64(TLArgs a) {
 			const double dvx = s.vx[j] - vxi, dvy = s.vy[j] - vyi;
 			const double xij = xi - s.x[j], yij = yi - s.y[j];
 			const double dot = fma(dvy, yij, dvx * xij);  // -v_ij . x_ij
-			if (__double2hiint(dot) > 0) {  // approaching (dot > 0 by its bits)
+			if (above0(dot)) {              // approaching
 				// with n = 2 h_ij dot, D = r^2 + eta^2 h_ij^2, rs = rho_i + rho_j and
 				// A = 1 / (D rs): Pi = n A (alpha c_ij + beta / 2 n A rs)
 				const double hs = hi + a.h[j], rs = rhoi + s.rho[j];

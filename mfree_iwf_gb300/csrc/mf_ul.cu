@@ -931,7 +931,7 @@ __device__ __forceinline__ void pair64_fast(uint32_t flags, const Row64& k, doub
 	double piij = 0.;
 	if (flags & A_ART_VISC) {
 		const double dot = fma(dvy, yij, dvx * xij);  // -v_ij . x_ij
-		const bool approach = __double2hiint(dot) > 0;  // dot > 0 by its bits
+		const bool approach = above0(dot);
 		const double hs = ri.h + rj.h;
 		const double D = approach ? fma(k.eta2q * hs, hs, r2) : 1.;
 		const double mu2 = hs * dot * rcp64(D);  // -2 mu_ij
