@@ -413,7 +413,7 @@ MF_API mf_status mf_mlp_set_data(mf_mlp* model, const float* x, const float* y, 
  * loss_history (may be NULL) receives [steps][members] minibatch losses. */
 MF_API mf_status mf_mlp_train(mf_mlp* model, int32_t steps, float lr0, float lr1, float* loss_history);
 /* Every member's outputs y [members][n][dims[L]] for x [n][dims[0]].  Between host arrays
- * the fused kernel works in chunks of up to 64 MB of staging, kept with the model. */
+ * it works in chunks of up to 64 MB of staging, kept with the model. */
 MF_API mf_status mf_mlp_predict(mf_mlp* model, const float* x, int32_t n, float* y);
 MF_API mf_status mf_mlp_launch_count(const mf_mlp* model, uint64_t* launches);
 MF_API mf_status mf_mlp_get_stream(const mf_mlp* model, void** stream);

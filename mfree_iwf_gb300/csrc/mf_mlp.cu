@@ -1336,7 +1336,7 @@ struct mf_mlp {
 	Buf<bf16> dzb[2];          // BF16 [members][rows][widest]: a layer's output gradient and the one before it
 	Buf<float> loss;           // [members]
 	Buf<float> Xin, Yin;       // batches from the host: [members][rows][in], [members][rows][out]
-	Buf<float> Xst, Yst;       // fused inference from or to the host: staged rows, st_rows of them
+	Buf<float> Xst, Yst;       // inference from or to the host: staged rows, st_rows of them
 	int st_rows = 0;
 	Buf<float> Xd, Yd;         // training set [n][in], [n][out]
 	Buf<float> hist;
@@ -1539,11 +1539,12 @@ bool device_pointer(const void* p) {
 	return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
-// forward pass of all members over `batch` rows already in H[0]
-// direct_out: when the last layer runs on tcgen05, write its unpadded outputs straight
-// into Yin ([members][rows][out], FP32) and set *wrote_direct (no unpadding pass then)
-cudaError_t forward_layers(mf_mlp* m, int batch, bool direct_out = false, bool* wrote_direct = nullptr) {
-	if (wrote_direct) *wrote_direct = false;
+// forward pass of all members over `batch` rows already in H[0], the padded outputs into Yp;
+// with y: the unpadded ones into y[z * sy + r * out + c] instead, by the last layer itself
+// where it runs on tcgen05
+cudaError_t forward_layers(mf_mlp* m, int batch, float* y = nullptr, long long sy = 0) {
+	const int out = m->dims[m->L];
+	bool direct = false;
 	for (int l = 0; l < m->L; l++) {
 		GemmArgs g{};
 		g.M = batch; g.N = m->pd[l + 1]; g.K = m->pd[l];
@@ -1555,16 +1556,21 @@ cudaError_t forward_layers(mf_mlp* m, int batch, bool direct_out = false, bool* 
 			g.relu = 1;
 		} else {
 			g.C = m->Yp.p; g.ldc = m->pd[l + 1]; g.sC = sH(m, l + 1);
-			if (direct_out && tc_eligible(m, g)) {
-				g.C = m->Yin.p; g.ldc = m->dims[m->L]; g.sC = (long long)m->rows * m->dims[m->L];
-				g.n_store = m->dims[m->L];
-				if (wrote_direct) *wrote_direct = true;
+			if (y && tc_eligible(m, g)) {
+				g.C = y; g.ldc = out; g.sC = sy;
+				g.n_store = out;
+				direct = true;
 			}
 		}
 		cudaError_t e = gemm(m, g);
 		if (e != cudaSuccess) return e;
 	}
-	return cudaSuccess;
+	if (y && !direct) {
+		const long long per = (long long)batch * out;
+		k_output<<<nblk(per * m->members, 256), 256, 0, m->stream>>>(m->members, batch, out, m->pd[m->L], m->Yp.p, sH(m, m->L), y, sy);
+		m->launches++;
+	}
+	return cudaGetLastError();
 }
 
 // gradients of the mean squared error against y (FP32 [members][rows][out]) into gW,
@@ -1896,7 +1902,7 @@ MF_API mf_status mf_mlp_train(mf_mlp* m, int32_t steps, float lr0, float lr1, fl
 	return tc_status(m);
 }
 
-// Rows of a chunk of fused inference between host arrays: as many as STAGE_BYTES of staging
+// Rows of a chunk of inference between host arrays: as many as STAGE_BYTES of staging
 // hold (kept with the model, grown as calls ask for it), never fewer than max_batch, whose
 // buffers are there anyway and serve where the memory for more is not.  (A launch of 512
 // rows for 5 members fills 10 of 152 SMs, and each chunk's copies wait for it: 10,000 rows
@@ -1920,15 +1926,35 @@ static int stage_chunk(mf_mlp* m, int n) {
 	return want;
 }
 
-// The pages of a result that is about to be copied into, made present by a write to each: a
-// copy into new host memory otherwise takes a fault of the device a page (30,000 rows x 5
-// members x 66, 40 MB: 32.4 ms, 1.8 this way).  Not for a result over the input: a write
-// could come before the copy that reads the input (those pages are present anyway).
-static void touch_pages(float* p, size_t bytes) {
+// Makes the pages of host memory that is about to be copied into present by a write to each.
+static void touch_pages(char* p, size_t bytes) {
 	const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-	volatile char* c = reinterpret_cast<volatile char*>(p);
+	volatile char* c = p;
 	for (size_t o = 0; o < bytes; o += page) c[o] = 0;
 	if (bytes) c[bytes - 1] = 0;
+}
+
+// Rows r0 .. r0 + b of every member's result, src [members][b][out] on the device, into the
+// host's y [members][n][out].  The pages are made present first, while the kernels run: a copy
+// into new host memory otherwise takes a fault of the device a page (30,000 rows x 5 members
+// x 66, 40 MB: 32.4 ms, 1.8 this way).  Not for a result over the input: a write could come
+// before the copy that reads the input (those pages are present anyway).  Several chunks: a
+// strided copy into pageable memory reaches a whole pitch behind its last row's start, from
+// the second chunk on past the end of y, which may be nobody's memory; the last member's rows
+// go in a copy of their own.
+static cudaError_t result_to_host(mf_mlp* m, const float* x, int n, float* y, int r0, int b, const float* src) {
+	const size_t row = (size_t)m->dims[m->L] * 4, part = b * row, pitch = n * row;
+	char* dst = reinterpret_cast<char*>(y) + r0 * row;
+	const uintptr_t xa = (uintptr_t)x, ya = (uintptr_t)y;
+	if (xa + (size_t)n * m->dims[0] * 4 <= ya || ya + m->members * pitch <= xa)
+		for (int z = 0; z < m->members; z++) touch_pages(dst + z * pitch, part);
+	const char* from = reinterpret_cast<const char*>(src);
+	if (b == n) return cudaMemcpyAsync(dst, from, m->members * part, cudaMemcpyDefault, m->stream);
+	const int strided = m->members - 1;
+	cudaError_t e = cudaSuccess;
+	if (strided) e = cudaMemcpy2DAsync(dst, pitch, from, part, part, strided, cudaMemcpyDefault, m->stream);
+	if (e != cudaSuccess) return e;
+	return cudaMemcpyAsync(dst + strided * pitch, from + strided * part, part, cudaMemcpyDefault, m->stream);
 }
 
 MF_API mf_status mf_mlp_predict(mf_mlp* m, const float* x, int32_t n, float* y) {
@@ -1944,8 +1970,6 @@ MF_API mf_status mf_mlp_predict(mf_mlp* m, const float* x, int32_t n, float* y) 
 			MCK(fused_forward(m, x, 0, n, y, (long long)n * out, out));
 		} else {
 			const int chunk = stage_chunk(m, n);
-			const uintptr_t xa = (uintptr_t)x, ya = (uintptr_t)y;
-			const bool apart = xa + (size_t)n * in * 4 <= ya || ya + (size_t)m->members * n * out * 4 <= xa;
 			float *xst = chunk > m->rows ? m->Xst.p : m->Xin.p, *yst = chunk > m->rows ? m->Yst.p : m->Yin.p;
 			for (int r0 = 0; r0 < n; r0 += chunk) {
 				const int b = std::min(chunk, n - r0);
@@ -1958,36 +1982,29 @@ MF_API mf_status mf_mlp_predict(mf_mlp* m, const float* x, int32_t n, float* y) 
 					MCK(fused_forward(m, xs, 0, b, y + (size_t)r0 * out, (long long)n * out, out));
 				} else {
 					MCK(fused_forward(m, xs, 0, b, yst, (long long)b * out, out));
-					for (int z = 0; apart && z < m->members; z++)  // (while the kernel runs)
-						touch_pages(y + ((size_t)z * n + r0) * out, (size_t)b * out * 4);
-					MCK(cudaMemcpy2DAsync(y + (size_t)r0 * out, (size_t)n * out * 4, yst, (size_t)b * out * 4, (size_t)b * out * 4,
-					                      m->members, cudaMemcpyDefault, s));
+					MCK(result_to_host(m, x, n, y, r0, b, yst));
 				}
 			}
 		}
 		MCK(cudaStreamSynchronize(s));
 		return tc_status(m);
 	}
-	for (int r0 = 0; r0 < n; r0 += m->rows) {
-		const int b = std::min(m->rows, n - r0);
-		MCK(cudaMemcpyAsync(m->Xin.p, x + (size_t)r0 * in, (size_t)b * in * 4, cudaMemcpyDefault, s));
-		const long long per = (long long)b * m->pd[0];
-		k_input<<<nblk(per * m->members, 256), 256, 0, s>>>(m->members, b, in, m->pd[0], m->Xin.p, 0, m->H[0].p, sH(m, 0));
-		m->launches++;
-		MCK(cudaGetLastError());
-		bool direct = false;
-		MCK(forward_layers(m, b, true, &direct));
-		// unpadded outputs into Yin ([members][rows][out]) -- written there by the last
-		// layer itself on the tcgen05 path -- then one 2D copy per chunk
-		if (!direct) {
-			const long long po = (long long)b * out;
-			k_output<<<nblk(po * m->members, 256), 256, 0, s>>>(m->members, b, out, m->pd[m->L], m->Yp.p, sH(m, m->L),
-			                                                   m->Yin.p, (long long)m->rows * out);
+	// the layers' own path: passes of max_batch rows, each straight into y or into the staging
+	const bool yd = n > 0 && device_pointer(y);
+	const int chunk = yd || n == 0 ? n : stage_chunk(m, n);
+	for (int r0 = 0; r0 < n; r0 += chunk) {
+		const int b = std::min(chunk, n - r0);
+		float* yo = yd ? y : chunk > m->rows ? m->Yst.p : m->Yin.p;
+		for (int q0 = 0; q0 < b; q0 += m->rows) {
+			const int c = std::min(m->rows, b - q0);
+			MCK(cudaMemcpyAsync(m->Xin.p, x + (size_t)(r0 + q0) * in, (size_t)c * in * 4, cudaMemcpyDefault, s));
+			const long long per = (long long)c * m->pd[0];
+			k_input<<<nblk(per * m->members, 256), 256, 0, s>>>(m->members, c, in, m->pd[0], m->Xin.p, 0, m->H[0].p, sH(m, 0));
 			m->launches++;
 			MCK(cudaGetLastError());
+			MCK(forward_layers(m, c, yo + (size_t)q0 * out, (long long)b * out));
 		}
-		MCK(cudaMemcpy2DAsync(y + (size_t)r0 * out, (size_t)n * out * 4, m->Yin.p, (size_t)m->rows * out * 4,
-		                      (size_t)b * out * 4, m->members, cudaMemcpyDefault, s));
+		if (!yd) MCK(result_to_host(m, x, n, y, r0, b, yo));
 	}
 	MCK(cudaStreamSynchronize(s));
 	return tc_status(m);
