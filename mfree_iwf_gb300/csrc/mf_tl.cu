@@ -883,16 +883,18 @@ __device__ __forceinline__ PairB tlB_load(const TLArgs& a, uint32_t flags, uint3
 	return p;
 }
 
-// Pass B's sums: of m_j / rho0 (P_i + P_j - rho0^2 Pi_ij I) grad w_ij, with the row's own P_i
-// by the sum of the gradients.  The stress forces and the viscosity share them, rho0^2 being
-// the common scale of the momentum equation's stress term (1 / rho0 at the end, so that no
-// intermediate holds more than one power of the density).
+// Pass B's sums: of m_j (P_i + P_j - rho0^2 Pi_ij I) grad w_ij, with the row's own P_i by
+// the sum of the gradients.  The stress forces and the viscosity share them, rho0^2 being
+// the common scale of the momentum equation's stress term (1 / rho0^2 at the end).
+// Densities are divided by s, the power of two below rho0, so that no intermediate holds more
+// than one power of the density (exact: the same bits in any mass unit).
 struct AccB {
 	float ax = 0.f, ay = 0.f, wx = 0.f, wy = 0.f;
 };
-// Per-row constants: 1/h; eta^2 / 4, beta / 2, alpha rho0 / 2, rho0; 3 fac invB / (C rho0)
+// Per-row constants: 1/h; eta^2 / 4, beta rho0^2 / 2s, alpha rho0^2 / 2s; 1/s, rho_i / s;
+// 3 fac invB / (C s)
 struct RowB {
-	float h1, eta2q, half_beta, half_alpha, rho0;
+	float h1, eta2q, half_beta, half_alpha, s1, rho;
 	float4 G;
 };
 __device__ __forceinline__ void tlB_add(uint32_t flags, const PairB& p, const RecB& ri, float4 Xi, const RowB& k, AccB& s) {
@@ -904,11 +906,11 @@ __device__ __forceinline__ void tlB_add(uint32_t flags, const PairB& p, const Re
 		const float dvx = ffd(p.v.x, p.v.y, ri.v.x, ri.v.y), dvy = ffd(p.v.z, p.v.w, ri.v.z, ri.v.w);
 		const float dot = dvx * xij + dvy * yij;  // -v_ij . x_ij
 		if (dot > 0.f) {                          // approaching
-			// with n = 2 h_ij dot, D = r^2 + eta^2 h_ij^2, rs = rho_i + rho_j and
-			// A = 1 / (D rs): Pi = n A (alpha c_ij + beta / 2 n A rs), each factor times rho0
-			const float hs = ri.hmrc.x + p.hmrc.x, rs = ri.hmrc.z + p.hmrc.z;
+			// with n = 2 h_ij dot, D = r^2 + eta^2 h_ij^2, rs = (rho_i + rho_j) / s and
+			// A = 1 / (D rs): Pi = n A / s (alpha c_ij + beta / 2 n A rs)
+			const float hs = ri.hmrc.x + p.hmrc.x, rs = __fmaf_rn(p.hmrc.z, k.s1, k.rho);
 			const float D = xij * xij + yij * yij + k.eta2q * hs * hs;
-			const float nA = __fdividef(hs * dot * k.rho0, D * rs);
+			const float nA = __fdividef(hs * dot, D * rs);
 			pi2 = nA * (k.half_alpha * (ri.hmrc.w + p.hmrc.w) + k.half_beta * rs * nA);
 		}
 	}
@@ -927,17 +929,21 @@ __global__ void __launch_bounds__(256, MB) k_tlB32r(TLArgs a) {
 	// (the stress sums only reach the momentum equation)
 	const uint32_t flags = (a.flags & A_MOMENTUM_TL) ? a.flags : a.flags & ~A_STRESS_TL;
 	const BodyParams& pr = a.params[a.body_of[i]];
-	const float rho0 = pr.frho0, r1 = 1.f / rho0;
-	const RecB ri = rb_load(a.recB, a.n_total, i);
+	const float rho0 = pr.frho0;
+	const uint32_t e0 = min(max(__float_as_uint(rho0) >> 23 & 0xffu, 1u), 253u);
+	const float s0 = __uint_as_float(e0 << 23), s1 = __uint_as_float((254u - e0) << 23);  // s, 1/s
+	const float m2 = (rho0 * s1) * (rho0 * s1);                                           // (rho0 / s)^2
+	RecB ri = rb_load(a.recB, a.n_total, i);
 	const float4 Xi = ((const float4*)a.XF)[i];
 	RowB rk;
 	rk.h1 = 1.f / ri.hmrc.x;
 	rk.eta2q = 0.25f * pr.feta2;
-	rk.half_alpha = 0.5f * pr.falpha * rho0;
-	rk.half_beta = 0.5f * pr.fbeta;
-	rk.rho0 = rho0;
+	rk.half_alpha = 0.5f * pr.falpha * m2 * s0;
+	rk.half_beta = 0.5f * pr.fbeta * m2 * s0;
+	rk.s1 = s1;
+	rk.rho = ri.hmrc.z * s1;
 	rk.G = ((const float4*)a.G)[i];
-	const float f3 = 3.f * K_SPLINE_2D * rk.h1 * rk.h1 * r1;
+	const float f3 = 3.f * K_SPLINE_2D * rk.h1 * rk.h1 * s1;
 	rk.G.x *= f3; rk.G.y *= f3; rk.G.z *= f3; rk.G.w *= f3;
 	AccB s;
 	uint32_t q = a.r_sl[i >> 5] + (i & 31u), nr = a.r_cnt[i];
@@ -956,13 +962,16 @@ __global__ void __launch_bounds__(256, MB) k_tlB32r(TLArgs a) {
 			}
 		}
 	}
-	// the sums over rho0 are handed on as the viscosity's share (tlB_finish adds the contact
-	// force)
+	// the sums over rho0^2 are handed on as the viscosity's share (tlB_finish adds the
+	// contact force)
 	if (flags & A_STRESS_TL) {
-		s.ax += ri.P.x * s.wx + ri.P.z * s.wy;
-		s.ay += ri.P.y * s.wx + ri.P.w * s.wy;
+		// (64 registers do not hold P through the walk)
+		const float4 P = MB < 4 ? ri.P : rb_field(a.recB, a.n_total, RB_P)[i];
+		s.ax += P.x * s.wx + P.z * s.wy;
+		s.ay += P.y * s.wx + P.w * s.wy;
 	}
-	tlB_finish(a, i, pr, rho0, 0.f, 0.f, 0.f, 0.f, s.ax * r1, s.ay * r1);
+	const float r21 = 1.f / m2 * s1;
+	tlB_finish(a, i, pr, rho0, 0.f, 0.f, 0.f, 0.f, s.ax * r21, s.ay * r21);
 }
 
 // ---- mixed form over halo tiles.  The same per-row arithmetic, in the same order, as
