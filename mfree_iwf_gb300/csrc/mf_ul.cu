@@ -1713,7 +1713,13 @@ __global__ void __launch_bounds__(ORD_THREADS, 4) k_pair_ordered(ULArgs a, const
 	pair32_row<false, FULL, 8, true>(a, P, G, st, k, t % 8, rows + threadIdx.x / 8);
 }
 
-constexpr uint32_t PAIR_ROWS_MB4 = 1u << 19;
+// Rows an SM from which the mixed pair pass runs with four blocks of 256 an SM at 64
+// registers (some constants of a row spilled) instead of three at 80: the deeper occupancy
+// pays once every SM has several rounds of blocks, 27 of 128 rows here.  Per step, three / four
+// blocks, ring impacts of 4k to 110k rows: 223,600 rows 355 / 380 us, 316,600 462 / 487,
+// 445,512 598 / 588, 518,680 671 / 681, 600,448 759 / 733, 1,053,456 1182 / 1155, 1,349,144
+// 1461 / 1430; of 4.4k rows: 331,944 452 / 476, 671,232 745 / 727, 3,348,184 3245 / 3090.
+constexpr uint32_t PAIR_ROWS_MB4 = 3450;
 
 // The mixed pair kernel.  Plain form: one thread per cell-ordered row.  Persistent form
 // (one launch per stage over all bodies): a fixed grid whose blocks take chunks of
@@ -1791,9 +1797,13 @@ unsigned row_block(const ULArgs& a) {
 	return bs;
 }
 
-// One block's FP64 divisions for the cell keys hold its SM's narrow pipe for 7.5 ns a row:
-// up to 1024 rows that is a fraction of the launches saved; a single body of 4,408 rows
-// takes 45 us this way and 26 with the general kernels, unless every SM has such a body.
+// One block's FP64 divisions for the cell keys hold its SM's narrow pipe for 7.5 ns a row.
+// Up to 1024 rows that is a fraction of the launches saved (one body of 856 rows, mixed step:
+// 63 us with the general kernels, 61 this way); from there on a lone body's block is the
+// longer one (1,684 rows 68 / 70 us, 2,608 72 / 80, 4,408 76 / 96).  With a body for every SM
+// the blocks share the work: 152 bodies of 1,096 rows 281 / 215 us, of 4,408 771 / 696 (FP64
+// 3044 / 2796 and 11,338 / 11,037).  The line between lies where every SM is known to have
+// one; it could lie lower (19 bodies of 1,096 rows 134 / 104 us, of 4,408 198 / 163).
 bool ul_small_grid(const ULArgs& a) {
 	const uint32_t limit = a.n_bodies >= a.sm_count && a.sm_count ? GRID_BODY_MAX : 1024u;
 	return a.max_body && a.max_body <= limit && a.n_bodies <= GRID_MAX_BODIES && !a.failed;
@@ -1882,10 +1892,7 @@ cudaError_t ul_stage(const ULArgs& args, bool mixed, cudaStream_t s) {
 		else if (split == 4) launch(god ? k_pair_split<true, false, 4> : full ? k_pair_split<false, true, 4> : k_pair_split<false, false, 4>);
 		else if (split == 8) launch(god ? k_pair_split<true, false, 8> : full ? k_pair_split<false, true, 8> : k_pair_split<false, false, 8>);
 		else if (god || !full) launch(god ? k_pair<true, false, 3> : k_pair<false, false, 3>);
-		// More warps pay once every SM has several rounds of blocks: 64 ring impacts (1.35M
-		// rows) 30.9 -> 30.0 ms for 20 steps, 256 small impacts (317k rows) 5.69 -> 5.83 ms
-		// for 10, the rings at dx = 1 mm (4,408 rows) 9.9 -> 11.3 ms for 100.
-		else launch(a.n_total >= PAIR_ROWS_MB4 ? k_pair<false, true, 4> : k_pair<false, true, 3>);
+		else launch(a.n_total / PAIR_ROWS_MB4 >= a.sm_count ? k_pair<false, true, 4> : k_pair<false, true, 3>);
 	} else {
 		const unsigned g64 = grid1(a.n_total, P64_ROWS);
 		if (god) launch_after(k_pair64<true>, g64, P64_THREADS, 0, s, a, a.params, a.geom, st);
