@@ -13,8 +13,10 @@
 //                the rows' stage state in cell order, with the per-particle actions
 //                EOS (material.h:37-64), artificial stress (correctors.h:37-81) and
 //                integration weights (riemann_integration.h:28-33) fused in
-//   ul_pair      one thread per row: walks the 3x3 cell stencil of the reference grid
-//                (grid.h:117-177), evaluates W/gradW (kernel.cpp:20-55) and every pair
+//   ul_pair      the row's cells of the stencil (FP64: 3x3 cells of the reference grid,
+//                grid.h:117-177, four lanes a row; mixed: up to 5x5 half-size cells, one
+//                thread a row, or eight lanes where rows are few): tests the candidates,
+//                evaluates W/gradW (kernel.cpp:20-55) and every pair
 //                action at once -- derive_stress_monaghan (derivatives.h:378-443),
 //                derive_velocity (:32-66), artificial viscosity (correctors.h:83-137),
 //                XSPH (:139-169) -- then the per-particle actions Jaumann rate
@@ -791,8 +793,8 @@ struct Acc64 {
 	double god_rho = 0., god_vx = 0., god_vy = 0.;
 };
 
-// All pair terms in the reference's expressions.  rho21: whether the records hold the
-// stress itself (1/rho^2 applied here) or already times 1/rho^2 (the fast gather).
+// All pair terms in the reference's expressions (the records hold the stress itself; 1/rho^2 is
+// applied here).
 template <bool GOD>
 __device__ __forceinline__ void pair64_ref(uint32_t flags, const BodyParams& pr, const Rec64& ri, const Rec64& rj,
                                            Acc64& s) {
