@@ -1751,6 +1751,7 @@ WeakArgs weak_args(mf_ctx* c) {
 	a.n_p = c->n_total; a.n_g = c->n_g; a.n_bodies = (uint32_t)c->bodies.size(); a.flags = c->flags;
 	a.block = c->tune.tl_block;
 	a.sm_count = (uint32_t)std::max(1, c->sm_count);
+	a.g_entries = c->g_entries;
 	a.params = c->params.p; a.body_of = c->body_of.p; a.gp_body = c->gp_body.p;
 	a.X = c->X.p; a.Y = c->Y.p; a.m = c->m.p; a.qw_p = c->qw0.p; a.gp_qw = c->gp_qw.p; a.fcx = c->fcx.p; a.fcy = c->fcy.p;
 	a.gp_ux = c->gp_ux.p; a.gp_uy = c->gp_uy.p;

@@ -204,6 +204,7 @@ constexpr uint32_t TL_RUN_MAX_LEN = 32;
 // Sxx, Sxy, Syy in the rho/Sxx/Sxy/Syy or *_f slots of the StateSoA).
 struct WeakArgs {
 	uint32_t n_p, n_g, n_bodies, stage, flags, block, sm_count;
+	uint64_t g_entries;  // list entries of all Gauss points
 	const BodyParams* params;
 	const uint32_t *body_of, *gp_body;
 	const double *X, *Y, *m, *qw_p, *gp_qw, *fcx, *fcy;

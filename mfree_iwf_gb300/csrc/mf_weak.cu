@@ -550,9 +550,12 @@ __device__ __forceinline__ void load8(const float4* p, float4& a, float4& b) {
 // blocks of 256 an SM (MB).  3.2M Gauss points, per stage: 261 us with two 16-byte loads and
 // 8 blocks, 247 now; also measured: one load at 8 blocks 279 (spills), two arrays 288,
 // velocities as FP32 in an array of their own 249, entries prefetched 2 to 4 ahead 340 to
-// 524.  Where 8 blocks an SM need a wave less, of one or two, they stay (gp_eight): plates
-// of 290k / 513k Gauss points 1885 / 2442 us for 5 steps with them, 1974 / 2469 with 6; at
-// 392k (two waves either way) 2290 and 2082, at 1.5M 5488 and 5388.
+// 524.  Short lists leave less to gather and more to hide (gp_eight): below GP_SHORT entries a
+// point on average two 16-byte loads at 8 blocks stay.  8 / 6 blocks, us a stage at 3.2M Gauss
+// points by entries a point: 7.9 141 / 146, 10.8 166 / 169, 16.4 212 / 208, 21.2 263 / 250,
+// 48 477 / 422; element functions (4 entries), 7.9M points: 259 / 288.  Where 8 blocks need a wave less, of one or two, they stay too: plates of 290k /
+// 513k Gauss points 1885 / 2442 us for 5 steps with them, 1974 / 2469 with 6; at 392k (two
+// waves either way) 2290 and 2082, at 1.5M 5488 and 5388.
 template <int MB>
 __global__ void __launch_bounds__(256, MB) k_gp_pass32(WeakArgs a) {
 	uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -746,7 +749,9 @@ cudaError_t weak_sell(uint32_t n, const uint32_t* off, const uint32_t* nbr, cons
 }
 
 // 8 blocks of 256 threads an SM in the mixed Gauss-point pass (see there)
+constexpr uint64_t GP_SHORT = 13;
 static bool gp_eight(const WeakArgs& a, unsigned bs) {
+	if (a.g_entries < GP_SHORT * a.n_g) return true;
 	auto waves = [&](unsigned per_sm) {
 		const unsigned slots = per_sm * 256u / bs * a.sm_count, blocks = grid1(a.n_g, bs);
 		return (blocks + slots - 1) / slots;
