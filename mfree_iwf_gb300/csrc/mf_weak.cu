@@ -305,22 +305,31 @@ __device__ __forceinline__ void gp_rk(const WeakArgs& a, uint32_t i, double dt, 
 	}
 }
 
-// RK4 update of one component of particle j (rk4.h:140-183) from its rate d, own row
-// only: in place; false when the step ends in a value that is not finite
-__device__ __forceinline__ bool p_rk64_one(const WeakArgs& a, double* bp, double* ap, double* sp, uint32_t j, double dt,
-                                           double d) {
+// RK4 update of N components of particle j (rk4.h:140-183) from their rates d, own row only:
+// in place; false when the step ends in a value that is not finite
+template <int N>
+__device__ __forceinline__ bool p_rk64(const WeakArgs& a, double* const (&bp)[N], double* const (&ap)[N],
+                                       double* const (&sp)[N], uint32_t j, double dt, const double (&d)[N]) {
 	const uint32_t stg = a.stage;
+	bool ok = true;
 	if (stg < 3) {
 		const double dts = (stg == 2 ? 1.0 : 0.5) * dt;
-		ap[j] = (stg == 0) ? d : ap[j] + 2 * d;
-		sp[j] = bp[j] + d * dts;
-		return true;
+#pragma unroll
+		for (int q = 0; q < N; q++) {
+			ap[q][j] = (stg == 0) ? d[q] : ap[q][j] + 2 * d[q];
+			sp[q][j] = bp[q][j] + d[q] * dts;
+		}
+	} else {
+		const double w6 = dt * 1. / 6.;
+#pragma unroll
+		for (int q = 0; q < N; q++) {
+			const double v = bp[q][j] + w6 * (ap[q][j] + d[q]);
+			bp[q][j] = v;
+			sp[q][j] = v;
+			ok = ok && isfinite(v);
+		}
 	}
-	const double w6 = dt * 1. / 6.;
-	const double v = bp[j] + w6 * (ap[j] + d);
-	bp[j] = v;
-	sp[j] = v;
-	return isfinite(v);
+	return ok;
 }
 
 #if !MF_STRICT_FORM
@@ -422,19 +431,19 @@ __global__ void __launch_bounds__(256) k_p_pass64(WeakArgs a) {
 		}
 	}
 	const mfk_host::StateSoA& s = a.st;
-	double d = 0.;  // the rate of component `lane`
+	double d[1] = {0.};  // the rate of component `lane`
 	if (lane < 2) {
-		if (flags & A_ADVECTION) d = (lane == 0 ? s.vx : s.vy)[j];
+		if (flags & A_ADVECTION) d[0] = (lane == 0 ? s.vx : s.vy)[j];
 	} else if (flags & A_MOMENTUM_W) {
-		d = ((lane == 2 ? a.fcx : a.fcy)[j] - (lane == 2 ? fx : fy)) * rcp64(a.m[j]);
+		d[0] = ((lane == 2 ? a.fcx : a.fcy)[j] - (lane == 2 ? fx : fy)) * rcp64(a.m[j]);
 	}
 	// (lanes 2 and 3 now replace the stage velocity that lanes 0 and 1 have read)
 	__syncwarp();
 	if (!live) return;
-	const bool ok = p_rk64_one(a, lane == 0 ? a.base.x : lane == 1 ? a.base.y : lane == 2 ? a.base.vx : a.base.vy,
-	                           lane == 0 ? a.acc.x : lane == 1 ? a.acc.y : lane == 2 ? a.acc.vx : a.acc.vy,
-	                           lane == 0 ? a.st.x : lane == 1 ? a.st.y : lane == 2 ? a.st.vx : a.st.vy, j,
-	                           a.params[a.body_of[j]].dt, d);
+	double* const bp[1] = {lane == 0 ? a.base.x : lane == 1 ? a.base.y : lane == 2 ? a.base.vx : a.base.vy};
+	double* const ap[1] = {lane == 0 ? a.acc.x : lane == 1 ? a.acc.y : lane == 2 ? a.acc.vx : a.acc.vy};
+	double* const sp[1] = {lane == 0 ? a.st.x : lane == 1 ? a.st.y : lane == 2 ? a.st.vx : a.st.vy};
+	const bool ok = p_rk64(a, bp, ap, sp, j, a.params[a.body_of[j]].dt, d);
 	if (!ok) raise(reinterpret_cast<DevStatus*>(a.status), ERR_NONFINITE, j);
 }
 
@@ -515,12 +524,10 @@ __global__ void __launch_bounds__(256) k_p_pass64(WeakArgs a) {
 		d[2] += 1. / m * (Pxx_x + Pyx_y) + a.fcx[j] / a.m[j];
 		d[3] += 1. / m * (Pxy_x + Pyy_y) + a.fcy[j] / a.m[j];
 	}
-	double* bp[4] = {a.base.x, a.base.y, a.base.vx, a.base.vy};
-	double* ap[4] = {a.acc.x, a.acc.y, a.acc.vx, a.acc.vy};
-	double* sp[4] = {a.st.x, a.st.y, a.st.vx, a.st.vy};
-	bool ok = true;
-#pragma unroll
-	for (int q = 0; q < 4; q++) ok = p_rk64_one(a, bp[q], ap[q], sp[q], j, pr.dt, d[q]) && ok;
+	double* const bp[4] = {a.base.x, a.base.y, a.base.vx, a.base.vy};
+	double* const ap[4] = {a.acc.x, a.acc.y, a.acc.vx, a.acc.vy};
+	double* const sp[4] = {a.st.x, a.st.y, a.st.vx, a.st.vy};
+	const bool ok = p_rk64(a, bp, ap, sp, j, pr.dt, d);
 	if (!ok) raise(reinterpret_cast<DevStatus*>(a.status), ERR_NONFINITE, j);
 }
 #endif

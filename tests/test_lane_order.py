@@ -34,7 +34,7 @@ def whole_warp_barriers(body):
             yield m.start()
 
 
-@pytest.mark.parametrize("file,kernel,read,write", [("mf_weak.cu", "k_p_pass64", r"\bs\.v[xy]\b", r"p_rk64_one\("),
+@pytest.mark.parametrize("file,kernel,read,write", [("mf_weak.cu", "k_p_pass64", r"\bs\.v[xy]\b", r"p_rk64\("),
                                                     ("mf_ul.cu", "k_pair64", r"\bsv\.S\w\w\[i\]", r"\bS\[i\] =")])
 def test_barrier_between_reads_and_writes_of_a_row(file, kernel, read, write):
     body = kernel_body(file, kernel)
