@@ -965,10 +965,11 @@ __global__ void __launch_bounds__(256, MB) k_tlB32r(TLArgs a) {
 	// the sums over rho0^2 are handed on as the viscosity's share (tlB_finish adds the
 	// contact force)
 	if (flags & A_STRESS_TL) {
-		// (64 registers do not hold P through the walk)
+		// (64 registers do not hold P through the walk; the contraction is spelled out: the same
+		// bits wherever P comes from)
 		const float4 P = MB < 4 ? ri.P : rb_field(a.recB, a.n_total, RB_P)[i];
-		s.ax += P.x * s.wx + P.z * s.wy;
-		s.ay += P.y * s.wx + P.w * s.wy;
+		s.ax = __fadd_rn(s.ax, __fmaf_rn(P.z, s.wy, __fmul_rn(P.x, s.wx)));
+		s.ay = __fadd_rn(s.ay, __fmaf_rn(P.w, s.wy, __fmul_rn(P.y, s.wx)));
 	}
 	const float r21 = 1.f / m2 * s1;
 	tlB_finish(a, i, pr, rho0, 0.f, 0.f, 0.f, 0.f, s.ax * r21, s.ay * r21);
