@@ -31,6 +31,7 @@ def test_nothing_past_the_result(lib, dims, members, rows, fused):
     whole = (size + page - 1) // page * page  # (the result's own last page is written anyway)
     behind = (rows * dims[-1] * 4 + page - 1) // page * page
     mem = mmap.mmap(-1, whole + behind)
+    mem.madvise(mmap.MADV_NOHUGEPAGE)  # (a huge page would hold both the result and what follows it)
     keep = ctypes.c_char.from_buffer(mem)
     addr = ctypes.addressof(keep)
     fp = ctypes.POINTER(ctypes.c_float)
