@@ -465,7 +465,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 //     chunks, through a ring of shared-memory stages with TMA, half of the chunk's N rows
 //     to each CTA, both reporting to the first CTA's barrier;
 //   - the MMA issuer (warp 1 of the first CTA) multiplies with cta_group::2: A = a half's
-//     256 rows, B = the chunk's N weight rows, each CTA holding half of both.  A layer's
+//     256 rows, B = the chunk's N weight rows, each CTA holding half of both (N padded by
+//     zeros to a multiple of 32, the widths that published code uses with M = 256).  A layer's
 //     chunks stay in the ring for both halves: half 0's epilogue runs under half 1's
 //     products, and half 0's next products under half 1's epilogue;
 //   - the epilogue warps (16 in each CTA: four TMEM lane quarters x two halves x two
@@ -500,11 +501,12 @@ constexpr int STAGES = 5;            // weight chunks in shared memory: a layer'
 constexpr uint32_t TMEM_COLS = 512;  // two accumulators of up to 256 columns
 
 struct Maps {
-	CUtensorMap w[MF_MLP_MAX_LAYERS];  // per layer: [members][N][K] BF16, boxes of 64 K x N / 2 rows
+	CUtensorMap w[MF_MLP_MAX_LAYERS];  // per layer: [members][N2][K] BF16, boxes of 64 K x N2 / 2 rows
 };
 struct Args {
 	int L, in, out, rows, kc_max, n_max;
-	int N[MF_MLP_MAX_LAYERS], KC[MF_MLP_MAX_LAYERS];  // MMA width (padded to 16); K / 64 (K padded to 64)
+	int N[MF_MLP_MAX_LAYERS], KC[MF_MLP_MAX_LAYERS];  // width (padded to 16); K / 64 (K padded to 64)
+	int N2[MF_MLP_MAX_LAYERS];                        // MMA width: N padded to 32
 	int b_off[MF_MLP_MAX_LAYERS];
 	const float* bias;
 	long long b_per;
@@ -703,7 +705,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 			for (int t = first; t < total && ok; t += pairs) {
 				const int z = t % a.members;
 				for (int l = 0; l < L && ok; l++) {
-					const int rows = a.N[l] >> 1;
+					const int rows = a.N2[l] >> 1;
 					for (int kc = 0; kc < a.KC[l]; kc++) {
 						if (loads == S && !(ok = mbar_wait(w_empty + st, ph))) break;
 						if (rank == 0) mbar_expect_tx(w_full + st, 2u * (uint32_t)rows * 128u);
@@ -739,7 +741,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 			for (int t = first; t < total && ok; t += pairs)
 				for (int l = 0; l < L && ok; l++, step++) {
 					const int KC = a.KC[l], layer_st = st;
-					const uint32_t idesc = idesc_bf16(2 * HALF, a.N[l]);
+					const uint32_t idesc = idesc_bf16(2 * HALF, a.N2[l]);
 					for (int h = 0; h < 2 && ok; h++) {
 						if (!(ok = wait_warp(act_ready + h, step & 1u))) break;
 						st = layer_st;
@@ -913,17 +915,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 		asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
 }
 
-// weights of one layer for the fused kernel: [members][N][Kp] BF16, K padded to Kp
-// (a multiple of 64) by zeros
-__global__ void k_pack_layer(int members, int N, int K, int Kp, const bf16* src, long long s_per, bf16* dst,
+// weights of one layer for the fused kernel: [members][Np][Kp] BF16, N and K padded to Np (a
+// multiple of 32) and Kp (of 64) by zeros
+__global__ void k_pack_layer(int members, int N, int K, int Np, int Kp, const bf16* src, long long s_per, bf16* dst,
                              long long d_per) {
 	const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-	const long long per = (long long)N * Kp;
+	const long long per = (long long)Np * Kp;
 	if (e >= per * members) return;
 	const int z = (int)(e / per);
 	const long long w = e % per;
 	const int o = (int)(w / Kp), i = (int)(w % Kp);
-	dst[z * d_per + w] = i < K ? src[z * s_per + (long long)o * K + i] : __float2bfloat16(0.f);
+	dst[z * d_per + w] = o < N && i < K ? src[z * s_per + (long long)o * K + i] : __float2bfloat16(0.f);
 }
 
 }  // namespace fz
@@ -1289,6 +1291,7 @@ __global__ void k_output(int members, int rows, int out, int out_p, const float*
 }
 
 inline int pad16(int v) { return (v + 15) / 16 * 16; }
+inline int pad32(int v) { return (v + 31) / 32 * 32; }
 inline unsigned nblk(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 template <class T>
@@ -1452,11 +1455,11 @@ long long sH(const mf_mlp* m, int l) { return (long long)m->rows * m->pd[l]; }
 // accumulator per half tile, at most four K chunks).
 void fused_plan(mf_mlp* m) {
 	m->fz_kc = 1;
-	m->fz_n = 16;
+	m->fz_n = 32;
 	bool fits = true;
 	for (int l = 0; l < m->L; l++) {
 		m->fz_kc = std::max(m->fz_kc, (m->pd[l] + 63) / 64);
-		m->fz_n = std::max(m->fz_n, m->pd[l + 1]);
+		m->fz_n = std::max(m->fz_n, pad32(m->pd[l + 1]));
 		fits = fits && m->pd[l] <= 256 && m->pd[l + 1] <= 256;
 	}
 	m->fz_fits = fits;
@@ -1465,7 +1468,7 @@ void fused_plan(mf_mlp* m) {
 bool fused_eligible(const mf_mlp* m) { return m->tc && m->fused && m->fz_fits; }
 
 // (re)packs the BF16 weights for the fused kernel and encodes one tensor map per layer:
-// [members][N][Kp] with member stride wf_per, boxes of 64 K x N / 2 rows x 1 member
+// [members][Np][Kp] with member stride wf_per, boxes of 64 K x Np / 2 rows x 1 member
 mf_status fused_prepare(mf_mlp* m) {
 	if (!m->wf_dirty) return MF_OK;
 	if (!m->Wf.p) {
@@ -1473,21 +1476,21 @@ mf_status fused_prepare(mf_mlp* m) {
 		m->wf_per = 0;
 		for (int l = 0; l < m->L; l++) {
 			m->wf_off.push_back(m->wf_per);
-			m->wf_per += (long long)m->pd[l + 1] * ((m->pd[l] + 63) / 64 * 64);
+			m->wf_per += (long long)pad32(m->pd[l + 1]) * ((m->pd[l] + 63) / 64 * 64);
 		}
 		MCK(m->Wf.alloc((size_t)m->wf_per * m->members));
 	}
 	EncodeTiled enc = tensor_map_encoder();
 	for (int l = 0; l < m->L; l++) {
-		const int N = m->pd[l + 1], K = m->pd[l], Kp = (K + 63) / 64 * 64;
-		const long long per = (long long)N * Kp * m->members;
-		fz::k_pack_layer<<<nblk(per, 256), 256, 0, m->stream>>>(m->members, N, K, Kp, m->Wb.p + m->w_off[l], m->w_per,
+		const int N = m->pd[l + 1], K = m->pd[l], Np = pad32(N), Kp = (K + 63) / 64 * 64;
+		const long long per = (long long)Np * Kp * m->members;
+		fz::k_pack_layer<<<nblk(per, 256), 256, 0, m->stream>>>(m->members, N, K, Np, Kp, m->Wb.p + m->w_off[l], m->w_per,
 		                                                      m->Wf.p + m->wf_off[l], m->wf_per);
 		m->launches++;
 		MCK(cudaGetLastError());
-		const cuuint64_t dW[3] = {(cuuint64_t)Kp, (cuuint64_t)N, (cuuint64_t)m->members};
+		const cuuint64_t dW[3] = {(cuuint64_t)Kp, (cuuint64_t)Np, (cuuint64_t)m->members};
 		const cuuint64_t sW[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)m->wf_per * 2};
-		const cuuint32_t bW[3] = {64, (cuuint32_t)(N / 2), 1}, e1[3] = {1, 1, 1};  // (N: a multiple of 16)
+		const cuuint32_t bW[3] = {64, (cuuint32_t)(Np / 2), 1}, e1[3] = {1, 1, 1};
 		if (enc(&m->maps.w[l], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, m->Wf.p + m->wf_off[l], dW, sW, bW, e1,
 		        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
 		        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
@@ -1511,6 +1514,7 @@ cudaError_t fused_forward(mf_mlp* m, const float* x, long long sx, int rows, flo
 	a.n_max = m->fz_n;
 	for (int l = 0; l < m->L; l++) {
 		a.N[l] = m->pd[l + 1];
+		a.N2[l] = pad32(m->pd[l + 1]);
 		a.KC[l] = (m->pd[l] + 63) / 64;
 		a.b_off[l] = (int)m->b_off[l];
 	}
